@@ -241,9 +241,7 @@ int db200_rbf_block_f64(db200_context* ctx, int m, int n, int d, const float* Xi
   double* sj = cv.take<double>(n);
   int st = rownorm_f64(ctx, Xi, ldxi, m, d, si);
   if (!st) st = rownorm_f64(ctx, Xj, ldxj, n, d, sj);
-  // G = Xi Xj^T on the FP64 tensor cores (the Gram kernel over the d features), then K in place
-  if (!st) st = gram<float, float>(ctx, d, m, n, Xi, ldxi, Xj, ldxj, nullptr, 1.0, 0.0, K, ldk, false);
-  if (!st) st = rbf_from_gram_f64(ctx, K, ldk, m, n, si, sj, yi, yj, gamma);
+  if (!st) st = rbf_block_f64_fused(ctx, m, n, d, Xi, ldxi, Xj, ldxj, si, sj, yi, yj, gamma, K, ldk);
   return st;
 }
 

@@ -7,6 +7,7 @@
 #include <cstdio>
 #include <type_traits>
 
+#include "dmm64.cuh"
 #include "internal.h"
 #include "la64.h"
 
@@ -14,380 +15,8 @@ namespace db200 {
 
 namespace {
 
-template <typename T>
-__device__ __forceinline__ double ld64(const T* p) { return (double)__ldg(p); }
-
-// C[p x q] (+)= alpha * A^T diag(w) B over rows [r0, r1) of A (n x p) and B (n x q); FP64 accumulation.
-// grid.z splits the rows; partial tiles are added with FP64 atomics when grid.z > 1.
-//
-// FP64 tensor cores (mma.sync.m16n8k8.f64): 128 x 128 output tile per CTA, 8 warps of 32 x 64 (2 x 8 MMA tiles,
-// 64 accumulators per thread).  Stages of 8 rows of A and B are fetched into registers one stage ahead (coalesced
-// column reads: consecutive threads walk consecutive rows) and parked transposed (k-major) in a double-buffered
-// shared tile; per stage a warp loads 2 A fragments (4 doubles each) and 8 B fragments (2 doubles each) for 16
-// MMAs.  Fragment layouts of m16n8k8 (g = lane / 4, t = lane % 4): A (16 x 8, row) a0..a3 = A[g][t], A[g+8][t],
-// A[g][t+4], A[g+8][t+4]; B (8 x 8, col) b0, b1 = B[t][g], B[t+4][g]; C (16 x 8) c0, c1 = C[g][2t + 0, 1],
-// c2, c3 = C[g+8][2t + 0, 1].
-constexpr int GT = 128;        // Gram output tile
-constexpr int GK = 8;          // rows per stage
-constexpr int GPAD = GT + 8;   // padded shared row: 4 consecutive k rows land 16 banks apart
-
-__device__ __forceinline__ void dmma16(double* d, const double* a, const double* b) {
-  asm volatile("mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
-               "{%0,%1,%2,%3};"
-               : "+d"(d[0]), "+d"(d[1]), "+d"(d[2]), "+d"(d[3])
-               : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(b[0]), "d"(b[1]));
-}
-
-constexpr int GTHREADS = 256;
-
-template <typename TA, typename TBt>
-__global__ void __launch_bounds__(GTHREADS, 1) gram_kernel(int n, int p, int q, const TA* __restrict__ A, long long lda,
-                                                      const TBt* __restrict__ B, long long ldb,
-                                                      const double* __restrict__ w, double alpha, double* C, int ldc,
-                                                      int rows_per_split, int upper_only, int atomic) {
-  const int bi = blockIdx.x, bj = blockIdx.y;
-  if (upper_only && bi > bj) return;
-  const int i0 = bi * GT, j0 = bj * GT;
-  const int r0 = blockIdx.z * rows_per_split;
-  const int r1 = min(n, r0 + rows_per_split);
-  __shared__ __align__(16) double sA[2][GK][GPAD];
-  __shared__ __align__(16) double sB[2][GK][GPAD];
-  const int lane = threadIdx.x % 32, warp = threadIdx.x / 32;
-  const int wm = warp / 2, wn = warp % 2;  // warp tile: rows 32 wm .. +31, columns 64 wn .. +63
-  const int fr = lane / 4, fk = lane % 4;  // fragment row / k index of this lane
-  double acc[2][8][4];
-#pragma unroll
-  for (int a = 0; a < 2; ++a)
-#pragma unroll
-    for (int b = 0; b < 8; ++b)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) acc[a][b][e] = 0.0;
-  const int kk = threadIdx.x % GK;   // row inside the stage this thread loads
-  const int c0 = threadIdx.x / GK;   // first column it loads (then +32, +64, +96)
-  double va[4], vb[4];
-  auto fetch = [&](int k0) {
-    const int k = k0 + kk;
-    const bool kin = k < r1;
-    const double wk = (w && kin) ? w[k] : 1.0;
-#pragma unroll
-    for (int s = 0; s < 4; ++s) {
-      const int c = c0 + 32 * s;
-      const int ia = i0 + c, jb = j0 + c;
-      va[s] = (kin && ia < p) ? wk * ld64(A + (long long)ia * lda + k) : 0.0;
-      vb[s] = (kin && jb < q) ? ld64(B + (long long)jb * ldb + k) : 0.0;
-    }
-  };
-  auto park = [&](int buf) {
-#pragma unroll
-    for (int s = 0; s < 4; ++s) {
-      sA[buf][kk][c0 + 32 * s] = va[s];
-      sB[buf][kk][c0 + 32 * s] = vb[s];
-    }
-  };
-  int buf = 0;
-  if (r0 < r1) {
-    fetch(r0);
-    park(0);
-  }
-  __syncthreads();
-  for (int k0 = r0; k0 < r1; k0 += GK) {
-    // the next stage's global loads are in flight while this stage is multiplied
-    const bool more = k0 + GK < r1;
-    if (more) fetch(k0 + GK);
-    {
-      double af[2][4], bf[8][2];
-#pragma unroll
-      for (int a = 0; a < 2; ++a) {
-        const int r = 32 * wm + 16 * a + fr;
-        af[a][0] = sA[buf][fk][r];
-        af[a][1] = sA[buf][fk][r + 8];
-        af[a][2] = sA[buf][fk + 4][r];
-        af[a][3] = sA[buf][fk + 4][r + 8];
-      }
-#pragma unroll
-      for (int b = 0; b < 8; ++b) {
-        const int c = 64 * wn + 8 * b + fr;
-        bf[b][0] = sB[buf][fk][c];
-        bf[b][1] = sB[buf][fk + 4][c];
-      }
-#pragma unroll
-      for (int a = 0; a < 2; ++a)
-#pragma unroll
-        for (int b = 0; b < 8; ++b) dmma16(acc[a][b], af[a], bf[b]);
-    }
-    if (more) park(buf ^ 1);  // the other buffer was last read one stage ago, before the barrier below
-    __syncthreads();
-    buf ^= 1;
-  }
-#pragma unroll
-  for (int a = 0; a < 2; ++a) {
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int i = i0 + 32 * wm + 16 * a + 8 * h + fr;
-      if (i >= p) continue;
-#pragma unroll
-      for (int b = 0; b < 8; ++b) {
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const int j = j0 + 64 * wn + 8 * b + 2 * fk + e;
-          if (j >= q) continue;
-          if (upper_only && i > j) continue;
-          double* dst = C + (long long)j * ldc + i;
-          const double v = alpha * acc[a][b][2 * h + e];
-          if (atomic)
-            atomicAdd(dst, v);
-          else
-            *dst += v;
-        }
-      }
-    }
-  }
-}
-
-// The same Gram for FP64 operands with 16-byte-aligned columns (base and leading dimensions), as a cp.async
-// pipeline: 16-row stages of A's and B's 128 columns land column-major in shared memory (padded so that the
-// fragment loads of a warp spread over the banks), GP_STAGES deep, while the 8 warps run the DMMA tiles of the
-// stage before; a stage's rows past the split's end or columns past p / q are zero-filled by the copy.  The weights
-// scale A's fragments.  Same tiles, accumulators and epilogue as gram_kernel.
-constexpr int GP_KS = 16;                   // rows per stage
-constexpr int GP_KPAD = GP_KS + 4;          // doubles per staged column (= 4 mod 16: conflict-free fragment loads)
-constexpr int GP_STAGES = 4;
-constexpr int GP_STAGE_DOUBLES = 2 * GT * GP_KPAD;  // A and B
-constexpr size_t GP_SMEM = (size_t)GP_STAGES * GP_STAGE_DOUBLES * sizeof(double);
-
-__device__ __forceinline__ void gp_cp16(double* smem, const double* gmem, int valid_doubles) {
-  const uint32_t sa = static_cast<uint32_t>(__cvta_generic_to_shared(smem));
-  const int bytes = valid_doubles <= 0 ? 0 : (valid_doubles >= 2 ? 16 : 8);  // the rest zero-filled
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(sa), "l"(gmem), "r"(bytes) : "memory");
-}
-
-__global__ void __launch_bounds__(GTHREADS, 1) gram_pipe_kernel(int n, int p, int q, const double* __restrict__ A,
-                                                               long long lda, const double* __restrict__ B,
-                                                               long long ldb, const double* __restrict__ w,
-                                                               double alpha, double* C, int ldc, int rows_per_split,
-                                                               int upper_only, int atomic) {
-  const int bi = blockIdx.x, bj = blockIdx.y;
-  if (upper_only && bi > bj) return;
-  extern __shared__ __align__(16) double gsm[];
-  const int i0 = bi * GT, j0 = bj * GT;
-  const int r0 = blockIdx.z * rows_per_split;
-  const int r1 = min(n, r0 + rows_per_split);
-  const int lane = threadIdx.x % 32, warp = threadIdx.x / 32;
-  const int wm = warp / 2, wn = warp % 2;  // warp tile: rows 32 wm .. +31, columns 64 wn .. +63
-  const int fr = lane / 4, fk = lane % 4;
-  const int nst = (r1 > r0) ? (r1 - r0 + GP_KS - 1) / GP_KS : 0;
-  // stage s: rows r0 + 16 s .. + 15; each thread copies 4 chunks of A and 4 of B (16 B = 2 rows of one column)
-  auto issue = [&](int st) {
-    double* sA = gsm + (size_t)(st % GP_STAGES) * GP_STAGE_DOUBLES;
-    double* sB = sA + GT * GP_KPAD;
-    const int kbase = r0 + st * GP_KS;
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int e = threadIdx.x + GTHREADS * u;  // 0 .. 1023: column e / 8, row pair e % 8
-      const int c = e >> 3, kp = (e & 7) * 2;
-      const int k = kbase + kp;
-      const int valid = (k < r1) ? min(2, r1 - k) : 0;
-      const int ia = i0 + c, jb = j0 + c;
-      gp_cp16(sA + c * GP_KPAD + kp, (ia < p && valid) ? A + (long long)ia * lda + k : A, ia < p ? valid : 0);
-      gp_cp16(sB + c * GP_KPAD + kp, (jb < q && valid) ? B + (long long)jb * ldb + k : B, jb < q ? valid : 0);
-    }
-  };
-  double acc[2][8][4];
-#pragma unroll
-  for (int a = 0; a < 2; ++a)
-#pragma unroll
-    for (int b = 0; b < 8; ++b)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) acc[a][b][e] = 0.0;
-#pragma unroll
-  for (int st = 0; st < GP_STAGES - 1; ++st) {
-    if (st < nst) issue(st);
-    asm volatile("cp.async.commit_group;" ::: "memory");
-  }
-  for (int st = 0; st < nst; ++st) {
-    asm volatile("cp.async.wait_group %0;" ::"n"(GP_STAGES - 2) : "memory");
-    __syncthreads();  // stage st visible to all; stage st - 1's buffer is free for the copy below
-    if (st + GP_STAGES - 1 < nst) issue(st + GP_STAGES - 1);
-    asm volatile("cp.async.commit_group;" ::: "memory");
-    const double* sA = gsm + (size_t)(st % GP_STAGES) * GP_STAGE_DOUBLES;
-    const double* sB = sA + GT * GP_KPAD;
-    const int kbase = r0 + st * GP_KS;
-#pragma unroll
-    for (int kk = 0; kk < GP_KS; kk += 8) {
-      double wa = 1.0, wb = 1.0;
-      if (w) {
-        const int ka = kbase + kk + fk, kb = ka + 4;
-        wa = ka < r1 ? __ldg(w + ka) : 0.0;
-        wb = kb < r1 ? __ldg(w + kb) : 0.0;
-      }
-      double af[2][4], bf[8][2];
-#pragma unroll
-      for (int a = 0; a < 2; ++a) {
-        const int r = 32 * wm + 16 * a + fr;
-        af[a][0] = wa * sA[r * GP_KPAD + kk + fk];
-        af[a][1] = wa * sA[(r + 8) * GP_KPAD + kk + fk];
-        af[a][2] = wb * sA[r * GP_KPAD + kk + fk + 4];
-        af[a][3] = wb * sA[(r + 8) * GP_KPAD + kk + fk + 4];
-      }
-#pragma unroll
-      for (int b = 0; b < 8; ++b) {
-        const int c = 64 * wn + 8 * b + fr;
-        bf[b][0] = sB[c * GP_KPAD + kk + fk];
-        bf[b][1] = sB[c * GP_KPAD + kk + fk + 4];
-      }
-#pragma unroll
-      for (int a = 0; a < 2; ++a)
-#pragma unroll
-        for (int b = 0; b < 8; ++b) dmma16(acc[a][b], af[a], bf[b]);
-    }
-  }
-  asm volatile("cp.async.wait_group 0;" ::: "memory");
-#pragma unroll
-  for (int a = 0; a < 2; ++a) {
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int i = i0 + 32 * wm + 16 * a + 8 * h + fr;
-      if (i >= p) continue;
-#pragma unroll
-      for (int b = 0; b < 8; ++b) {
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const int j = j0 + 64 * wn + 8 * b + 2 * fk + e;
-          if (j >= q) continue;
-          if (upper_only && i > j) continue;
-          double* dst = C + (long long)j * ldc + i;
-          const double v = alpha * acc[a][b][2 * h + e];
-          if (atomic)
-            atomicAdd(dst, v);
-          else
-            *dst += v;
-        }
-      }
-    }
-  }
-}
-
-// Whether gram_pipe_kernel can stage A and B (16-byte copies: aligned bases, even leading dimensions).
-inline bool gram_pipe_ok(const double* A, long long lda, const double* B, long long ldb) {
-  return (reinterpret_cast<uintptr_t>(A) % 16 == 0) && (reinterpret_cast<uintptr_t>(B) % 16 == 0) && lda % 2 == 0 &&
-         ldb % 2 == 0;
-}
-
-// Launch of the FP64 Gram tiles (pipelined when the operands allow it), grid (tp, tq, splits).
-int launch_gram64(db200_context* ctx, dim3 grid, int n, int p, int q, const double* A, long long lda, const double* B,
-                  long long ldb, const double* w, double alpha, double* C, int ldc, int rows, bool upper_only,
-                  bool atomic) {
-  if (gram_pipe_ok(A, lda, B, ldb)) {
-    DB200_CUDA(ctx, cudaFuncSetAttribute(gram_pipe_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)GP_SMEM));
-    gram_pipe_kernel<<<grid, GTHREADS, GP_SMEM, ctx->stream>>>(n, p, q, A, lda, B, ldb, w, alpha, C, ldc, rows,
-                                                               upper_only ? 1 : 0, atomic ? 1 : 0);
-  } else {
-    gram_kernel<double, double><<<grid, GTHREADS, 0, ctx->stream>>>(n, p, q, A, lda, B, ldb, w, alpha, C, ldc, rows,
-                                                                    upper_only ? 1 : 0, atomic ? 1 : 0);
-  }
-  DB200_CUDA(ctx, cudaGetLastError());
-  count_launch(ctx);
-  return DB200_OK;
-}
-
-// C[n x q] = alpha * A[n x p] * op(B) + beta * C (op(B) = B, p x q, or B^T with B q x p when transB) on the FP64
-// tensor cores: one 128 x 128 tile of C per CTA with the whole reduction over p inside it, the warp layout and
-// m16n8k8 fragments of gram_kernel.  Stages of 8 columns of A (128 contiguous rows each, one coalesced 256-byte
-// read per warp and column) and 8 rows of op(B) are fetched into registers one stage ahead and parked k-major in
-// a double-buffered shared tile.
-template <typename TA, typename TC>
-__global__ void __launch_bounds__(GTHREADS, 1) tall_kernel(int n, int p, int q, const TA* __restrict__ A, long long lda,
-                                                           const double* __restrict__ B, int ldb, int transB,
-                                                           double alpha, double beta, TC* C, long long ldc) {
-  const int i0 = blockIdx.x * GT, j0 = blockIdx.y * GT;
-  __shared__ __align__(16) double sA[2][GK][GPAD];
-  __shared__ __align__(16) double sB[2][GK][GPAD];
-  const int lane = threadIdx.x % 32, warp = threadIdx.x / 32;
-  const int wm = warp / 2, wn = warp % 2;
-  const int fr = lane / 4, fk = lane % 4;
-  double acc[2][8][4];
-#pragma unroll
-  for (int a = 0; a < 2; ++a)
-#pragma unroll
-    for (int b = 0; b < 8; ++b)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) acc[a][b][e] = 0.0;
-  // A: column k0 + ak, rows i0 + ar + 32 s.  op(B): row k0 + bk, columns j0 + bj + 32 s (B^T rows are contiguous
-  // in j, B's columns contiguous in k: consecutive threads walk the contiguous index either way).
-  const int ak = threadIdx.x / 32, ar = threadIdx.x % 32;
-  const int bk = transB ? threadIdx.x / 32 : threadIdx.x % GK;
-  const int bj = transB ? threadIdx.x % 32 : threadIdx.x / GK;
-  double va[4], vb[4];
-  auto fetch = [&](int k0) {
-    const int ka = k0 + ak, kb = k0 + bk;
-#pragma unroll
-    for (int s = 0; s < 4; ++s) {
-      const int i = i0 + ar + 32 * s, j = j0 + bj + 32 * s;
-      va[s] = (ka < p && i < n) ? ld64(A + (long long)ka * lda + i) : 0.0;
-      vb[s] = (kb < p && j < q) ? (transB ? B[(long long)kb * ldb + j] : B[(long long)j * ldb + kb]) : 0.0;
-    }
-  };
-  auto park = [&](int buf) {
-#pragma unroll
-    for (int s = 0; s < 4; ++s) {
-      sA[buf][ak][ar + 32 * s] = va[s];
-      sB[buf][bk][bj + 32 * s] = vb[s];
-    }
-  };
-  int buf = 0;
-  fetch(0);
-  park(0);
-  __syncthreads();
-  for (int k0 = 0; k0 < p; k0 += GK) {
-    const bool more = k0 + GK < p;
-    if (more) fetch(k0 + GK);
-    {
-      double af[2][4], bf[8][2];
-#pragma unroll
-      for (int a = 0; a < 2; ++a) {
-        const int r = 32 * wm + 16 * a + fr;
-        af[a][0] = sA[buf][fk][r];
-        af[a][1] = sA[buf][fk][r + 8];
-        af[a][2] = sA[buf][fk + 4][r];
-        af[a][3] = sA[buf][fk + 4][r + 8];
-      }
-#pragma unroll
-      for (int b = 0; b < 8; ++b) {
-        const int c = 64 * wn + 8 * b + fr;
-        bf[b][0] = sB[buf][fk][c];
-        bf[b][1] = sB[buf][fk + 4][c];
-      }
-#pragma unroll
-      for (int a = 0; a < 2; ++a)
-#pragma unroll
-        for (int b = 0; b < 8; ++b) dmma16(acc[a][b], af[a], bf[b]);
-    }
-    if (more) park(buf ^ 1);
-    __syncthreads();
-    buf ^= 1;
-  }
-#pragma unroll
-  for (int a = 0; a < 2; ++a) {
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int i = i0 + 32 * wm + 16 * a + 8 * h + fr;
-      if (i >= n) continue;
-#pragma unroll
-      for (int b = 0; b < 8; ++b) {
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const int j = j0 + 64 * wn + 8 * b + 2 * fk + e;
-          if (j >= q) continue;
-          TC* dst = C + (long long)j * ldc + i;
-          double v = alpha * acc[a][b][2 * h + e];
-          if (beta != 0.0) v += beta * (double)*dst;
-          *dst = (TC)v;
-        }
-      }
-    }
-  }
-}
+// The Cholesky's trailing matrix takes whole DMM tiles once it holds a wave of them (128 x 128 upper tiles).
+constexpr int GT = 128;
 
 // One block column of the right-looking blocked upper Cholesky: the kb x kb diagonal block (kb <= 64) is factored
 // in every CTA (redundantly; 64 steps with one barrier each, the block's elements in registers, only a reciprocal
@@ -581,24 +210,46 @@ __global__ void zero_lower_kernel(double* A, int lda, int l) {
   }
 }
 
-// X = R^-1 for upper triangular R (l x l): one warp per column j solves R x = e_j by column-oriented
-// back substitution.
-__global__ void trinv_upper_kernel(const double* R, int ldr, int l, double* X, int ldx) {
-  const int warps = blockDim.x / 32;
-  const int j = blockIdx.x * warps + threadIdx.x / 32;
-  const int lane = threadIdx.x % 32;
-  if (j >= l) return;
-  double* x = X + (long long)j * ldx;
-  for (int i = lane; i < l; i += 32) x[i] = (i == j) ? 1.0 : 0.0;
-  __syncwarp();
-  for (int i = j; i >= 0; --i) {
-    const double xi = x[i] / R[(long long)i * ldr + i];
-    __syncwarp();
-    if (lane == 0) x[i] = xi;
-    const double* ri = R + (long long)i * ldr;
-    for (int k = lane; k < i; k += 32) x[k] -= ri[k] * xi;
-    __syncwarp();
+// Diagonal blocks of X = R^-1 (upper triangular, l x l): one warp per 32 x 32 block, lane j holding column j of the
+// block's inverse in registers (column-oriented back substitution; R's columns are read from shared memory as
+// broadcasts).  Rows and columns past l behave as identity and are not stored.
+constexpr int TI = 32;
+constexpr int TI_WARPS = 4;
+__global__ void __launch_bounds__(32 * TI_WARPS) trinv_diag_kernel(const double* R, int ldr, int l, double* X,
+                                                                   int ldx) {
+  __shared__ double sR[TI_WARPS][TI][TI + 1];  // column i of the block at sR[i]
+  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+  const int r0 = (blockIdx.x * TI_WARPS + warp) * TI;
+  if (r0 >= l) return;
+  double(*S)[TI + 1] = sR[warp];
+#pragma unroll 4
+  for (int i = 0; i < TI; ++i) {
+    const bool in = r0 + i < l && r0 + lane < l;
+    S[i][lane] = in ? R[(long long)(r0 + i) * ldr + r0 + lane] : (i == lane ? 1.0 : 0.0);
   }
+  __syncwarp();
+  double x[TI];
+#pragma unroll
+  for (int i = 0; i < TI; ++i) x[i] = (i == lane) ? 1.0 : 0.0;
+#pragma unroll
+  for (int i = TI - 1; i >= 0; --i) {
+    x[i] = x[i] / S[i][i];
+#pragma unroll
+    for (int k = 0; k < i; ++k) x[k] = fma(-S[i][k], x[i], x[k]);
+  }
+  if (r0 + lane < l) {
+    double* col = X + (long long)(r0 + lane) * ldx + r0;
+#pragma unroll
+    for (int i = 0; i < TI; ++i)
+      if (r0 + i < l) col[i] = x[i];
+  }
+}
+
+// Clears the rows below the diagonal of every block pair (blockIdx.y) of trinv_upper's level h.
+__global__ void trinv_clear_kernel(double* X, int ldx, int l, int h) {
+  const int r0 = 2 * h * (int)blockIdx.y, q = min(h, l - r0 - h);
+  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < q * h; e += gridDim.x * blockDim.x)
+    X[(long long)(r0 + e / q) * ldx + r0 + h + e % q] = 0.0;
 }
 
 // Single-CTA triangular solves with an upper factor R (and its transpose L = R^T stored separately so every
@@ -794,22 +445,6 @@ __global__ void sumsq_f32_kernel(const float* A, long long lda, int m, int n, do
   }
 }
 
-// FP64 kernel block from a Gram block: K[i + j*ldk] = yi_i yj_j exp(-gamma max(si_i + sj_j - 2 G, 0)) in place
-// (G = Xi^T Xj formed by the FP64 Gram kernel); the comparator arithmetic of include/dkernel.cu:116-129 in FP64.
-__global__ void rbf_from_gram_f64_kernel(double* K, long long ldk, int m, int n, const double* si, const double* sj,
-                                         const float* yi, const float* yj, double gamma) {
-  const long long total = (long long)m * n;
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total; e += (long long)gridDim.x * blockDim.x) {
-    const int i = (int)(e % m), j = (int)(e / m);
-    double* k = K + j * ldk + i;
-    const double d2 = fmax(si[i] + sj[j] - 2.0 * *k, 0.0);
-    double v = exp(-gamma * d2);
-    if (yi) v *= (double)yi[i];
-    if (yj) v *= (double)yj[j];
-    *k = v;
-  }
-}
-
 // s_i = sum_k x_ik^2 in FP64 for point-major X (d x n, ldx): vecnorm (include/dkernel.cu:102-114) in FP64
 __global__ void rownorm_f64_kernel(const float* X, long long ldx, int n, int d, double* s) {
   const int lane = threadIdx.x % 32;
@@ -933,38 +568,29 @@ int gram(db200_context* ctx, int n, int p, int q, const TA* A, long long lda, co
   scale_kernel<<<grid_for((long long)p * q, 256, 4096), 256, 0, ctx->stream>>>(C, ldc, p, q, beta, upper_only ? 1 : 0);
   count_launch(ctx);
   if (n <= 0) return DB200_OK;
-  const int tp = (p + GT - 1) / GT, tq = (q + GT - 1) / GT;
-  const int tiles = upper_only ? (tp * (tp + 1)) / 2 : tp * tq;
-  // row splits: fill whole waves of one CTA per SM (at least two waves' worth of CTAs)
-  int splits = 1;
-  {
-    const int sms = ctx->num_sms;
-    int best = 1;
-    double best_eff = -1.0;
-    for (int waves = 2; waves <= 8; ++waves) {
-      const int sp = (waves * sms) / tiles;
-      if (sp < 1) continue;
-      const long long ctas = (long long)sp * tiles;
-      const double eff = (double)ctas / (double)(((ctas + sms - 1) / sms) * sms);
-      if (eff > best_eff + 1e-9) {
-        best_eff = eff;
-        best = sp;
-      }
-    }
-    splits = best;
-  }
-  int rows = (n + splits - 1) / splits;
-  rows = round_up(rows < GK ? GK : rows, GK);
-  splits = (n + rows - 1) / rows;
-  if (splits > 65535) return fail(ctx, DB200_ERR_UNSUPPORTED, "gram: too many row splits");
-  dim3 grid(tp, tq, splits);
-  if constexpr (std::is_same<TA, double>::value && std::is_same<TBt, double>::value)
-    return launch_gram64(ctx, grid, n, p, q, A, lda, B, ldb, w, alpha, C, ldc, rows, upper_only, splits > 1);
-  gram_kernel<TA, TBt><<<grid, GTHREADS, 0, ctx->stream>>>(n, p, q, A, lda, B, ldb, w, alpha, C, ldc, rows,
-                                                     upper_only ? 1 : 0, splits > 1 ? 1 : 0);
-  DB200_CUDA(ctx, cudaGetLastError());
-  count_launch(ctx);
-  return DB200_OK;
+  DmmArgs g;
+  g.m = p;
+  g.q = q;
+  g.p = n;
+  g.A = A;
+  g.lda = lda;
+  g.B = B;
+  g.ldb = ldb;
+  g.w = w;
+  g.alpha = alpha;
+  g.C = C;
+  g.ldc = ldc;
+  g.upper = upper_only ? 1 : 0;
+  // Row splits, added with FP64 atomics: about eight waves of two CTAs per SM (upper tiles carry unequal strips, so
+  // several waves are needed for the SMs to end together: with four, the busiest SM had 0.77 of its tensor pipe in use
+  // and the idlest 0.55), no split shorter than 64 rows (a CTA's prologue and its atomics then outweigh its stages).
+  const long long tp = (p + DMM_BM - 1) / DMM_BM, tq = (q + 63) / 64;
+  const long long tiles = upper_only ? std::max(1LL, tp * tq / 2 + tp) : tp * tq;
+  int splits = (int)std::max(1LL, std::min((long long)n / 64, 16LL * ctx->num_sms / tiles));
+  g.kps = round_up((n + splits - 1) / splits, DMM_KS);
+  splits = (n + g.kps - 1) / g.kps;
+  g.epi = splits > 1 ? DMM_ATOMIC : DMM_ADD;
+  return dmm_launch<TA, TBt, double, true, true>(ctx, g, splits);
 }
 
 template int gram<float, float>(db200_context*, int, int, int, const float*, long long, const float*, long long,
@@ -976,25 +602,50 @@ template int gram<double, float>(db200_context*, int, int, int, const double*, l
 
 template <typename TA, typename TC>
 int gemm_tall(db200_context* ctx, int n, int p, int q, const TA* A, long long lda, const double* B, int ldb,
-              bool transB, double beta, TC* C, long long ldc, double alpha) {
+              bool transB, double beta, TC* C, long long ldc, double alpha, int tri) {
   if (n <= 0 || q <= 0) return DB200_OK;
-  dim3 grid((n + GT - 1) / GT, (q + GT - 1) / GT);
-  if (grid.y > 65535) return fail(ctx, DB200_ERR_UNSUPPORTED, "gemm_tall: q too large");
-  tall_kernel<TA, TC><<<grid, GTHREADS, 0, ctx->stream>>>(n, p, q, A, lda, B, ldb, transB ? 1 : 0, alpha, beta, C,
-                                                          ldc);
-  DB200_CUDA(ctx, cudaGetLastError());
-  count_launch(ctx);
-  return DB200_OK;
+  DmmArgs g;
+  g.m = n;
+  g.q = q;
+  g.p = p;
+  g.A = A;
+  g.lda = lda;
+  g.B = B;
+  g.ldb = ldb;
+  g.alpha = alpha;
+  g.beta = beta;
+  g.C = C;
+  g.ldc = ldc;
+  g.tri = tri;
+  return transB ? dmm_launch<TA, double, TC, false, false>(ctx, g) : dmm_launch<TA, double, TC, false, true>(ctx, g);
 }
 
 template int gemm_tall<float, double>(db200_context*, int, int, int, const float*, long long, const double*, int,
-                                      bool, double, double*, long long, double);
+                                      bool, double, double*, long long, double, int);
 template int gemm_tall<double, double>(db200_context*, int, int, int, const double*, long long, const double*, int,
-                                       bool, double, double*, long long, double);
+                                       bool, double, double*, long long, double, int);
 template int gemm_tall<double, float>(db200_context*, int, int, int, const double*, long long, const double*, int,
-                                      bool, double, float*, long long, double);
+                                      bool, double, float*, long long, double, int);
 template int gemm_tall<float, float>(db200_context*, int, int, int, const float*, long long, const double*, int,
-                                     bool, double, float*, long long, double);
+                                     bool, double, float*, long long, double, int);
+
+// C (p x q, upper entries only) -= P^T P' for the k rows of a factored panel, in place (the Cholesky's updates)
+static int syrk_update(db200_context* ctx, int k, int p, int q, const double* P, int ldp, double* C, int ldc) {
+  DmmArgs g;
+  g.m = p;
+  g.q = q;
+  g.p = k;
+  g.A = P;
+  g.lda = ldp;
+  g.B = P;
+  g.ldb = ldp;
+  g.alpha = -1.0;
+  g.C = C;
+  g.ldc = ldc;
+  g.upper = 1;
+  g.epi = DMM_ADD;
+  return dmm_launch<double, double, double, true, true>(ctx, g);
+}
 
 int potrf_upper(db200_context* ctx, double* A, int lda, int l, int* d_status, int* d_bad, int nb) {
   if (nb < 1 || nb > 64) nb = 64;
@@ -1030,8 +681,7 @@ int potrf_upper(db200_context* ctx, double* A, int lda, int l, int* d_status, in
       if (pr > 0) {
         const double* P = A + (long long)(k0 + kb) * lda + k0;
         double* C = A + (long long)(k0 + kb) * lda + k0 + kb;
-        const int s2 = launch_gram64(ctx, dim3((pr + GT - 1) / GT, (rest + GT - 1) / GT, 1), kb, pr, rest, P, lda, P,
-                                     lda, nullptr, -1.0, C, lda, kb, true, false);
+        const int s2 = syrk_update(ctx, kb, pr, rest, P, lda, C, lda);
         if (s2) return s2;
       }
     }
@@ -1041,9 +691,7 @@ int potrf_upper(db200_context* ctx, double* A, int lda, int l, int* d_status, in
       const double* P = A + (long long)(K0 + KB) * lda + K0;
       double* C = A + (long long)(K0 + KB) * lda + K0 + KB;
       if (KB > nb || big(rest)) {
-        const int tp = (rest + GT - 1) / GT;
-        const int s2 = launch_gram64(ctx, dim3(tp, tp, 1), KB, rest, rest, P, lda, P, lda, nullptr, -1.0, C, lda, KB,
-                                     true, false);
+        const int s2 = syrk_update(ctx, KB, rest, rest, P, lda, C, lda);
         if (s2) return s2;
       } else {
         // the r ~ 500..2000 capacity factors of the barrier: 32 x 32 tiles, so that they spread over the GPU
@@ -1060,10 +708,53 @@ int potrf_upper(db200_context* ctx, double* A, int lda, int l, int* d_status, in
   return DB200_OK;
 }
 
+// X = R^-1 by block doubling: the 32 x 32 diagonal blocks, then for half = 32, 64, 128, ... every pair of inverted
+// blocks X11, X22 (the second one possibly shorter) becomes one with X12 = -X11 R12 X22, two batched products per
+// level on the FP64 tensor cores.  The first product is kept transposed, T^T = (R12 X22)^T, in the pair's place
+// below the diagonal (q x half, exactly its shape), cleared before the next level reads the blocks.  One warp per column doing its own
+// back substitution over global memory (the form before) took 1.01 ms at l = 528 and 3.4 ms at l = 1024, a chain of l
+// dependent memory round trips; the levels are log2(l / 32) pairs of launches.
 int trinv_upper(db200_context* ctx, const double* R, int ldr, int l, double* X, int ldx) {
-  trinv_upper_kernel<<<(l + 7) / 8, 256, 0, ctx->stream>>>(R, ldr, l, X, ldx);
+  trinv_diag_kernel<<<(l + TI * TI_WARPS - 1) / (TI * TI_WARPS), 32 * TI_WARPS, 0, ctx->stream>>>(R, ldr, l, X, ldx);
   DB200_CUDA(ctx, cudaGetLastError());
   count_launch(ctx);
+  for (int h = TI; h < l; h *= 2) {
+    const int pairs = (l - h + 2 * h - 1) / (2 * h);  // pairs whose second half is not empty
+    const int widest = std::min(h, l - h);            // rows of the longest second half
+    const long long sr = 2LL * h * (ldr + 1LL), sx = 2LL * h * (ldx + 1LL);
+    DmmArgs g;
+    g.bl = l;
+    g.bs = h;
+    g.ldc = ldx;
+    g.sC = sx;
+    // T^T (q x h) = X22^T R12^T
+    g.m = g.p = widest;
+    g.q = h;
+    g.vary = 1;
+    g.A = X + h * (ldx + 1LL);
+    g.lda = ldx;
+    g.sA = sx;
+    g.B = R + (long long)h * ldr;
+    g.ldb = ldr;
+    g.sB = sr;
+    g.C = X + h;
+    int st = dmm_launch<double, double, double, true, false>(ctx, g, 1, pairs);
+    if (st) return st;
+    // X12 (h x q) = -X11 T
+    g.m = g.p = h;
+    g.q = widest;
+    g.vary = 2;
+    g.A = X;
+    g.B = X + h;
+    g.ldb = ldx;
+    g.sB = sx;
+    g.C = X + (long long)h * ldx;
+    g.alpha = -1.0;
+    if ((st = dmm_launch<double, double, double, false, false>(ctx, g, 1, pairs))) return st;
+    trinv_clear_kernel<<<dim3(grid_for((long long)h * widest, 256, 128), pairs), 256, 0, ctx->stream>>>(X, ldx, l, h);
+    DB200_CUDA(ctx, cudaGetLastError());
+    count_launch(ctx);
+  }
   return DB200_OK;
 }
 
@@ -1133,13 +824,29 @@ int sumsq_f32(db200_context* ctx, const float* A, long long lda, int m, int n, d
   return DB200_OK;
 }
 
-int rbf_from_gram_f64(db200_context* ctx, double* K, long long ldk, int m, int n, const double* si, const double* sj,
-                      const float* yi, const float* yj, double gamma) {
-  rbf_from_gram_f64_kernel<<<grid_for((long long)m * n, 256, 16 * ctx->num_sms), 256, 0, ctx->stream>>>(
-      K, ldk, m, n, si, sj, yi, yj, gamma);
-  DB200_CUDA(ctx, cudaGetLastError());
-  count_launch(ctx);
-  return DB200_OK;
+// The FP64 kernel block in one launch: cross terms on the FP64 tensor cores over the d features, the norms, exp and
+// labels in the epilogue, K written once.  Bound by the d-long products and the exp (131072 x 1024, d = 64: 0.46 ms
+// of tensor pipe, 0.17 ms of stores); clearing K, a Gram added into it and a second pass over it took 3.4 ms.
+int rbf_block_f64_fused(db200_context* ctx, int m, int n, int d, const float* Xi, long long ldxi, const float* Xj,
+                        long long ldxj, const double* si, const double* sj, const float* yi, const float* yj,
+                        double gamma, double* K, long long ldk) {
+  DmmArgs g;
+  g.m = m;
+  g.q = n;
+  g.p = d;
+  g.A = Xi;
+  g.lda = ldxi;
+  g.B = Xj;
+  g.ldb = ldxj;
+  g.C = K;
+  g.ldc = ldk;
+  g.epi = DMM_RBF;
+  g.si = si;
+  g.sj = sj;
+  g.yi = yi;
+  g.yj = yj;
+  g.gamma = gamma;
+  return dmm_launch<float, float, double, true, true>(ctx, g);
 }
 
 int rownorm_f64(db200_context* ctx, const float* X, long long ldx, int n, int d, double* s) {

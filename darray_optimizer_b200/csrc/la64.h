@@ -10,10 +10,13 @@ template <typename TA, typename TBt>
 int gram(db200_context* ctx, int n, int p, int q, const TA* A, long long lda, const TBt* B, long long ldb,
          const double* w, double alpha, double beta, double* C, int ldc, bool upper_only);
 
-// C[n x q] = A[n x p] * op(B) + beta * C,  op(B) = B (p x q, ldb) or B^T (B stored q x p) when transB.
+enum { kFullB = 0, kUpperB = 1, kLowerB = 2 };  // op(B) of gemm_tall: full, upper or lower triangular
+
+// C[n x q] = A[n x p] * op(B) + beta * C,  op(B) = B (p x q, ldb) or B^T (B stored q x p) when transB.  tri: op(B) is
+// upper (kUpperB) or lower (kLowerB) triangular with exact zeros, which are not multiplied.
 template <typename TA, typename TC>
 int gemm_tall(db200_context* ctx, int n, int p, int q, const TA* A, long long lda, const double* B, int ldb,
-              bool transB, double beta, TC* C, long long ldc, double alpha = 1.0);
+              bool transB, double beta, TC* C, long long ldc, double alpha = 1.0, int tri = 0);
 
 // In-place upper Cholesky (A = R^T R) with block size nb <= 64; the strictly lower part is zeroed.  A
 // non-positive pivot sets *d_status = DB200_ERR_NOT_SPD and *d_bad = first row of the failing block.
@@ -45,9 +48,10 @@ int axpby_f32(db200_context* ctx, float* C, long long ldc, const double* T, long
               double alpha, double beta);
 // *d_out += sum of squares of an m x n float block
 int sumsq_f32(db200_context* ctx, const float* A, long long lda, int m, int n, double* d_out);
-// K = yi yj exp(-gamma max(si + sj - 2 G, 0)) in place over an m x n FP64 Gram block
-int rbf_from_gram_f64(db200_context* ctx, double* K, long long ldk, int m, int n, const double* si, const double* sj,
-                      const float* yi, const float* yj, double gamma);
+// K(i, j) = yi yj exp(-gamma max(si + sj - 2 x_i.x_j, 0)) in FP64 for point-major float points (norms si, sj given)
+int rbf_block_f64_fused(db200_context* ctx, int m, int n, int d, const float* Xi, long long ldxi, const float* Xj,
+                        long long ldxj, const double* si, const double* sj, const float* yi, const float* yj,
+                        double gamma, double* K, long long ldk);
 // FP64 squared norms of the n points of a point-major float matrix
 int rownorm_f64(db200_context* ctx, const float* X, long long ldx, int n, int d, double* s);
 // Fused FP64 RBF x sketch (rbf64.cu): Y = diag(yi) K(Xi, Xj) diag(yj) Omega, FP64 throughout, K never stored.

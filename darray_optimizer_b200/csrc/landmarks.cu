@@ -605,7 +605,7 @@ int db200_ridge_leverage(db200_context* ctx, int n, int r, const double* Z, int 
   DB200_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   if (hs[0]) return fail(ctx, DB200_ERR_NOT_SPD, "ridge_leverage: Z^T Z + lambda I not positive definite");
   if ((st = trinv_upper(ctx, G, r, r, Xi, r))) return st;
-  if ((st = gemm_tall<double, double>(ctx, n, r, r, Z, ldz, Xi, r, false, 0.0, W, n))) return st;
+  if ((st = gemm_tall<double, double>(ctx, n, r, r, Z, ldz, Xi, r, false, 0.0, W, n, 1.0, kUpperB))) return st;
   row_sumsq64_kernel<<<blocks_for(n, 256, 4096), 256, 0, ctx->stream>>>(n, r, W, n, lev);
   DB200_CUDA(ctx, cudaGetLastError());
   count_launch(ctx);
@@ -878,7 +878,7 @@ static int landmark_factor_impl(db200_context* ctx, int n, int d, const float* X
   if (!ok) return fail(ctx, DB200_ERR_NOT_SPD, "landmark_factor: K(L, L) + nu I not positive definite after 12 shifts");
   // Z = C R^-1
   if ((st = trinv_upper(ctx, R, r, r, Xinv, r))) return st;
-  if ((st = gemm_tall<TC, double>(ctx, n, r, r, Cm, n, Xinv, r, false, 0.0, Z, ldz))) return st;
+  if ((st = gemm_tall<TC, double>(ctx, n, r, r, Cm, n, Xinv, r, false, 0.0, Z, ldz, 1.0, kUpperB))) return st;
   if (nu_out) *nu_out = nu;
   return db200_synchronize(ctx);
 }

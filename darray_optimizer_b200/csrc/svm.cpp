@@ -107,7 +107,7 @@ int cholqr_pass(db200_context* ctx, int n, int l, const double* Yin, int ldin, d
   if (pst) return fail(ctx, DB200_ERR_NOT_SPD, "CholeskyQR: Gram matrix not positive definite at row " +
                                                    std::to_string(bad));
   if ((st = trinv_upper(ctx, R, l, l, Rinv, l))) return st;
-  return gemm_tall<double, double>(ctx, n, l, l, Yin, ldin, Rinv, l, false, 0.0, Yout, ldout);
+  return gemm_tall<double, double>(ctx, n, l, l, Yin, ldin, Rinv, l, false, 0.0, Yout, ldout, 1.0, kUpperB);
 }
 
 }  // namespace
@@ -148,13 +148,13 @@ int cholqr2_impl(db200_context* ctx, int n, int l, double* Y, int ldy, double* R
   // second pass T -> Y
   if ((st = cholqr_pass(ctx, n, l, T, n, Y, ldy, R2, Rinv, 0.0, d_pair, d_scalar, tc_gram, dist))) return st;
   // R = R2 R1 (upper * upper)
-  if ((st = gemm_tall<double, double>(ctx, l, l, l, R2, l, R1, l, false, 0.0, Racc, l))) return st;
+  if ((st = gemm_tall<double, double>(ctx, l, l, l, R2, l, R1, l, false, 0.0, Racc, l, 1.0, kUpperB))) return st;
   if (shifted) {
     // third pass Y -> T, then copy back; R = R3 (R2 R1)
     if ((st = cholqr_pass(ctx, n, l, Y, ldy, T, n, R3, Rinv, 0.0, d_pair, d_scalar, tc_gram, dist))) return st;
     DB200_CUDA(ctx, cudaMemcpy2DAsync(Y, sizeof(double) * ldy, T, sizeof(double) * n, sizeof(double) * n, l,
                                       cudaMemcpyDeviceToDevice, ctx->stream));
-    if ((st = gemm_tall<double, double>(ctx, l, l, l, R3, l, Racc, l, false, 0.0, R1, l))) return st;
+    if ((st = gemm_tall<double, double>(ctx, l, l, l, R3, l, Racc, l, false, 0.0, R1, l, 1.0, kUpperB))) return st;
     Racc = R1;
   }
   if (Rout) {
@@ -723,7 +723,7 @@ int nystrom_core(db200_context* ctx, int n, int l, const double* Q, const TY* Yk
   }
   if (!ok) return fail(ctx, DB200_ERR_NOT_SPD, "lowrank: Q^T K Q + nu I not positive definite after 12 shifts");
   // Z = Q R^T
-  if ((st = gemm_tall<double, double>(ctx, n, l, l, Q, n, R, l, true, 0.0, Z, ldz))) return st;
+  if ((st = gemm_tall<double, double>(ctx, n, l, l, Q, n, R, l, true, 0.0, Z, ldz, 1.0, kLowerB))) return st;
   if (nu_out) *nu_out = nu;
   return DB200_OK;
 }
