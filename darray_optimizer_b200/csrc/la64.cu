@@ -10,6 +10,7 @@
 #include "dmm64.cuh"
 #include "internal.h"
 #include "la64.h"
+#include "potrf64.cuh"
 
 namespace db200 {
 
@@ -19,147 +20,50 @@ namespace {
 constexpr int GT = 128;
 
 // One block column of the right-looking blocked upper Cholesky: the kb x kb diagonal block (kb <= 64) is factored
-// in every CTA (redundantly; 64 steps with one barrier each, the block's elements in registers, only a reciprocal
-// of the pivot on the sequential path, the row scaling by 1/sqrt(pivot) done for all rows afterwards), the last CTA
-// to have staged the block writes R11 back (zeros below its diagonal), and CTA c >= 1 overwrites the 64 panel
-// columns [k0 + kb + 64 (c - 1), +64) with R11^-T A12 by forward substitution (one warp per 8 columns, the
-// solution held two rows per lane and broadcast by shuffles).  The write-back waits for nothing: every CTA counts
-// itself in `arrivals` after staging A11, and the CTA that arrives last, when every other CTA has read A11, is
-// the one that overwrites it (and re-arms the counter for the next launch).  On a non-positive or NaN pivot
-// nothing is written, status <- DB200_ERR_NOT_SPD and *bad <- k0 (first failing block).  A block column after a
-// failed one writes nothing.  Follows cholesky_factorize (include/lapack_like.h:10-57): potrf of the diagonal
-// block, trsm of the panel, syrk of the trailing matrix (the DMMA gram_kernel or syrk_update_kernel launched after
-// this one).
-__global__ void __launch_bounds__(256) potrf_block_kernel(double* A, int lda, int k0, int kb, int l, int* status,
-                                                          int* bad, int* arrivals) {
-  __shared__ double rs[64][65];  // staging, then R11 (row-major: rs[i][j] = R[k0 + i][k0 + j])
-  __shared__ double rowk[2][64];
-  __shared__ double inv[64];
-  __shared__ double dsq[64];
-  __shared__ int writer;
-  const int t = threadIdx.x;
-  // stage the diagonal block coalesced (column j contiguous in i)
-  for (int e = t; e < 64 * 64; e += 256) {
-    const int i = e & 63, j = e >> 6;
-    rs[i][j] = (i < kb && j < kb && i <= j) ? A[(long long)(k0 + j) * lda + k0 + i] : 0.0;
+// in every CTA (redundantly), whose other four warps solve 64 columns of the block row, the columns
+// [k0 + kb + 64 blockIdx.x, +64), at the same time (p64_run, potrf64.cuh).  The last CTA to have read the block writes
+// R11 back (zeros below its diagonal), and that write waits for nothing: every CTA counts itself in `arrivals` after
+// its reads of A11, and the CTA that arrives last, when every other one has read A11, is the one that overwrites
+// it (and re-arms the counter for the next launch).  On a non-positive or NaN pivot nothing is written, status <-
+// DB200_ERR_NOT_SPD and *bad <- k0 (first failing block).  A block column after a failed one writes nothing.  Follows
+// cholesky_factorize (include/lapack_like.h:10-57): potrf of the diagonal block, trsm of the panel, syrk of the
+// trailing matrix (launched after this one).
+template <bool VEC>
+__global__ void __launch_bounds__(P64_THREADS) potrf_block_kernel(double* A, int lda, int k0, int kb, int l,
+                                                                  int* status, int* bad, int* arrivals) {
+  extern __shared__ __align__(16) unsigned char raw[];
+  P64Smem& S = *reinterpret_cast<P64Smem*>(raw);
+  const int t = threadIdx.x, warp = t / 32;
+  int group = warp, col = k0 + 16 * warp, cl = k0 + kb;
+  if (warp >= 4) {
+    col = k0 + kb + 64 * (int)blockIdx.x + 16 * (warp - 4);
+    cl = l;
+    group = col < l ? warp : -1;
   }
+  double acc[8][4];
+  if (group >= 0) p64_load<VEC>(acc, A, lda, k0, kb, col, cl, warp < 4 ? warp : -1);
   __syncthreads();  // this CTA's reads of A11 are done
   if (t == 0) {
     __threadfence();
     const int before = atomicAdd(arrivals, 1);
-    writer = (before == (int)gridDim.x - 1);
-    if (writer) *arrivals = 0;  // every CTA has arrived: re-armed for the next launch
+    S.flag = (before == (int)gridDim.x - 1);
+    if (S.flag) *arrivals = 0;  // every CTA has arrived: re-armed for the next launch
+    __threadfence();
   }
-  __syncthreads();
   if (*(volatile int*)status) return;  // an earlier block column failed (checked after counting in)
-  // Thread t owns column j = t & 63 and the rows rg + 4 q.  The 64 steps run as 16 groups of 4 (a rolled loop, so
-  // that the kernel's code stays small: fully unrolled it missed the instruction cache most of the time when it ran
-  // between other kernels); the owners of the group's rows 4 kk .. 4 kk + 3 hold them in a[0], and after each
-  // group every thread shifts its column down by one row slot (a[q] holds row rg + 4 (q + kk)), so that no register
-  // is indexed at run time.
-  const int j = t & 63, rg = t >> 6;
-  double a[16];
-#pragma unroll
-  for (int q = 0; q < 16; ++q) a[q] = rs[rg + 4 * q][j];
-  bool failed = false;
-#pragma unroll 1
-  for (int kk = 0; 4 * kk < kb && !failed; ++kk) {
-#pragma unroll
-    for (int kr = 0; kr < 4; ++kr) {
-      const int k = 4 * kk + kr;
-      if (k >= kb) break;
-      const double own = a[0];  // row k's element of column j for its owners (rg == kr)
-      if (rg == kr) rowk[k & 1][j] = own;
-      __syncthreads();  // row k published; also orders the staging reads before the first rs write below
-      const double piv = rowk[k & 1][k];
-      if (!(piv > 0.0)) {  // the same value in every thread: a uniform exit
-        failed = true;
-        break;
-      }
-      const double u = 1.0 / piv;
-      const double ckj = rowk[k & 1][j] * u;
-#pragma unroll
-      for (int q = 0; q < 16; ++q) {
-        const int i = rg + 4 * (q + kk);
-        if (i > k && i < 64) a[q] -= rowk[k & 1][i] * ckj;  // i > j entries are never read back
-      }
-      if (rg == kr) rs[k][j] = (j >= k) ? own : 0.0;  // row k as eliminated (pivot at j == k)
-    }
-#pragma unroll
-    for (int q = 0; q < 15; ++q) a[q] = a[q + 1];
-    a[15] = 0.0;
-  }
-  if (failed) {
+  const bool ok = p64_run(S, acc, group);
+  const bool writer = S.flag != 0;  // visible: p64_run passed a barrier
+  if (!ok) {
     if (writer && t == 0 && atomicCAS(status, 0, DB200_ERR_NOT_SPD) == 0) *bad = k0;
     return;
   }
-  // R[k][j] = a_kj / sqrt(a_kk), off the sequential path: square roots first, then every row in parallel
-  __syncthreads();
-  if (t < kb) {
-    const double sd = sqrt(rs[t][t]);
-    dsq[t] = sd;
-    inv[t] = 1.0 / sd;
-  }
-  __syncthreads();
-  for (int e = t; e < kb * 64; e += 256) {
-    const int i = e >> 6, jj = e & 63;
-    if (jj > i) rs[i][jj] /= dsq[i];
-  }
-  __syncthreads();
-  if (t < kb) rs[t][t] = dsq[t];
-  __syncthreads();
   if (writer) {
-    for (int e = t; e < kb * 64; e += 256) {
-      const int i = e & 63, jj = e >> 6;
-      if (i < kb) A[(long long)(k0 + jj) * lda + k0 + i] = (i <= jj) ? rs[i][jj] : 0.0;
+    for (int e = t; e < kb * P64_NB; e += P64_THREADS) {
+      const int i = e % P64_NB, j = e / P64_NB;
+      if (i < kb) A[(long long)(k0 + j) * lda + k0 + i] = (i <= j) ? S.R[j * P64_RLD + i] : 0.0;
     }
   }
-  if (blockIdx.x == 0) return;
-  // panel: x = R11^-T b for 8 columns per warp; lane holds rows lane and lane + 32
-  const int warp = t >> 5, lane = t & 31;
-  const int c0 = k0 + kb + (blockIdx.x - 1) * 64 + warp * 8;
-  double v[8][2];
-#pragma unroll
-  for (int cc = 0; cc < 8; ++cc) {
-    const bool ok = c0 + cc < l;
-    const double* col = A + (long long)(c0 + cc) * lda + k0;
-    v[cc][0] = (ok && lane < kb) ? col[lane] : 0.0;
-    v[cc][1] = (ok && lane + 32 < kb) ? col[lane + 32] : 0.0;
-  }
-  // rows 0..31 of the solution (held in v[.][0]), then rows 32..63 (v[.][1]): two rolled loops, each with constant
-  // register indices
-#pragma unroll 4
-  for (int i = 0; i < 32; ++i) {
-    if (i >= kb) break;
-    const double ri = inv[i];
-    const double r0 = rs[i][lane], r1 = rs[i][lane + 32];  // R[i][row] for this lane's two rows
-#pragma unroll
-    for (int cc = 0; cc < 8; ++cc) {
-      const double x = __shfl_sync(0xffffffffu, v[cc][0], i) * ri;
-      if (lane == i) v[cc][0] = x;
-      if (lane > i) v[cc][0] -= r0 * x;
-      v[cc][1] -= r1 * x;  // lane + 32 > i for every lane
-    }
-  }
-#pragma unroll 4
-  for (int i = 32; i < 64; ++i) {
-    if (i >= kb) break;
-    const double ri = inv[i];
-    const double r1 = rs[i][lane + 32];
-#pragma unroll
-    for (int cc = 0; cc < 8; ++cc) {
-      const double x = __shfl_sync(0xffffffffu, v[cc][1], i - 32) * ri;
-      if (lane == i - 32) v[cc][1] = x;
-      if (lane + 32 > i) v[cc][1] -= r1 * x;
-    }
-  }
-#pragma unroll
-  for (int cc = 0; cc < 8; ++cc) {
-    if (c0 + cc >= l) continue;
-    double* col = A + (long long)(c0 + cc) * lda + k0;
-    if (lane < kb) col[lane] = v[cc][0];
-    if (lane + 32 < kb) col[lane + 32] = v[cc][1];
-  }
+  if (group >= 4) p64_store<VEC>(acc, A, lda, k0, kb, col, cl);
 }
 
 // Trailing update of the blocked Cholesky: C[m x m] (upper triangle) -= P^T P for the kb x m panel P (kb <= 64, the
@@ -655,6 +559,10 @@ int potrf_upper(db200_context* ctx, double* A, int lda, int l, int* d_status, in
     const int s = potrf_cluster(ctx, A, lda, l, d_status, d_bad);
     if (s != DB200_ERR_UNSUPPORTED) return s;
   }
+  // (k0 is a multiple of nb: 16-byte loads need an even one too)
+  const bool vec = reinterpret_cast<uintptr_t>(A) % 16 == 0 && lda % 2 == 0 && nb % 2 == 0;
+  DB200_CUDA(ctx, cudaFuncSetAttribute(vec ? potrf_block_kernel<true> : potrf_block_kernel<false>,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(P64Smem)));
   // the diagonal-block kernel's arrival counter starts every factorisation at zero
   DB200_CUDA(ctx, cudaMemsetAsync(ctx->d_status + 1, 0, sizeof(int), ctx->stream));
   // A trailing matrix of at least one wave of 128 x 128 upper tiles takes its update on the FP64 tensor cores
@@ -674,8 +582,13 @@ int potrf_upper(db200_context* ctx, double* A, int lda, int l, int* d_status, in
     for (int k0 = K0; k0 < K0 + KB; k0 += nb) {
       const int kb = (K0 + KB - k0 < nb) ? K0 + KB - k0 : nb;
       const int rest = l - k0 - kb;
-      potrf_block_kernel<<<1 + (rest + 63) / 64, 256, 0, ctx->stream>>>(A, lda, k0, kb, l, d_status, d_bad,
-                                                                         ctx->d_status + 1);
+      const unsigned ctas = rest > 64 ? (unsigned)((rest + 63) / 64) : 1u;
+      if (vec)
+        potrf_block_kernel<true><<<ctas, P64_THREADS, sizeof(P64Smem), ctx->stream>>>(A, lda, k0, kb, l, d_status,
+                                                                                      d_bad, ctx->d_status + 1);
+      else
+        potrf_block_kernel<false><<<ctas, P64_THREADS, sizeof(P64Smem), ctx->stream>>>(A, lda, k0, kb, l, d_status,
+                                                                                       d_bad, ctx->d_status + 1);
       count_launch(ctx);
       const int pr = K0 + KB - (k0 + kb);  // rows of this panel below the block
       if (pr > 0) {
