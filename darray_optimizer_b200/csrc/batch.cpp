@@ -124,6 +124,10 @@ int db200_rbf_sketch_batched(db200_context* ctx, int count, const db200_sketch_j
       return fail(ctx, DB200_ERR_INVALID, "rbf_sketch_batched: bad job " + std::to_string(b));
     plans[(size_t)b] = job_plan(J.l, J.n_panels, J.panel, J.g_bufs);
     bytes += packed_bytes(J.m, J.n, J.d, J.Xi == J.Xj && J.ldxi == J.ldxj && J.m == J.n, plans[(size_t)b]);
+    const int mp = point_pad(J.m), np = point_pad(J.n);
+    bytes += align_up(sketch_slab_floats(plans[(size_t)b], mp, np, J.l, sketch_split(ctx, plans[(size_t)b], mp, np, J.l)) *
+                          4,
+                      256);
   }
   void* ws = workspace(ctx, bytes);
   if (!ws) return DB200_ERR_NOMEM;
@@ -146,6 +150,9 @@ int db200_rbf_sketch_batched(db200_context* ctx, int count, const db200_sketch_j
     T.gamma = J.gamma;
     T.out = J.Y;
     T.ldo = J.ldy;
+    const int split = sketch_split(ctx, P.plan, P.npad_i, P.npad_j, J.l);
+    const size_t slab = sketch_slab_floats(P.plan, P.npad_i, P.npad_j, J.l, split);
+    if (slab) T.set_split(split, cv.take<float>(slab));
   }
   TilePlan plan;
   int st = prepare_rbf_tiles(ctx, RBF_MODE_SKETCH, tj.data(), count, nullptr, 0, &plan);
@@ -180,6 +187,13 @@ int db200_svm_solve_batched(db200_context* ctx, int count, const db200_svm_insta
 
   // ---- device buffers: packed points and test matrices (workspace), per-instance pass outputs (pipeline slot)
   std::vector<SketchPlan> plans((size_t)count);
+  // slab floats of an instance's split pass (the final one promotes every two j tiles)
+  std::vector<size_t> slab_floats((size_t)count);
+  auto pass_slab = [&](SketchPlan p, const db200_svm_instance& I, bool final_pass) -> size_t {
+    if (final_pass) p.promote = 2;
+    const int np = point_pad(I.n);
+    return sketch_slab_floats(p, np, np, I.l, sketch_split(ctx, p, np, np, I.l));
+  };
   size_t wbytes = 4096, pbytes = 4096 + (size_t)workers * 256;  // + the final pass's instance table, below
   int njobs = 0;  // tile-engine instances: default multi-panel plans split into exact-width panels
   for (int b = 0; b < count; ++b) {
@@ -188,6 +202,10 @@ int db200_svm_solve_batched(db200_context* ctx, int count, const db200_svm_insta
     // kernel passes with the compensated sketch product unless the fast mixed form is asked for
     if (P.precision != DB200_MIXED_FAST) plans[(size_t)b] = comp_plan(plans[(size_t)b], I.l);
     wbytes += packed_bytes(I.n, I.n, I.d, true, plans[(size_t)b]);
+    slab_floats[(size_t)b] = pass_slab(plans[(size_t)b], I, false);
+    if (plans[(size_t)b].comp == 2)
+      slab_floats[(size_t)b] = std::max(slab_floats[(size_t)b], pass_slab(plans[(size_t)b], I, true));
+    wbytes += align_up(slab_floats[(size_t)b] * 4, 256);
     njobs += (I.n_panels <= 0) ? plans[(size_t)b].n_panels : 1;
     const size_t nl = (size_t)I.n * I.l, ll = (size_t)I.l * I.l;
     pbytes += 2 * align_up(nl * 4, 256) + align_up(nl * 8, 256) + 2 * align_up(ll * 8, 256);
@@ -224,8 +242,8 @@ int db200_svm_solve_batched(db200_context* ctx, int count, const db200_svm_insta
     if (st) return st;
     R.ms_pack = t.stop();
   }
-  // Tile-engine instances.  A default plan of several panels is split into exact-width panels, as the
-  // single-problem path splits it, so each instance's passes are the single solve's to the bit; an explicit
+  // Tile-engine instances.  A default plan of several panels is split into exact-width panels and ranges of the points j,
+  // as the single-problem path splits it, so each instance's passes are the single solve's to the bit; an explicit
   // (autotuned) plan is kept as one instance of equal panels.
   std::vector<TileJob> tj;
   tj.reserve((size_t)njobs);
@@ -241,6 +259,14 @@ int db200_svm_solve_batched(db200_context* ctx, int count, const db200_svm_insta
     T.gamma = inst[b].gamma;
     T.out = Y32[(size_t)b];
     T.ldo = inst[b].n;
+    const int np = T.pi.npad;
+    if (slab_floats[(size_t)b])
+      T.set_split(sketch_split(ctx, T.plan, np, np, T.l), cw.take<float>(slab_floats[(size_t)b]));
+    if (T.plan.comp == 2) {  // the final pass's ranges: the same slabs, multiples of its own chunks
+      SketchPlan pf = T.plan;
+      pf.promote = 2;
+      T.split_final = T.slab ? sketch_split(ctx, pf, np, np, T.l) : 0;
+    }
     if (inst[b].n_panels <= 0) exact_panel_jobs(T, tj);
     else tj.push_back(T);
   }
@@ -250,7 +276,10 @@ int db200_svm_solve_batched(db200_context* ctx, int count, const db200_svm_insta
   // the final pass (Y = K Q, contracted into the Nystrom core, whose scale the accumulation's truncation would
   // shrink) promotes every two j tiles, as db200_lowrank's final pass does; its instance table is in the workspace
   for (TileJob& T : tj)
-    if (T.plan.comp == 2) T.plan.promote = 2;
+    if (T.plan.comp == 2) {
+      T.plan.promote = 2;
+      T.split_tiles = T.split_final;
+    }
   {
     void* table_final = cw.take<char>(tile_table_bytes(nj));
     if ((st = prepare_rbf_tiles(ctx, RBF_MODE_SKETCH, tj.data(), nj, table_final, tile_table_bytes(nj),

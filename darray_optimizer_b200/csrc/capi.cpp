@@ -331,14 +331,18 @@ int db200_rbf_sketch_ex(db200_context* ctx, int m, int n, int d, int l, const fl
   if (promoted) plan.promote = (product == DB200_SKETCH_COMPENSATED_PROMOTED) ? 2 : 8;
   const int npad = point_pad(n);
   const size_t op_halves = packed_sketch_halves(plan, npad);
+  // few row blocks: ranges of the points j, their partial sums in slabs after the packed operands
+  const int split = sketch_split(ctx, plan, point_pad(m), npad, l);
+  const size_t slab_floats = sketch_slab_floats(plan, point_pad(m), npad, l, split);
   PackedPoints pi, pj;
   Carve carve{nullptr};
-  st = pack_pair(ctx, m, n, d, Xi, ldxi, Xj, ldxj, x_layout, op_halves * 2 + 256, pi, pj, carve);
+  st = pack_pair(ctx, m, n, d, Xi, ldxi, Xj, ldxj, x_layout, op_halves * 2 + slab_floats * 4 + 512, pi, pj, carve);
   if (st) return st;
   void* op = carve.take<uint16_t>(op_halves);
+  float* slab = slab_floats ? carve.take<float>(slab_floats) : nullptr;
   st = pack_sketch(ctx, Omega, ldo, yj, n, l, npad, plan.lrows, op, plan.comp);
   if (st) return st;
-  return launch_rbf_sketch_exact(ctx, pi, pj, yi, op, plan, l, gamma, Y, ldy);
+  return launch_rbf_sketch_exact(ctx, pi, pj, yi, op, plan, l, gamma, Y, ldy, split, slab);
 }
 
 int db200_rbf_sketch(db200_context* ctx, int m, int n, int d, int l, const float* Xi, int ldxi, const float* Xj,

@@ -158,10 +158,28 @@ struct TileJob {
   float gamma = 0.f;
   float* out = nullptr;
   long long ldo = 0;
+  // split_tiles > 0: the j tiles in ranges of that many (tile_split); a split SKETCH job sums its ranges through slabs of
+  // slab_stride floats (leading dimension slab_ld)
+  int split_tiles = 0, split_final = 0;  // split_final: the batch's final pass
+  float* slab = nullptr;
+  long long slab_ld = 0, slab_stride = 0;
+  void set_split(int tiles, float* slabs) {  // after pi and l
+    split_tiles = slabs ? tiles : 0;
+    slab = slabs;
+    slab_ld = pi.npad;
+    slab_stride = (long long)l * pi.npad;
+  }
 };
+// Ranges of the j tiles of one job, from its sizes and the GPU's alone (so that a problem gives the same result alone and
+// in a batch): tiles per range for a sketch of that plan, the floats of its slabs (0 when it stays whole).
+int tile_split(const db200_context* ctx, int row_blocks, int n_jtiles, int unit, int per_item, int per_split,
+               int max_ranges = 32);
+int sketch_split(const db200_context* ctx, const SketchPlan& plan, int npad_i, int npad_j, int l);
+size_t sketch_slab_floats(const SketchPlan& plan, int npad_i, int npad_j, int l, int split_tiles);
 // A prepared launch: the instance table is on the device; launch_rbf_plan only launches (graph-capturable).
 struct TilePlan {
-  int mode = 0, count = 0, n_items = 0, nsx = 0, nso = 0, nkc_max = 0, panel_max = 0, om_mult = 1;
+  int mode = 0, count = 0, n_items = 0, nsx = 0, nso = 0, nkc_max = 0, panel_max = 0, om_mult = 1, kblock = 0;
+  int red_m = 0, red_l = 0;  // largest split sketch (0: none): its ranges are summed after the tile launch
   int clusters = 0;  // persistent grid: CTA pairs resident at once (at most one per item)
   bool lean = false; // SKETCH with the single product and no promotion in every instance: the lean kernel
   size_t smem = 0;
@@ -220,6 +238,7 @@ int launch_rbf_tiles(db200_context* ctx, int mode, const PackedPoints& pi, const
 void exact_panel_jobs(const TileJob& base, std::vector<TileJob>& out);
 // The sketch as one launch over per-panel instances of exact widths (plan.n_panels panels covering roundup(l, 16)).
 int launch_rbf_sketch_exact(db200_context* ctx, const PackedPoints& pi, const PackedPoints& pj, const float* yi,
-                            const void* op, const SketchPlan& plan, int l, float gamma, float* out, int ldo);
+                            const void* op, const SketchPlan& plan, int l, float gamma, float* out, int ldo,
+                            int split_tiles = 0, float* slab = nullptr);
 
 }  // namespace db200

@@ -109,22 +109,23 @@ __global__ void gather_rows_kernel(const float* __restrict__ X, int ldx, const i
   }
 }
 
-// out[i] = sqrt of the k-th smallest of the 32 candidates part[32 i ..] (four sorted quarters of 8).
-__global__ void knn_merge_kernel(int n, const float* __restrict__ part, int k, float* __restrict__ out) {
+// out[i] = sqrt of the k-th smallest of the `cand` candidates part[cand i ..] (sorted lists of 8).
+__global__ void knn_merge_kernel(int n, const float* __restrict__ part, int cand, int k, float* __restrict__ out) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   float best[8];
 #pragma unroll
   for (int t = 0; t < 8; ++t) best[t] = INFINITY;
-  const float* p = part + (size_t)i * 32;
-#pragma unroll 4
-  for (int c = 0; c < 32; ++c) {
-    float x = p[c];
+  const float4* p = reinterpret_cast<const float4*>(part + (size_t)i * cand);
+#pragma unroll 2
+  for (int c = 0; c < cand / 4; ++c) {
+    const float4 q = p[c];
 #pragma unroll
-    for (int t = 0; t < 8; ++t) {
-      const float lo = fminf(best[t], x), hi = fmaxf(best[t], x);
-      best[t] = lo;
-      x = hi;
+    for (int e = 0; e < 4; ++e) {
+      const float x = e == 0 ? q.x : e == 1 ? q.y : e == 2 ? q.z : q.w;
+#pragma unroll
+      for (int t = 7; t > 0; --t) best[t] = fminf(best[t], fmaxf(best[t - 1], x));
+      best[0] = fminf(best[0], x);
     }
   }
   float v = best[0];
@@ -503,8 +504,10 @@ int knn_distance(db200_context* ctx, int n, int d, const float* X, int ldx, int 
     // registers (RBF_MODE_KNN), then the quarters merged.  The reference points are gathered and packed as the
     // second point set; their indices skip each point's own distance.
     const int dp = feature_pad(d), npad = point_pad(n), spad = point_pad(s);
+    // ranges of the reference points, so that the query blocks fill the GPU: a list of 8 per quarter and range
+    const int split = tile_split(ctx, npad / 256, spad / 128, 1, 2, 2), ranges = (spad / 128 + split - 1) / split;
     const size_t bytes = 4096 + (size_t)s * d * 4 + (size_t)npad * 2 * dp * 2 + packed_norm_floats(npad) * 4 +
-                         (size_t)spad * 2 * dp * 2 + packed_norm_floats(spad) * 4 + (size_t)n * 32 * 4 + 8 * 256;
+                         (size_t)spad * 2 * dp * 2 + packed_norm_floats(spad) * 4 + (size_t)n * 32 * ranges * 4 + 8 * 256;
     char* ws = static_cast<char*>(workspace(ctx, bytes));
     if (!ws) return DB200_ERR_NOMEM;
     Carve cv{ws};
@@ -513,7 +516,7 @@ int knn_distance(db200_context* ctx, int n, int d, const float* X, int ldx, int 
     float* nq = cv.take<float>(packed_norm_floats(npad));
     void* xr = cv.take<uint16_t>((size_t)spad * 2 * dp);
     float* nr = cv.take<float>(packed_norm_floats(spad));
-    float* part = cv.take<float>((size_t)n * 32);
+    float* part = cv.take<float>((size_t)n * 32 * ranges);
     gather_rows_kernel<<<blocks_for((long long)s * d, 256, 65535LL * 8), 256, 0, ctx->stream>>>(X, ldx, ref, s, d, R);
     DB200_CUDA(ctx, cudaGetLastError());
     count_launch(ctx);
@@ -535,10 +538,11 @@ int knn_distance(db200_context* ctx, int n, int d, const float* X, int ldx, int 
     J.gamma = 1.0f;
     J.out = part;
     J.ldo = 32;
+    J.split_tiles = split;
     TilePlan T;
     if ((st = prepare_rbf_tiles(ctx, RBF_MODE_KNN, &J, 1, nullptr, 0, &T))) return st;
     if ((st = launch_rbf_plan(ctx, T))) return st;
-    knn_merge_kernel<<<(unsigned)((n + 255) / 256), 256, 0, ctx->stream>>>(n, part, k, out);
+    knn_merge_kernel<<<(unsigned)((n + 255) / 256), 256, 0, ctx->stream>>>(n, part, 32 * ranges, k, out);
     DB200_CUDA(ctx, cudaGetLastError());
     count_launch(ctx);
     return DB200_OK;

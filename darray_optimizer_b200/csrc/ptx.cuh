@@ -419,4 +419,18 @@ __device__ __forceinline__ bool elect_one() {
   return pred != 0;
 }
 
+// Tiled TMA store of a box in this CTA's shared memory (generic-proxy writes before it need fence_proxy_async); waits
+// for the thread's committed stores to have read their source, and to have completed.
+__device__ __forceinline__ void tma_store_2d(const void* tmap, uint32_t smem, int x, int y) {
+  asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%1, %2}], [%3];" ::"l"(tmap), "r"(x),
+               "r"(y), "r"(smem)
+               : "memory");
+}
+__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+__device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
+__device__ __forceinline__ void fence_proxy_async_cta() {
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+}
+
 }  // namespace db200

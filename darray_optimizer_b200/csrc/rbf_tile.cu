@@ -66,6 +66,10 @@ constexpr int SMEM_LIMIT = 232448;  // dynamic shared memory per block on sm_100
 constexpr int BAR_BYTES = 1024;     // barrier region: barriers, TMEM slot, abort flag
 constexpr int MAX_NSX = 16, MAX_NSO = 4;
 constexpr float LOG2E = 1.4426950408889634f;
+// A sketch item's fill and drain in units of one tile's time (promoted items drain while they compute, single-product ones
+// store their whole panel at the end), and the summation of split ranges.  Fitted to 59 to 158 items of 157 to 470 tiles
+// cut into 1 to 16 ranges.
+constexpr int SKETCH_ITEM_TILES = 8, PROMOTED_ITEM_TILES = 2, SKETCH_SPLIT_TILES = 4;
 
 // One instance of the tile engine.  A launch walks a work list over a table of instances in global memory (one
 // instance for the single-problem entry points, many for the batched one); work item k belongs to the instance
@@ -92,6 +96,12 @@ struct alignas(64) TileInst {
   int om_lo;             // row offset of the Omega~ lo rows inside the packed operand (comp = 2)
   int promote;           // j tiles per TMEM accumulation chunk, each chunk added into Y in fp32 (0: whole item)
   int item_begin;        // first work item of this instance
+  // The points j in n_splits ranges of split_tiles tiles (the last one shorter), each a work item of its own: KBLOCK and
+  // KNN items write disjoint columns / candidate slots; SKETCH items write partial sums into slabs (out + range *
+  // split_stride), which the reduction adds in order into red_out.
+  int n_splits, split_tiles;
+  long long split_stride, red_ldo;
+  float* red_out;
   float c_row, c_dot;    // -gamma*log2e, 2*gamma*log2e
 };
 
@@ -104,23 +114,28 @@ struct LaunchArgs {
   int nsx, nso;          // Xj and Omega ring stages
   int nkc_max, panel_max;  // shared-memory layout covers every instance
   int om_mult;           // Omega stage copies: 1, or 2 when an instance loads hi and lo rows (comp = 2)
+  int kblock;            // KBLOCK and KNN: 1 (labels / shared bounds); 2 when KBLOCK tiles leave by TMA stores (tm1[2])
   int* status;
 };
 
 struct SmemLayout {
   int om_stage;  // bytes of one Omega stage in one CTA: (panel / 2) rows x 128 B, twice with lo rows
-  size_t off_xi, off_xj, off_om, off_sj, off_bar, total;
+  size_t off_xi, off_xj, off_om, off_st, off_sj, off_bar, total;
 };
-constexpr int SJ_BYTES = NUM_EPI_WARPS * 2 * EPI_COLS * 4;  // per epilogue warp: two tiles' column norms
+// per epilogue warp: two tiles' column norms; KBLOCK: as much again for labels, KNN: a 64-bit shared bound per row
+constexpr int SJ_BYTES = NUM_EPI_WARPS * 2 * EPI_COLS * 4;
+constexpr int ST_WARP = 32 * EPI_COLS * 4;                  // KBLOCK: an epilogue warp's 32 rows x 32 columns, fp32
 
-__host__ __device__ inline SmemLayout make_layout(int nkc, int panel, int nsx, int nso, int om_mult) {
+__host__ __device__ inline SmemLayout make_layout(int nkc, int panel, int nsx, int nso, int om_mult,
+                                                   int kblock) {
   SmemLayout L;
   L.om_stage = (panel / 2) * 128 * om_mult;
   L.off_xi = 0;
   L.off_xj = L.off_xi + (size_t)nkc * XI_CHUNK;
   L.off_om = L.off_xj + (size_t)nsx * XJ_CHUNK;
-  L.off_sj = L.off_om + (size_t)nso * L.om_stage;
-  L.off_bar = L.off_sj + SJ_BYTES;
+  L.off_st = L.off_om + (size_t)nso * L.om_stage;
+  L.off_sj = L.off_st + (kblock == 2 ? NUM_EPI_WARPS * ST_WARP : 0);
+  L.off_bar = L.off_sj + (kblock ? 2 : 1) * SJ_BYTES;
   L.total = L.off_bar + BAR_BYTES;
   return L;
 }
@@ -156,6 +171,21 @@ __device__ __forceinline__ int find_inst(const TileInst* inst, int count, int k)
     else hi = mid - 1;
   }
   return lo;
+}
+
+// Place of work item `item` of instance I: row block, panel and range of the j tiles.
+struct ItemPos {
+  int it, pn, sp, jt0, njt;
+};
+__device__ __forceinline__ ItemPos item_pos(const TileInst* I, int item) {
+  ItemPos P;
+  const int li = item - I->item_begin, rest = li / I->n_itiles;
+  P.it = li % I->n_itiles;
+  P.pn = rest % I->n_panels;
+  P.sp = rest / I->n_panels;
+  P.jt0 = P.sp * I->split_tiles;
+  P.njt = min(I->split_tiles, I->n_jtiles - P.jt0);
+  return P;
 }
 
 template <int V>
@@ -331,12 +361,16 @@ __device__ __forceinline__ void red_add_f32(float* p, float v) {
 // load latency (a load-add-store drain made the pass 2x slower).  Every element has one owner thread, whose first
 // chunk stores and later chunks add, in program order to the same address.  Kept out of line: its registers
 // would otherwise stay reserved across the epilogue's exp loop.
-__device__ __noinline__ void drain_sketch_chunk(const TileInst* I, int item, uint32_t rank, int row, int qc,
+__device__ __noinline__ void drain_sketch_chunk(const TileInst* I, int item, int i, int qc,
                                                 uint32_t t_lane_base, bool accumulate) {
-  const int li = item - I->item_begin;
-  const int pn = li / I->n_itiles, m = I->m;
-  const int i = (li % I->n_itiles) * PAIR_M + (int)rank * BM + row;
-  float* const out_i = I->out + i;
+  int pn = 0, sp = 0;
+  if (I->n_panels * I->n_splits > 1) {  // (the divisions of item_pos cost 3 % of a pass that drains every two tiles)
+    const int rest = (item - I->item_begin) / I->n_itiles;
+    pn = rest % I->n_panels;
+    sp = rest / I->n_panels;
+  }
+  const int m = I->m;
+  float* const out_i = I->out + sp * I->split_stride + i;
   const long long ldo = I->ldo;
   const float y_i = (i < m && I->yi) ? I->yi[i] : 1.0f;
   const int panel = I->panel, l = I->l;
@@ -374,7 +408,7 @@ template <int MODE, bool LEAN>
 __global__ void __launch_bounds__(NUM_THREADS, 1) rbf_tile_kernel(const __grid_constant__ LaunchArgs args) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  const SmemLayout L = make_layout(args.nkc_max, args.panel_max, args.nsx, args.nso, args.om_mult);
+  const SmemLayout L = make_layout(args.nkc_max, args.panel_max, args.nsx, args.nso, args.om_mult, args.kblock);
   const int nsx = args.nsx, nso = args.nso;
   const uint32_t s_xi = smem_u32(smem + L.off_xi);
   const uint32_t s_xj = smem_u32(smem + L.off_xj);
@@ -396,6 +430,9 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) rbf_tile_kernel(const __grid_c
   // a wait that gives up also stops the other CTA of the pair
   auto give_up = [&]() { st_shared_remote_u32(mapa_shared(smem_u32((const void*)abort_flag), rank ^ 1u), 1u); };
 
+  if (MODE == RBF_MODE_KNN)  // no item's number
+    for (int e = threadIdx.x; e < SJ_BYTES / 8; e += NUM_THREADS)
+      reinterpret_cast<unsigned long long*>(smem + L.off_sj + SJ_BYTES)[e] = ~0ull;
   if (threadIdx.x == 0) {
     *abort_flag = 0;
     mbar_init(bar(B_XI_FULL), 1);
@@ -440,9 +477,9 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) rbf_tile_kernel(const __grid_c
       for (int item = cid; item < n_items && ok; item += ncl, ++items_done) {
         const int b = find_inst(args.inst, args.count, item);
         const TileInst* I = args.inst + b;
-        const int li = item - I->item_begin;
-        const int it = li % I->n_itiles, pn = li / I->n_itiles;
-        const int nkc = I->nkc, njt = I->n_jtiles;
+        const ItemPos pos = item_pos(I, item);
+        const int it = pos.it, pn = pos.pn;
+        const int nkc = I->nkc, njt = pos.njt;
         const bool one = (args.count == 1);
         const CUtensorMap* t_xi = one ? &args.tm1[0] : &I->tm_xi;
         const CUtensorMap* t_xj = one ? &args.tm1[1] : &I->tm_xj;
@@ -472,7 +509,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) rbf_tile_kernel(const __grid_c
               if (!mbar_wait(bar(XJ_EMPTY + xs), xph ^ 1, abort_flag)) { ok = false; break; }
               if (leader) mbar_arrive_expect_tx(bar(XJ_FULL + xs), 2 * XJ_CHUNK);
               tma_load_2d_pair(s_xj + xs * XJ_CHUNK, t_xj, lbar(XJ_FULL + xs), c * KC,
-                               jt * BN + (int)rank * BN_HALF);
+                               (pos.jt0 + jt) * BN + (int)rank * BN_HALF);
               if (++xs == (uint32_t)nsx) { xs = 0; xph ^= 1; }
             }
           } else if (MODE == RBF_MODE_SKETCH) {
@@ -482,7 +519,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) rbf_tile_kernel(const __grid_c
               // rows of this CTA: [r*n1/2, (r+1)*n1/2) of the first instruction's n1 columns, then the same
               // half of the second instruction's n2 columns (or, compensated, of the lo rows)
               const uint32_t dst = s_om + os * L.om_stage;
-              const int x = jt * BN + c * KC, y0 = pn * panel;
+              const int x = (pos.jt0 + jt) * BN + c * KC, y0 = pn * panel;
               tma_load_2d_pair(dst, t_om1, lbar(OM_FULL + os), x, y0 + (int)rank * (n1 / 2));
               if (n2 > 0)
                 tma_load_2d_pair(dst + (n1 / 2) * 128, t_om2, lbar(OM_FULL + os), x,
@@ -537,7 +574,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) rbf_tile_kernel(const __grid_c
       for (int item = cid; item < n_items && ok; item += ncl, ++items_done) {
         // every per-instance value in registers before the tile loop (no global reads between MMAs)
         const TileInst* I = args.inst + find_inst(args.inst, args.count, item);
-        const int nkc = I->nkc, njt = I->n_jtiles, g_bufs = I->g_bufs;
+        const int nkc = I->nkc, njt = item_pos(I, item).njt, g_bufs = I->g_bufs;
         const int n1 = I->n1, n2 = I->n2;
         const bool two = n2 > 0;
         SketchMma Y;
@@ -587,18 +624,20 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) rbf_tile_kernel(const __grid_c
     // for the next tile from global memory before the current tile's exp, and parks it here afterwards, so the
     // global latency never sits between a G tile and its P tile.
     float* sjbuf = reinterpret_cast<float*>(smem + L.off_sj) + ew * 2 * EPI_COLS;
+    float* yjbuf = sjbuf + SJ_BYTES / 4;  // KBLOCK: the columns' labels
+    float* stage = reinterpret_cast<float*>(smem + L.off_st + (size_t)ew * ST_WARP);  // [column][32 rows]
     uint32_t kp = 0, items_done = 0, ydone = 0;  // ydone: Y accumulations drained (B_Y_FULL phases)
     uint32_t guse0 = 0, guse1 = 0, gnext = 0;  // the same G-buffer sequence as the MMA issuer
     bool ok = true;
     for (int item = cid; item < n_items && ok; item += ncl, ++items_done) {
       const TileInst* I = args.inst + find_inst(args.inst, args.count, item);
-      const int li = item - I->item_begin;
-      const int it = li % I->n_itiles, pn = li / I->n_itiles;
-      const int njt = I->n_jtiles, g_bufs = I->g_bufs, m = I->m;
+      const ItemPos pos = item_pos(I, item);
+      const int it = pos.it;
+      const int njt = pos.njt, g_bufs = I->g_bufs, m = I->m;
       const bool p_lo = !LEAN && (I->comp >= 1);
       const int promote = (MODE == RBF_MODE_SKETCH && !LEAN) ? I->promote : 0;
       const float c_row = I->c_row;
-      const float* sj = I->sj;
+      const float* sj = I->sj + pos.jt0 * BN;
       const uint32_t t_p = tmem_base + t_lane + (uint32_t)I->tmem_p + (uint32_t)(qc * (EPI_COLS / 2));
       const long long ldo = I->ldo;
       const int n_cols = I->n;
@@ -609,6 +648,13 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) rbf_tile_kernel(const __grid_c
       const float c_dot = I->c_dot * *I->fi * *I->fj;  // x_i.x_j = 2^-(e_I + e_J) G
       const float y_i = (i < m && I->yi) ? I->yi[i] : 1.0f;
       sjbuf[lane] = sj[qc * EPI_COLS + lane];  // tile 0 of this item
+      auto label_j = [&](int j) -> float { return (yj_all && j < n_cols) ? __ldg(yj_all + j) : 1.0f; };
+      // KNN: yj carries the points' indices; -(1 << 30) (no row of any warp) past the end
+      auto index_j = [&](int j) -> int {
+        return j < n_cols ? __ldg(reinterpret_cast<const int*>(yj_all) + j) : -(1 << 30);
+      };
+      int idx_now = MODE == RBF_MODE_KNN ? index_j(pos.jt0 * BN + qc * EPI_COLS + lane) : 0;
+      if (MODE == RBF_MODE_KBLOCK) yjbuf[lane] = label_j(pos.jt0 * BN + qc * EPI_COLS + lane);
       __syncwarp();
       float best[8];  // KNN: this row's 8 smallest squared distances in this column quarter, ascending
 #pragma unroll
@@ -617,7 +663,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) rbf_tile_kernel(const __grid_c
       auto drain = [&](bool accumulate) -> bool {
         if (!__all_sync(0xffffffffu, mbar_wait(bar(B_Y_FULL), ydone & 1, abort_flag))) return false;
         tc_fence_after();
-        drain_sketch_chunk(I, item, rank, row, qc, tmem_base + t_lane, accumulate);
+        drain_sketch_chunk(I, item, i, qc, tmem_base + t_lane, accumulate);
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive_remote(lbar(B_Y_EMPTY));
@@ -627,6 +673,11 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) rbf_tile_kernel(const __grid_c
       for (int jt = 0; jt < njt; ++jt) {
         // sj is padded to n_jtiles * BN
         const float sj_next = (jt + 1 < njt) ? sj[(jt + 1) * BN + qc * EPI_COLS + lane] : 0.0f;
+        const int idx_next =
+            (MODE == RBF_MODE_KNN && jt + 1 < njt) ? index_j((pos.jt0 + jt + 1) * BN + qc * EPI_COLS + lane) : 0;
+        const float yj_next = (MODE == RBF_MODE_KBLOCK && jt + 1 < njt)
+                                  ? label_j((pos.jt0 + jt + 1) * BN + qc * EPI_COLS + lane)
+                                  : 0.0f;
         const uint32_t b = gnext;
         const uint32_t guse = b ? guse1 : guse0;
         if (!__all_sync(0xffffffffu, mbar_wait(bar(B_G_FULL0 + b), guse & 1, abort_flag))) { ok = false; break; }
@@ -643,27 +694,60 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) rbf_tile_kernel(const __grid_c
         __syncwarp();
         if (lane == 0) mbar_arrive_remote(lbar(B_G_EMPTY0 + b));
 
-        const int j0 = jt * BN + qc * EPI_COLS;
+        const int j0 = (pos.jt0 + jt) * BN + qc * EPI_COLS;
         if (MODE == RBF_MODE_KNN) {
           // d^2 = |x_i|^2 + |x_j|^2 - 2 x.y (x.y = c_dot G), inserted into the sorted list; padding columns and the
           // point itself skipped
           const float* sjt = sjbuf + (jt & 1) * EPI_COLS;
-          const int* idx_j = reinterpret_cast<const int*>(yj_all);
           const float s_i = I->si[i];
+          // The row's four lists (column quarters) share a bound: two of them holding four values each at or below the
+          // second smallest of their fourth entries, nothing at or above it can be among the row's 8 smallest (about 13
+          // candidates lie below it, 32 below a list's own last entry).  The quarters' warps publish their fourth entry
+          // with the item's number; an older value of the same item is only a looser bound.
+          volatile unsigned long long* bounds = reinterpret_cast<volatile unsigned long long*>(smem + L.off_sj + SJ_BYTES);
+          float f[4];
 #pragma unroll
-          for (int c = 0; c < EPI_COLS; ++c) {
-            const int j = j0 + c;
-            const float d2 = fmaf(-2.0f * c_dot, v[c], s_i + sjt[c]);
-            if (j < n_cols && d2 < best[7] && __ldg(idx_j + j) != i) {
-              float x = d2;
+          for (int t = 0; t < 4; ++t) {
+            const unsigned long long w = bounds[(q * 4 + t) * 32 + lane];
+            f[t] = (int)(w >> 32) == item ? __uint_as_float((unsigned)w) : INFINITY;
+          }
+          const float shared = fminf(fmaxf(fminf(f[0], f[1]), fminf(f[2], f[3])),
+                                     fminf(fmaxf(f[0], f[1]), fmaxf(f[2], f[3])));
+          // Columns go four at a time against the bound, skipped when no lane has one below it.  An insertion is
+          // b[t] = min(b[t], max(b[t - 1], x)) from the old entries: eight independent steps (moving x down the list made
+          // them one chain), and a no-op in lanes whose x is not below the list, so the warp never diverges.  The point
+          // itself is looked for only in tiles that hold an index of this warp's rows (or columns past the end).
+          float bound = fminf(best[7], shared);
+          const int il = idx_now - (i - lane);  // the row (of this warp) that this lane's column is
+          const bool special = j0 + EPI_COLS > n_cols || __any_sync(0xffffffffu, il >= 0 && il < 32);
 #pragma unroll
-              for (int t = 0; t < 8; ++t) {  // insertion: x moves down while it is smaller
-                const float lo = fminf(best[t], x), hi = fmaxf(best[t], x);
-                best[t] = lo;
-                x = hi;
+          for (int c = 0; c < EPI_COLS; c += 4) {
+            float d2[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) d2[e] = fmaf(-2.0f * c_dot, v[c + e], s_i + sjt[c + e]);
+            if (special) {
+#pragma unroll
+              for (int e = 0; e < 4; ++e) {
+                const int skip = __shfl_sync(0xffffffffu, il, c + e);
+                if (j0 + c + e >= n_cols || skip == lane) d2[e] = INFINITY;
+              }
+            }
+            if (__any_sync(0xffffffffu, fminf(fminf(d2[0], d2[1]), fminf(d2[2], d2[3])) < bound)) {
+#pragma unroll
+              for (int e = 0; e < 4; ++e) {
+                if (__any_sync(0xffffffffu, d2[e] < bound)) {
+                  const float x = d2[e] < bound ? d2[e] : INFINITY;  // NaN is never inserted
+#pragma unroll
+                  for (int t = 7; t > 0; --t) best[t] = fminf(best[t], fmaxf(best[t - 1], x));
+                  best[0] = fminf(best[0], x);
+                  bound = fminf(best[7], bound);
+                }
               }
             }
           }
+          bounds[(q * 4 + qc) * 32 + lane] =
+              ((unsigned long long)(unsigned)item << 32) | (unsigned long long)__float_as_uint(best[3]);
+          idx_now = idx_next;
         }
         if (MODE != RBF_MODE_UPDATE && MODE != RBF_MODE_KNN) {
           const float4* sj4 = reinterpret_cast<const float4*>(sjbuf + (jt & 1) * EPI_COLS);
@@ -678,6 +762,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) rbf_tile_kernel(const __grid_c
         }
 
         sjbuf[((jt + 1) & 1) * EPI_COLS + lane] = sj_next;
+        if (MODE == RBF_MODE_KBLOCK) yjbuf[((jt + 1) & 1) * EPI_COLS + lane] = yj_next;
         __syncwarp();
         if (MODE == RBF_MODE_SKETCH) {
           // P_hi = fp16(P); with the compensated product also P_lo = fp16(P - P_hi), the exact residual of the hi
@@ -741,21 +826,40 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) rbf_tile_kernel(const __grid_c
             }
           }
         } else {
-          if (i < m) {
+          const float* yjt = yjbuf + (jt & 1) * EPI_COLS;
+          if (args.kblock == 2) {
+            // The warp's 32 x 32 values go to its stage (a column's 32 rows are one conflict-free store) and leave by one
+            // TMA store, which clips at n and at m rounded down to 4 rows (it writes 16-byte pieces: up to three last
+            // rows are stored by their threads); the stage is free once the previous tile's store has read it.  Stores by
+            // the threads held the next tile's exp back (8192 x 8192, 268 MB: 115 us against 75).
+            if (lane == 0) bulk_wait_read();
+            __syncwarp();
+#pragma unroll
+            for (int c = 0; c < EPI_COLS; ++c) stage[c * 32 + lane] = y_i * yjt[c] * v[c];
+            fence_proxy_async_cta();
+            __syncwarp();
+            const int i0 = i - lane;
+            if (lane == 0 && i0 < (m & ~3) && j0 < n_cols) {
+              tma_store_2d(&args.tm1[2], smem_u32(stage), i0, j0);
+              bulk_commit();
+            }
+            if (i >= (m & ~3) && i < m) {
+#pragma unroll
+              for (int c = 0; c < EPI_COLS; ++c)
+                if (j0 + c < n_cols) out_i[(size_t)(j0 + c) * ldo] = y_i * yjt[c] * v[c];
+            }
+          } else if (i < m) {
 #pragma unroll
             for (int c = 0; c < EPI_COLS; ++c) {
               const int j = j0 + c;
-              if (j < n_cols) {
-                const float yj = yj_all ? __ldg(yj_all + j) : 1.0f;
-                out_i[(size_t)j * ldo] = y_i * yj * v[c];
-              }
+              if (j < n_cols) out_i[(size_t)j * ldo] = y_i * yjt[c] * v[c];
             }
           }
         }
       }
       if (!ok) break;
       if (MODE == RBF_MODE_KNN && i < m) {
-        float* o = I->out + (size_t)i * 32 + qc * 8;
+        float* o = I->out + ((size_t)i * I->n_splits + pos.sp) * 32 + qc * 8;
 #pragma unroll
         for (int t = 0; t < 8; ++t) o[t] = best[t];
       }
@@ -763,6 +867,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) rbf_tile_kernel(const __grid_c
         if (!drain(false)) { ok = false; break; }
       }
     }
+    if (MODE == RBF_MODE_KBLOCK && lane == 0) bulk_wait_all();  // this thread's stores have left its shared memory
     if (!ok && lane == 0) give_up();
     __syncwarp();
   }
@@ -776,40 +881,78 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) rbf_tile_kernel(const __grid_c
   if (warp == 1) tmem_dealloc_pair(tmem_base, TMEM_COLS);
 }
 
-// ------------------------------------------------------------------ packing kernels
-// Largest |x_ik| of a point set (non-negative floats order like their bit patterns): block maxima, then one
-// atomicMax per block into *out, which the caller zeroes first.
-__global__ void absmax_points_kernel(const float* __restrict__ X, long long sp, long long sf, int n, int d,
-                                     unsigned* __restrict__ out) {
-  const long long total = (long long)n * d;
-  float mx = 0.f;
-  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < total;
-       e += (long long)gridDim.x * blockDim.x) {
-    const long long i = e / d, k = e % d;
-    const float a = fabsf(X[i * sp + k * sf]);
-    if (a <= 3.0e38f) mx = fmaxf(mx, a);  // NaN and inf do not set the scale
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-  __shared__ float wmax[32];
-  if ((threadIdx.x & 31) == 0) wmax[threadIdx.x / 32] = mx;
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    mx = (threadIdx.x < blockDim.x / 32) ? wmax[threadIdx.x] : 0.f;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    if (threadIdx.x == 0) atomicMax(out, __float_as_uint(mx));
+// Y(i, c) = the sum over the ranges of the j tiles, in their order, of the partial sums in the slabs (blockIdx.z: the
+// instance; those of one range wrote Y themselves).
+__global__ void __launch_bounds__(256) sum_slabs_kernel(const TileInst* __restrict__ inst) {
+  const TileInst* I = inst + blockIdx.z;
+  const int S = I->n_splits, i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (S <= 1 || i >= I->m) return;
+  const long long stride = I->split_stride, ldo = I->ldo, ldy = I->red_ldo;
+  for (int c = blockIdx.y; c < I->l; c += gridDim.y) {
+    const float* p = I->out + c * ldo + i;
+    float acc = p[0];
+#pragma unroll 4
+    for (int k = 1; k < S; ++k) acc += p[k * stride];
+    I->red_out[c * ldy + i] = acc;
   }
 }
 
-// One warp per point.  Every point of the set is scaled by the same 2^e, e = 14 - ceil(log2 max |x_ik|) (largest
-// |coordinate| in [2^13, 2^14)), and split into fp16 hi = fp16(2^e x), lo = fp16(2^e x - hi).  norms[i] =
-// ||x||^2 (0 on padding rows) and norms[npad + 1] = 2^-e; norms[npad] holds the set's max |x| bits from
-// absmax_points_kernel, and norms[npad + 2] becomes nonzero when some lo part is (zeroed beforehand).  d <= dp <= 128, so each lane holds its (up to 4) coordinates in registers.
-__global__ void pack_points_kernel(const float* __restrict__ X, long long sp, long long sf, int n, int d, int dp,
-                                   int npad, __half* __restrict__ Xp, float* __restrict__ norms) {
-  const int lane = threadIdx.x & 31;
-  const long long warps = (long long)gridDim.x * (blockDim.x / 32);
+// ------------------------------------------------------------------ packing kernels
+// Largest |x| of `rows` rows of `cols` contiguous floats, ld apart (non-negative floats order like their bit
+// patterns): block maxima, then one atomicMax per block into *out, which the caller zeroes first.  A set without gaps
+// is passed as one row; otherwise a warp walks a row.  vec: 16-byte loads (aligned base, and ld when rows > 1).  Bound
+// by reading the set once (131072 x 128: 67 MB, 19 us; with a 64-bit division per element it took 87 us).
+__global__ void __launch_bounds__(256) absmax_points_kernel(const float* __restrict__ X, long long rows, long long cols,
+                                                            long long ld, int vec, unsigned* __restrict__ out) {
+  float mx = 0.f;
+  auto take = [&](float x) {
+    const float a = fabsf(x);
+    if (a <= 3.0e38f) mx = fmaxf(mx, a);  // NaN and inf do not set the scale
+  };
+  const long long step = rows == 1 ? (long long)gridDim.x * blockDim.x : 32;
+  const long long lane = rows == 1 ? (long long)blockIdx.x * blockDim.x + threadIdx.x : threadIdx.x & 31;
+  const long long r0 = rows == 1 ? 0 : (long long)blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
+  for (long long r = r0; r < rows; r += (long long)gridDim.x * (blockDim.x / 32)) {
+    const float* row = X + r * ld;
+    const long long c4 = vec ? cols / 4 : 0;
+#pragma unroll 4
+    for (long long c = lane; c < c4; c += step) {
+      const float4 v = __ldg(reinterpret_cast<const float4*>(row) + c);
+      take(v.x);
+      take(v.y);
+      take(v.z);
+      take(v.w);
+    }
+    for (long long c = 4 * c4 + lane; c < cols; c += step) take(__ldg(row + c));
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  __shared__ float wmax[8];
+  if ((threadIdx.x & 31) == 0) wmax[threadIdx.x / 32] = mx;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+#pragma unroll
+    for (int w = 1; w < 8; ++w) mx = fmaxf(mx, wmax[w]);
+    atomicMax(out, __float_as_uint(mx));
+  }
+}
+
+// Split-fp16 pack of 32 points per block, a thread per point and 8 features (32 dp / 8 threads; neighbouring threads
+// take neighbouring features of point-major points, neighbouring points of feature-major ones, so both read whole
+// lines).  Every point of the set is scaled by the same 2^e, e = 14 - ceil(log2 max |x_ik|) (largest |coordinate| in
+// [2^13, 2^14)), and split into fp16 hi = fp16(2^e x), lo = fp16(2^e x - hi), each written as one 16-byte piece.
+// norms[i] = ||x||^2 (0 on padding rows) and norms[npad + 1] = 2^-e; norms[npad] holds the set's max |x| bits from
+// absmax_points_kernel, and norms[npad + 2] becomes nonzero when some lo part is (zeroed beforehand).  vec: 16-byte
+// loads.  Bound by the bytes (131072 x 128: 134 MB, 25 us; with a warp per point and 2-byte stores it took 167 us).
+constexpr int PACK_POINTS = 32;
+__global__ void __launch_bounds__(512) pack_points_kernel(const float* __restrict__ X, long long ldx, int feature_major,
+                                                          int vec, int n, int d, int dp, int npad,
+                                                          __half* __restrict__ Xp, float* __restrict__ norms) {
+  __shared__ float part[16][PACK_POINTS];
+  const int G = dp / 8;
+  const int pt = feature_major ? threadIdx.x % PACK_POINTS : threadIdx.x / G;
+  const int gr = feature_major ? threadIdx.x / PACK_POINTS : threadIdx.x % G;
+  const int i = blockIdx.x * PACK_POINTS + pt, k0 = 8 * gr;
   const float mx = __uint_as_float(*reinterpret_cast<const unsigned*>(norms + npad));
   int e = 0;
   if (mx > 0.f) {
@@ -819,48 +962,92 @@ __global__ void pack_points_kernel(const float* __restrict__ X, long long sp, lo
   }
   const float sc = ldexpf(1.0f, e);
   if (blockIdx.x == 0 && threadIdx.x == 0) norms[npad + 1] = ldexpf(1.0f, -e);
-  unsigned* lo_flag = reinterpret_cast<unsigned*>(norms + npad + 2);
-  for (long long i = (long long)blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32; i < npad; i += warps) {
-    float acc = 0.f;
-    bool has_lo = false;
-    __half* row = Xp + i * (2 * dp);
+  float x[8];
 #pragma unroll
-    for (int t = 0; t < 4; ++t) {
-      const int k = lane + 32 * t;
-      if (k < dp) {
-        const float x = ((i < n && k < d) ? X[i * sp + (long long)k * sf] : 0.f) * sc;  // exact: power of two
-        const __half hi = __float2half_rn(x);
-        const __half lo = __float2half_rn(x - __half2float(hi));
-        row[k] = hi;
-        row[dp + k] = lo;
-        // ||x||^2 from the same split products the distance MMA forms (hi.hi + 2 hi.lo), so that
-        // ||x||^2 + ||y||^2 - 2 x.y cancels to ~fp32 round-off for coincident points
-        const float h = __half2float(hi), l = __half2float(lo);
-        acc = fmaf(h, h, fmaf(2.0f * h, l, acc));
-        if (l != 0.0f) has_lo = true;
+  for (int u = 0; u < 8; ++u) x[u] = 0.f;
+  if (i < n) {
+    if (feature_major) {
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        if (k0 + u < d) x[u] = __ldg(X + (long long)(k0 + u) * ldx + i);
+    } else {
+      const float* row = X + (long long)i * ldx + k0;
+      if (vec && k0 + 8 <= d) {
+        const float4 a = __ldg(reinterpret_cast<const float4*>(row)), b = __ldg(reinterpret_cast<const float4*>(row) + 1);
+        x[0] = a.x, x[1] = a.y, x[2] = a.z, x[3] = a.w, x[4] = b.x, x[5] = b.y, x[6] = b.z, x[7] = b.w;
+      } else {
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+          if (k0 + u < d) x[u] = __ldg(row + u);
       }
     }
-    if (__any_sync(0xffffffffu, has_lo) && lane == 0) atomicOr(lo_flag, 1u);
+  }
+  float acc = 0.f;
+  bool has_lo = false;
+  __align__(16) __half hi[8], lo[8];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if (lane == 0) norms[i] = ldexpf(acc, -2 * e);
+  for (int u = 0; u < 8; ++u) {
+    const float v = x[u] * sc;  // exact: power of two
+    hi[u] = __float2half_rn(v);
+    const float h = __half2float(hi[u]);
+    lo[u] = __float2half_rn(v - h);
+    const float l = __half2float(lo[u]);
+    // ||x||^2 from the same split products the distance MMA forms (hi.hi + 2 hi.lo), so that
+    // ||x||^2 + ||y||^2 - 2 x.y cancels to ~fp32 round-off for coincident points
+    acc = fmaf(h, h, fmaf(2.0f * h, l, acc));
+    if (l != 0.0f) has_lo = true;
+  }
+  __half* row = Xp + (long long)i * (2 * dp) + k0;
+  *reinterpret_cast<uint4*>(row) = *reinterpret_cast<const uint4*>(hi);
+  *reinterpret_cast<uint4*>(row + dp) = *reinterpret_cast<const uint4*>(lo);
+  part[gr][pt] = acc;
+  const int any = __syncthreads_or(has_lo);
+  unsigned* lo_flag = reinterpret_cast<unsigned*>(norms + npad + 2);
+  if (threadIdx.x == 0 && any && *(volatile unsigned*)lo_flag == 0u) atomicOr(lo_flag, 1u);
+  if (threadIdx.x < PACK_POINTS) {
+    float s = 0.f;
+    for (int q = 0; q < G; ++q) s += part[q][threadIdx.x];
+    norms[blockIdx.x * PACK_POINTS + threadIdx.x] = ldexpf(s, -2 * e);
   }
 }
 
-// Omega~^T rows in fp16: Op[c][j] = fp16(y_j Omega[j + c*ldo]) for c < lrows; with `comp`, rows lrows + c hold
-// the lo parts fp16(y_j Omega - hi).
-__global__ void pack_sketch_kernel(const float* __restrict__ Om, long long ldo, const float* __restrict__ yj, int n,
-                                   int l, int njpad, int lrows, int comp, __half* __restrict__ Op) {
+// Omega~^T rows in fp16: Op[c][j] = fp16(y_j Omega[j + c*ldo]) for c = blockIdx.y < lrows; with `comp`, rows lrows + c
+// hold the lo parts fp16(y_j Omega - hi).  A thread takes 8 points j (njpad is a multiple of 8): two 16-byte loads (vec)
+// and one 16-byte store per part.  Bound by the bytes (131072 x 528: 415 MB, 90 us; element by element 250 us).
+__global__ void __launch_bounds__(256) pack_sketch_kernel(const float* __restrict__ Om, long long ldo, int vec,
+                                                          const float* __restrict__ yj, int n, int l, int njpad,
+                                                          int lrows, int comp, __half* __restrict__ Op) {
   const long long total = (long long)njpad * lrows;
-  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < total;
-       e += (long long)gridDim.x * blockDim.x) {
-    const int j = (int)(e % njpad);
-    const int c = (int)(e / njpad);
-    float v = 0.f;
-    if (j < n && c < l) v = Om[j + (long long)c * ldo] * (yj ? yj[j] : 1.0f);
-    const __half hi = __float2half_rn(v);
-    Op[e] = hi;
-    if (comp) Op[total + e] = __float2half_rn(v - __half2float(hi));
+  const int j0 = 8 * (blockIdx.x * blockDim.x + threadIdx.x);
+  if (j0 >= njpad) return;
+  float y[8];
+#pragma unroll
+  for (int u = 0; u < 8; ++u) y[u] = (yj && j0 + u < n) ? __ldg(yj + j0 + u) : 1.0f;
+  for (int c = blockIdx.y; c < lrows; c += gridDim.y) {
+    float v[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) v[u] = 0.f;
+    if (c < l) {
+      const float* src = Om + (long long)c * ldo + j0;
+      if (vec && j0 + 8 <= n) {
+        const float4 a = __ldg(reinterpret_cast<const float4*>(src)), b = __ldg(reinterpret_cast<const float4*>(src) + 1);
+        v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w, v[4] = b.x, v[5] = b.y, v[6] = b.z, v[7] = b.w;
+      } else {
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+          if (j0 + u < n) v[u] = __ldg(src + u);
+      }
+    }
+    __align__(16) __half hi[8], lo[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const float w = v[u] * y[u];
+      hi[u] = __float2half_rn(w);
+      lo[u] = __float2half_rn(w - __half2float(hi[u]));
+    }
+    __half* dst = Op + (long long)c * njpad + j0;
+    *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(hi);
+    if (comp) *reinterpret_cast<uint4*>(dst + total) = *reinterpret_cast<const uint4*>(lo);
   }
 }
 
@@ -893,6 +1080,20 @@ bool make_tmap(CUtensorMap* tm, const void* base, uint64_t inner, uint64_t outer
                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS;
+}
+
+// Map of a column-major fp32 output (rows contiguous; m rounded down to 4 of them) in boxes of 32 x 32; false where TMA
+// cannot write it (base or leading dimension not 16-byte aligned, fewer than 4 rows).
+bool make_out_tmap(CUtensorMap* tm, float* out, int m, int n, long long ldo) {
+  auto enc = get_encode();
+  if (!enc || reinterpret_cast<uintptr_t>(out) % 16 != 0 || ldo % 4 != 0 || m < 4) return false;
+  cuuint64_t dims[2] = {(cuuint64_t)(m & ~3), (cuuint64_t)n};
+  cuuint64_t strides[1] = {(cuuint64_t)ldo * 4};
+  cuuint32_t box[2] = {32, (cuuint32_t)EPI_COLS};
+  cuuint32_t estr[2] = {1, 1};
+  return enc(tm, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, out, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+             CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE,
+             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 cudaLaunchConfig_t launch_config(cudaLaunchAttribute* attr, int clusters, size_t smem, cudaStream_t st) {
@@ -959,22 +1160,26 @@ SketchPlan plan_sketch(int l, int comp) {
 
 int pack_points(db200_context* ctx, const float* X, int ldx, int layout, int n, int d, int dp, int npad, void* xp,
                 float* norms) {
-  const long long sp = (layout == DB200_POINT_MAJOR) ? ldx : 1;
-  const long long sf = (layout == DB200_POINT_MAJOR) ? 1 : ldx;
+  const bool point_major = layout == DB200_POINT_MAJOR;
+  const bool aligned = reinterpret_cast<uintptr_t>(X) % 16 == 0;
   unsigned* mx = reinterpret_cast<unsigned*>(norms + npad);
   DB200_CUDA(ctx, cudaMemsetAsync(mx, 0, 4 * sizeof(unsigned), ctx->stream));  // max |x|, scale, lo flag
   if (n > 0) {
-    long long mblocks = ((long long)n * d + 255) / 256;
-    if (mblocks > (long long)ctx->num_sms * 4) mblocks = (long long)ctx->num_sms * 4;
-    absmax_points_kernel<<<(unsigned)mblocks, 256, 0, ctx->stream>>>(X, sp, sf, n, d, mx);
+    long long rows = point_major ? n : d, cols = point_major ? d : n;
+    if (ldx == cols) {
+      cols *= rows;
+      rows = 1;
+    }
+    const bool vec = aligned && (rows == 1 || ldx % 4 == 0);
+    const long long work = rows == 1 ? (cols + 4095) / 4096 : (rows + 7) / 8;  // 16 elements a thread, a row a warp
+    const unsigned blocks = (unsigned)std::max(1LL, std::min(work, 8LL * ctx->num_sms));
+    absmax_points_kernel<<<blocks, 256, 0, ctx->stream>>>(X, rows, cols, ldx, vec ? 1 : 0, mx);
     DB200_CUDA(ctx, cudaGetLastError());
     count_launch(ctx);
   }
-  const int threads = 256;
-  long long blocks = ((long long)npad * 32 + threads - 1) / threads;
-  if (blocks > 65535LL * 4) blocks = 65535LL * 4;
-  pack_points_kernel<<<(unsigned)blocks, threads, 0, ctx->stream>>>(X, sp, sf, n, d, dp, npad,
-                                                                    static_cast<__half*>(xp), norms);
+  const bool vec = point_major && aligned && ldx % 4 == 0;
+  pack_points_kernel<<<npad / PACK_POINTS, PACK_POINTS * (dp / 8), 0, ctx->stream>>>(
+      X, ldx, point_major ? 0 : 1, vec ? 1 : 0, n, d, dp, npad, static_cast<__half*>(xp), norms);
   DB200_CUDA(ctx, cudaGetLastError());
   count_launch(ctx);
   return DB200_OK;
@@ -982,11 +1187,10 @@ int pack_points(db200_context* ctx, const float* X, int ldx, int layout, int n, 
 
 int pack_sketch(db200_context* ctx, const float* Omega, int ldo, const float* yj, int n, int l, int njpad, int lrows,
                 void* op, int comp) {
-  const long long total = (long long)njpad * lrows;
-  long long blocks = (total + 255) / 256;
-  if (blocks > (long long)ctx->num_sms * 32) blocks = (long long)ctx->num_sms * 32;
-  pack_sketch_kernel<<<(unsigned)blocks, 256, 0, ctx->stream>>>(Omega, ldo, yj, n, l, njpad, lrows,
-                                                                comp == 2 ? 1 : 0, static_cast<__half*>(op));
+  const bool vec = reinterpret_cast<uintptr_t>(Omega) % 16 == 0 && ldo % 4 == 0;
+  const dim3 grid((unsigned)((njpad / 8 + 255) / 256), (unsigned)std::min(lrows, 65535));
+  pack_sketch_kernel<<<grid, 256, 0, ctx->stream>>>(Omega, ldo, vec ? 1 : 0, yj, n, l, njpad, lrows,
+                                                    comp == 2 ? 1 : 0, static_cast<__half*>(op));
   DB200_CUDA(ctx, cudaGetLastError());
   count_launch(ctx);
   return DB200_OK;
@@ -998,7 +1202,8 @@ int prepare_rbf_tiles(db200_context* ctx, int mode, const TileJob* jobs, int cou
                       size_t table_capacity, TilePlan* plan) {
   if (count < 1 || !jobs || !plan) return fail(ctx, DB200_ERR_INVALID, "rbf tiles: empty job list");
   std::vector<TileInst> host((size_t)count);
-  int items = 0, nkc_max = 1, panel_max = 16, om_mult = 1;
+  int items = 0, nkc_max = 1, panel_max = 16, om_mult = 1, red_m = 0, red_l = 0;
+  int kblock = (mode == RBF_MODE_KBLOCK || mode == RBF_MODE_KNN) ? 1 : 0;
   for (int b = 0; b < count; ++b) {
     const TileJob& J = jobs[b];
     const PackedPoints &pi = J.pi, &pj = J.pj;
@@ -1040,7 +1245,8 @@ int prepare_rbf_tiles(db200_context* ctx, int mode, const TileJob* jobs, int cou
       I.promote = P.promote;
       om_mult = std::max(om_mult, P.comp == 2 ? 2 : 1);
     } else {
-      I.tm_om1 = I.tm_om2 = I.tm_xj;  // unused
+      I.tm_om1 = I.tm_om2 = I.tm_xj;  // unused, or KBLOCK's output map
+      if (mode == RBF_MODE_KBLOCK && count == 1 && make_out_tmap(&I.tm_om1, J.out, pi.n, pj.n, J.ldo)) kblock = 2;
       I.n_panels = 1;
       I.panel = 16;
       I.n1 = 16;
@@ -1073,7 +1279,20 @@ int prepare_rbf_tiles(db200_context* ctx, int mode, const TileJob* jobs, int cou
     I.out = J.out;
     I.ldo = J.ldo;
     I.item_begin = items;
-    items += I.n_itiles * I.n_panels;
+    I.split_tiles = J.split_tiles > 0 ? J.split_tiles : I.n_jtiles;
+    I.n_splits = (I.n_jtiles + I.split_tiles - 1) / I.split_tiles;
+    if (mode == RBF_MODE_SKETCH && I.n_splits > 1) {
+      if (!J.slab || (P.promote && I.split_tiles % P.promote))
+        return fail(ctx, DB200_ERR_INVALID, "rbf tiles: split sketch without slabs or off its chunks");
+      I.red_out = I.out;
+      I.red_ldo = I.ldo;
+      I.out = J.slab;
+      I.ldo = J.slab_ld;
+      I.split_stride = J.slab_stride;
+      red_m = std::max(red_m, I.m);
+      red_l = std::max(red_l, I.l);
+    }
+    items += I.n_itiles * I.n_panels * I.n_splits;
     nkc_max = std::max(nkc_max, I.nkc);
     panel_max = std::max(panel_max, I.panel);
   }
@@ -1081,21 +1300,24 @@ int prepare_rbf_tiles(db200_context* ctx, int mode, const TileJob* jobs, int cou
   T.mode = mode;
   T.count = count;
   T.n_items = items;
+  T.red_m = red_m;
+  T.red_l = red_l;
   T.nkc_max = nkc_max;
   T.panel_max = panel_max;
   T.nso = (mode == RBF_MODE_SKETCH) ? MAX_NSO : 0;
   T.lean = (mode == RBF_MODE_SKETCH);
   for (int b = 0; b < count; ++b) T.lean = T.lean && host[(size_t)b].comp == 0 && host[(size_t)b].promote == 0;
   T.om_mult = om_mult;
+  T.kblock = kblock;
   {  // the Xj ring takes whatever shared memory is left
-    const SmemLayout L0 = make_layout(nkc_max, panel_max, 0, T.nso, om_mult);
+    const SmemLayout L0 = make_layout(nkc_max, panel_max, 0, T.nso, om_mult, T.kblock);
     const long long left = (long long)SMEM_LIMIT - 1024 - (long long)L0.total;
     int nsx = (int)(left / XJ_CHUNK);
     if (nsx > MAX_NSX) nsx = MAX_NSX;
     if (nsx < 2) return fail(ctx, DB200_ERR_UNSUPPORTED, "rbf tiles: shared memory plan does not fit");
     T.nsx = nsx;
   }
-  T.smem = make_layout(nkc_max, panel_max, T.nsx, T.nso, om_mult).total + 1024;
+  T.smem = make_layout(nkc_max, panel_max, T.nsx, T.nso, om_mult, T.kblock).total + 1024;
   {
     const int max_clusters = ctx->num_sms / 2;
     cudaError_t e =
@@ -1140,6 +1362,7 @@ int launch_rbf_plan(db200_context* ctx, const TilePlan& T) {
   a.nsx = T.nsx;
   a.nso = T.nso;
   a.om_mult = T.om_mult;
+  a.kblock = T.kblock;
   a.nkc_max = T.nkc_max;
   a.panel_max = T.panel_max;
   a.status = ctx->d_status;
@@ -1155,7 +1378,56 @@ int launch_rbf_plan(db200_context* ctx, const TilePlan& T) {
   DB200_CUDA(ctx, err);
   prof_end(ctx, e0);
   count_launch(ctx);
+  if (T.red_m > 0) {
+    const dim3 grid((unsigned)((T.red_m + 255) / 256), (unsigned)std::min(T.red_l, 256), (unsigned)T.count);
+    sum_slabs_kernel<<<grid, 256, 0, ctx->stream>>>(static_cast<const TileInst*>(T.table));
+    DB200_CUDA(ctx, cudaGetLastError());
+    count_launch(ctx);
+  }
   return DB200_OK;
+}
+
+// Length in j tiles of the ranges (multiples of `unit`) that `row_blocks` work items of n_jtiles tiles each are cut
+// into so that they fill the CTA pairs: the least waves x (tiles of a range + per_item) + per_split x (ranges > 1), in
+// units of one tile's time.  A row block count a little above a multiple of the pairs otherwise leaves most of them
+// idle in its last wave, and a small one from the start.  Whole and cut, us: promoted sketch 4096 x 4096, l = 138, 132 and
+// 58; 15005 x 30011, l = 272, 1671 and 1406; 5000 x 60000, l = 100, 1552 and 462; kernel block 8192 x 8192 (TMA stores) 148
+// and 89; nearest neighbours 4096 x 4096, 120 and 71.  Where the whole one is chosen (131072 rows) a cut costs 2 to 18 %.
+int tile_split(const db200_context* ctx, int row_blocks, int n_jtiles, int unit, int per_item, int per_split,
+               int max_ranges) {
+  const int pairs = std::max(1, ctx->num_sms / 2);
+  int best_len = n_jtiles;
+  long long best = -1;
+  for (int s = 1; s <= max_ranges; ++s) {
+    const int len = round_up((n_jtiles + s - 1) / s, unit);
+    if (len >= n_jtiles && s > 1) continue;
+    const int ranges = (n_jtiles + len - 1) / len;
+    const long long waves = ((long long)row_blocks * ranges + pairs - 1) / pairs;
+    const long long cost = waves * (std::min(len, n_jtiles) + per_item) + (ranges > 1 ? per_split : 0);
+    // a split has to give a fortieth of the time: its sums take memory and a pass of their own
+    if (best < 0 || cost + best / 40 < best) {
+      best = cost;
+      best_len = len;
+    }
+  }
+  return best_len;
+}
+
+// A single-product sketch stays whole beyond 4096 points: its one accumulation truncates ~2^-25 of its value per step
+// (1e-4 of it at 60000 points), and ranges would change a result by that much, if toward the exact one.  A promoted
+// sketch sums the same chunks either way.
+int sketch_split(const db200_context* ctx, const SketchPlan& plan, int npad_i, int npad_j, int l) {
+  if (!plan.promote && npad_j > 4096) return npad_j / BN;
+  // slabs of at most 128 MB
+  const long long most = (128LL << 20) / (4LL * std::max(l, 1) * npad_i);
+  return tile_split(ctx, npad_i / PAIR_M * plan.n_panels, npad_j / BN, plan.promote ? plan.promote : 1,
+                    plan.promote ? PROMOTED_ITEM_TILES : SKETCH_ITEM_TILES, SKETCH_SPLIT_TILES,
+                    (int)std::max(1LL, std::min(32LL, most)));
+}
+
+size_t sketch_slab_floats(const SketchPlan& plan, int npad_i, int npad_j, int l, int split_tiles) {
+  const int ranges = (npad_j / BN + split_tiles - 1) / split_tiles;
+  return ranges > 1 ? (size_t)ranges * l * npad_i : 0;
 }
 
 int launch_rbf_tiles(db200_context* ctx, int mode, const PackedPoints& pi, const PackedPoints& pj, const float* yi,
@@ -1173,6 +1445,7 @@ int launch_rbf_tiles(db200_context* ctx, int mode, const PackedPoints& pi, const
   J.gamma = gamma;
   J.out = out;
   J.ldo = ldo;
+  if (mode == RBF_MODE_KBLOCK) J.split_tiles = tile_split(ctx, pi.npad / PAIR_M, pj.npad / BN, 1, 1, 0);
   TilePlan T;
   int st = prepare_rbf_tiles(ctx, mode, &J, 1, table_storage, table_capacity, &T);
   if (st) return st;
@@ -1204,13 +1477,15 @@ void exact_panel_jobs(const TileJob& base, std::vector<TileJob>& out) {
     J.om_lo = plan.lrows;  // lo rows of the whole packed operand follow its plan.lrows hi rows
     J.l = std::min(w, l - off);
     J.out = base.out + (size_t)off * base.ldo;
+    if (base.slab) J.slab = base.slab + (size_t)off * base.slab_ld;
     out.push_back(J);
     off += w;
   }
 }
 
 int launch_rbf_sketch_exact(db200_context* ctx, const PackedPoints& pi, const PackedPoints& pj, const float* yi,
-                            const void* op, const SketchPlan& plan, int l, float gamma, float* out, int ldo) {
+                            const void* op, const SketchPlan& plan, int l, float gamma, float* out, int ldo,
+                            int split_tiles, float* slab) {
   TileJob base;
   base.pi = pi;
   base.pj = pj;
@@ -1222,6 +1497,7 @@ int launch_rbf_sketch_exact(db200_context* ctx, const PackedPoints& pi, const Pa
   base.gamma = gamma;
   base.out = out;
   base.ldo = ldo;
+  base.set_split(split_tiles, slab);
   std::vector<TileJob> jobs;
   exact_panel_jobs(base, jobs);
   TilePlan T;
