@@ -115,26 +115,28 @@ struct LaunchArgs {
   int nkc_max, panel_max;  // shared-memory layout covers every instance
   int om_mult;           // Omega stage copies: 1, or 2 when an instance loads hi and lo rows (comp = 2)
   int kblock;            // KBLOCK and KNN: 1 (labels / shared bounds); 2 when KBLOCK tiles leave by TMA stores (tm1[2])
+  int yacc;              // promoted chunks are summed in shared memory
   int* status;
 };
 
 struct SmemLayout {
   int om_stage;  // bytes of one Omega stage in one CTA: (panel / 2) rows x 128 B, twice with lo rows
-  size_t off_xi, off_xj, off_om, off_st, off_sj, off_bar, total;
+  size_t off_xi, off_xj, off_om, off_st, off_acc, off_sj, off_bar, total;
 };
 // per epilogue warp: two tiles' column norms; KBLOCK: as much again for labels, KNN: a 64-bit shared bound per row
 constexpr int SJ_BYTES = NUM_EPI_WARPS * 2 * EPI_COLS * 4;
 constexpr int ST_WARP = 32 * EPI_COLS * 4;                  // KBLOCK: an epilogue warp's 32 rows x 32 columns, fp32
 
 __host__ __device__ inline SmemLayout make_layout(int nkc, int panel, int nsx, int nso, int om_mult,
-                                                   int kblock) {
+                                                   int kblock, int yacc) {
   SmemLayout L;
   L.om_stage = (panel / 2) * 128 * om_mult;
   L.off_xi = 0;
   L.off_xj = L.off_xi + (size_t)nkc * XI_CHUNK;
   L.off_om = L.off_xj + (size_t)nsx * XJ_CHUNK;
   L.off_st = L.off_om + (size_t)nso * L.om_stage;
-  L.off_sj = L.off_st + (kblock == 2 ? NUM_EPI_WARPS * ST_WARP : 0);
+  L.off_acc = L.off_st + (kblock == 2 ? NUM_EPI_WARPS * ST_WARP : 0);
+  L.off_sj = L.off_acc + (yacc ? (size_t)panel * BM * 4 : 0);
   L.off_bar = L.off_sj + (kblock ? 2 : 1) * SJ_BYTES;
   L.total = L.off_bar + BAR_BYTES;
   return L;
@@ -355,43 +357,68 @@ __device__ __forceinline__ void red_add_f32(float* p, float v) {
   asm volatile("red.global.add.f32 [%0], %1;" ::"l"(p), "f"(v) : "memory");
 }
 
-// Drain of the sketch accumulator by one epilogue warp: its 32 rows (TMEM lanes from t_lane) x panel/4 columns,
-// 8 columns per TMEM load batch.  accumulate: add into Y with fp32 reductions (red.global.add, round to nearest,
-// performed in L2) instead of storing.  A reduction does not wait for the old value, so the drain costs no global
-// load latency (a load-add-store drain made the pass 2x slower).  Every element has one owner thread, whose first
-// chunk stores and later chunks add, in program order to the same address.  Kept out of line: its registers
-// would otherwise stay reserved across the epilogue's exp loop.
-__device__ __noinline__ void drain_sketch_chunk(const TileInst* I, int item, int i, int qc,
-                                                uint32_t t_lane_base, bool accumulate) {
+// Drain of the sketch accumulator by one epilogue warp: its 32 rows (TMEM lanes from t_lane) x panel/4 columns, 8
+// columns per TMEM load batch.  The accumulator is handed back (y_empty, the leader's barrier) once the last batch is in
+// registers.  A promoted pass closes a chunk every `promote` tiles and sums the chunks in fp32 with round to nearest:
+//   acc (shared memory, [column][128 rows], this thread's elements its own): the first chunk stores, later ones add, and
+//     the item's last one leaves the sum in Y;
+//   without room for it: fp32 reductions into Y, performed in L2 (red.global.add; the first chunk stores).  Their L2
+//     traffic, n / 256 times the size of Y, set the pace of such a pass: 3.6 us for a chunk of 128 rows x 176 columns per
+//     CTA, during which its sketch MMA waits.
+// Either way an element has one owner thread.  Kept out of line: its registers would otherwise stay reserved across the
+// epilogue's exp loop (and no wider batches: what it uses, the loop's callers spill).
+__device__ __noinline__ void drain_sketch_chunk(const TileInst* I, int item, int i, int qc, uint32_t t_lane_base,
+                                                bool first, bool last, float* acc, uint32_t y_empty) {
   int pn = 0, sp = 0;
   if (I->n_panels * I->n_splits > 1) {  // (the divisions of item_pos cost 3 % of a pass that drains every two tiles)
     const int rest = (item - I->item_begin) / I->n_itiles;
     pn = rest % I->n_panels;
     sp = rest / I->n_panels;
   }
-  const int m = I->m;
-  float* const out_i = I->out + sp * I->split_stride + i;
-  const long long ldo = I->ldo;
-  const float y_i = (i < m && I->yi) ? I->yi[i] : 1.0f;
-  const int panel = I->panel, l = I->l;
+  const int panel = I->panel;
   const int quarter = panel / 4;  // panel is a multiple of 16
+  const bool row = i < I->m;
+  const float y_i = (row && I->yi) ? I->yi[i] : 1.0f;
+  const int col0 = pn * panel + qc * quarter;
+  const long long ldo = I->ldo;
+  float* out = I->out + sp * I->split_stride + (long long)col0 * ldo + i;
+  const int ncols = row ? min(quarter, I->l - col0) : 0;  // columns of Y this thread writes
+  const bool to_y = !acc || last;
+  if (acc) acc += qc * quarter * BM;
   for (int cc = 0; cc < quarter; cc += 8) {
     float yv[8];
     const int nc = min(8, quarter - cc);  // 4 or 8
     const uint32_t ta = t_lane_base + I->tmem_y + qc * quarter + cc;
     tmem_ld4(ta, yv);
     if (nc > 4) tmem_ld4(ta + 4, yv + 4);
-    tmem_wait_ld();
-    if (i < m) {
-      const int col0 = pn * panel + qc * quarter + cc;
+    if (acc && !first) {
+      float s[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) s[e] = e < nc ? acc[(cc + e) * BM] : 0.0f;
+      tmem_wait_ld();
+#pragma unroll
+      for (int e = 0; e < 8; ++e) yv[e] += s[e];
+    } else {
+      tmem_wait_ld();
+    }
+    if (cc + nc == quarter) {
+      tc_fence_before();
+      __syncwarp();
+      if (threadIdx.x % 32 == 0) mbar_arrive_remote(y_empty);
+    }
+    if (to_y) {
 #pragma unroll
       for (int e = 0; e < 8; ++e) {
-        if (e < nc && col0 + e < l) {
-          float* dst = out_i + (size_t)(col0 + e) * ldo;
-          if (accumulate) red_add_f32(dst, y_i * yv[e]);
-          else *dst = y_i * yv[e];
+        if (cc + e < ncols) {
+          float* dst = out + (cc + e) * ldo;
+          if (acc || first) *dst = y_i * yv[e];
+          else red_add_f32(dst, y_i * yv[e]);
         }
       }
+    } else {
+#pragma unroll
+      for (int e = 0; e < 8; ++e)
+        if (e < nc) acc[(cc + e) * BM] = yv[e];
     }
   }
 }
@@ -408,7 +435,7 @@ template <int MODE, bool LEAN>
 __global__ void __launch_bounds__(NUM_THREADS, 1) rbf_tile_kernel(const __grid_constant__ LaunchArgs args) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  const SmemLayout L = make_layout(args.nkc_max, args.panel_max, args.nsx, args.nso, args.om_mult, args.kblock);
+  const SmemLayout L = make_layout(args.nkc_max, args.panel_max, args.nsx, args.nso, args.om_mult, args.kblock, args.yacc);
   const int nsx = args.nsx, nso = args.nso;
   const uint32_t s_xi = smem_u32(smem + L.off_xi);
   const uint32_t s_xj = smem_u32(smem + L.off_xj);
@@ -659,14 +686,14 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) rbf_tile_kernel(const __grid_c
       float best[8];  // KNN: this row's 8 smallest squared distances in this column quarter, ascending
 #pragma unroll
       for (int t = 0; t < 8; ++t) best[t] = INFINITY;
-      bool pending_drain = false, pending_acc = false;
-      auto drain = [&](bool accumulate) -> bool {
+      bool pending_drain = false;
+      int chunks = 0;  // of this item, drained
+      auto drain = [&](bool first, bool last) -> bool {
         if (!__all_sync(0xffffffffu, mbar_wait(bar(B_Y_FULL), ydone & 1, abort_flag))) return false;
         tc_fence_after();
-        drain_sketch_chunk(I, item, i, qc, tmem_base + t_lane, accumulate);
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive_remote(lbar(B_Y_EMPTY));
+        drain_sketch_chunk(I, item, i, qc, tmem_base + t_lane, first, last,
+                           promote && args.yacc ? reinterpret_cast<float*>(smem + L.off_acc) + row : nullptr,
+                           lbar(B_Y_EMPTY));
         ++ydone;
         return true;
       };
@@ -796,13 +823,14 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) rbf_tile_kernel(const __grid_c
           // Up to two drains here (one call site): the chunk closed by the previous tile, then, on the item's last
           // tile, the chunk this tile closes (nothing follows it to overlap with).  The first chunk of an item
           // stores, later chunks add.
-          const bool closes = promote && ((jt + 1) % promote == 0 || jt == njt - 1);
-          bool dq[2] = {pending_drain, closes && jt == njt - 1};
-          bool da[2] = {pending_acc, jt >= promote};
-          pending_drain = closes && jt < njt - 1;
-          pending_acc = jt >= promote;
-          for (int dd = 0; dd < 2 && ok; ++dd)
-            if (dq[dd] && !drain(da[dd])) ok = false;
+          const bool closes = promote && ((jt + 1) % promote == 0 || jt == njt - 1), end = jt == njt - 1;
+          const bool dq[2] = {pending_drain, closes && end};
+          pending_drain = closes && !end;
+          for (int dd = 0; dd < 2 && ok; ++dd) {
+            if (!dq[dd]) continue;
+            if (!drain(chunks == 0, dd == 1)) ok = false;
+            ++chunks;
+          }
           if (!ok) break;
         } else if (MODE == RBF_MODE_KNN) {
           // (the list was updated above)
@@ -864,7 +892,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) rbf_tile_kernel(const __grid_c
         for (int t = 0; t < 8; ++t) o[t] = best[t];
       }
       if (MODE == RBF_MODE_SKETCH && !promote) {
-        if (!drain(false)) { ok = false; break; }
+        if (!drain(true, true)) { ok = false; break; }
       }
     }
     if (MODE == RBF_MODE_KBLOCK && lane == 0) bulk_wait_all();  // this thread's stores have left its shared memory
@@ -1306,18 +1334,33 @@ int prepare_rbf_tiles(db200_context* ctx, int mode, const TileJob* jobs, int cou
   T.panel_max = panel_max;
   T.nso = (mode == RBF_MODE_SKETCH) ? MAX_NSO : 0;
   T.lean = (mode == RBF_MODE_SKETCH);
+  int chunk = 0;  // shortest promoted chunk
+  for (int b = 0; b < count; ++b) {
+    const int p = host[(size_t)b].promote;
+    if (p > 0) chunk = chunk > 0 ? std::min(chunk, p) : p;
+  }
   for (int b = 0; b < count; ++b) T.lean = T.lean && host[(size_t)b].comp == 0 && host[(size_t)b].promote == 0;
   T.om_mult = om_mult;
   T.kblock = kblock;
-  {  // the Xj ring takes whatever shared memory is left
-    const SmemLayout L0 = make_layout(nkc_max, panel_max, 0, T.nso, om_mult, T.kblock);
+  // Promoted chunks are summed in shared memory where the panel's sums leave room for the rings: two Omega stages and 3
+  // Xj stages for chunks of two tiles (256 points; 40000 x 40000, d = 128, l = 528: 10.0 -> 8.9 ms; l = 256, five stages:
+  // 5.9 -> 4.4 ms), 6 for longer ones, which drain seldom and need their rings more (with 3 stages 6.9 -> 7.7 ms).  The
+  // Xj ring takes whatever is left.
+  auto ring = [&](int yacc, int nso) -> int {
+    const SmemLayout L0 = make_layout(nkc_max, panel_max, 0, nso, om_mult, T.kblock, yacc);
     const long long left = (long long)SMEM_LIMIT - 1024 - (long long)L0.total;
-    int nsx = (int)(left / XJ_CHUNK);
-    if (nsx > MAX_NSX) nsx = MAX_NSX;
-    if (nsx < 2) return fail(ctx, DB200_ERR_UNSUPPORTED, "rbf tiles: shared memory plan does not fit");
-    T.nsx = nsx;
-  }
-  T.smem = make_layout(nkc_max, panel_max, T.nsx, T.nso, om_mult, T.kblock).total + 1024;
+    return left < 0 ? 0 : (int)std::min<long long>(MAX_NSX, left / XJ_CHUNK);
+  };
+  T.yacc = 0;
+  if (chunk > 0)
+    for (int nso = MAX_NSO; nso >= 2 && !T.yacc; --nso)
+      if (ring(1, nso) >= (chunk <= 2 ? 3 : 6)) {
+        T.yacc = 1;
+        T.nso = nso;
+      }
+  T.nsx = ring(T.yacc, T.nso);
+  if (T.nsx < 2) return fail(ctx, DB200_ERR_UNSUPPORTED, "rbf tiles: shared memory plan does not fit");
+  T.smem = make_layout(nkc_max, panel_max, T.nsx, T.nso, om_mult, T.kblock, T.yacc).total + 1024;
   {
     const int max_clusters = ctx->num_sms / 2;
     cudaError_t e =
@@ -1363,6 +1406,7 @@ int launch_rbf_plan(db200_context* ctx, const TilePlan& T) {
   a.nso = T.nso;
   a.om_mult = T.om_mult;
   a.kblock = T.kblock;
+  a.yacc = T.yacc;
   a.nkc_max = T.nkc_max;
   a.panel_max = T.panel_max;
   a.status = ctx->d_status;
