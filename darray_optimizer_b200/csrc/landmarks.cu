@@ -241,76 +241,202 @@ __global__ void radix_compact_kernel(int n, const float* __restrict__ keys, unsi
 }
 
 // ------------------------------------------------------------------ MLP
-// C(i, j) = sum_k A(i, k) B(k, j), A(i, k) = A[i*a_i + k*a_k], B(k, j) = B[k*b_k + j*b_j], 64 x 64 tiles, 16-deep
-// stages, 256 threads with 4 x 4 outputs each, fp32 accumulation.  grid.z splits K (EPI_ATOMIC only).
-enum { EPI_HIDDEN = 0, EPI_OUT = 1, EPI_DH = 2, EPI_ATOMIC = 3 };
-constexpr int MT = 64, MK = 16;
+// C(i, j) = sum_k A(i, k) B(k, j) in fp32, every output one fused-multiply-add chain over ascending k (activations are
+// rounded to bf16 between layers, so another order of the sums would move later layers by whole bf16 steps).
+// AK / BK: k is the contiguous index (A[i * lda + k], B[j * ldb + k]), else i / j is (A[k * lda + i], B[k * ldb + j]).
+//
+// Bound by the FP32 pipe.  128 x 128 per CTA of 256 threads; a warp owns 64 x 32, a lane 8 x 8 as two by two 4 x 4 blocks,
+// so that a k step is four conflict-free 16-byte shared loads for 32 packed multiply-adds (fma.rn.f32x2: two outputs per
+// instruction, each rounded as fmaf).  Stages of 16 k are fetched into registers one stage ahead (16-byte pieces where
+// the operand's rows allow it), converted to fp32 and parked [k][row] in a double buffer.  One training
+// step's products over 16384 rows of the 66 -> 256 x 3 -> 1 net take 425 us (37 TFLOP/s); 64 x 64 tiles with 4 x 4 outputs
+// and scalar loads took 800, 128 x 256 tiles (fewer shared loads, one CTA per SM) 455.  grid.z splits k (EPI_ATOMIC only).
+enum { EPI_HIDDEN = 0, EPI_DH = 2, EPI_ATOMIC = 3 };
+constexpr int MT = 128, MK = 16, MLD = MT + 4;
 
-template <typename T>
-__device__ __forceinline__ float tof(T v) { return (float)v; }
-template <>
-__device__ __forceinline__ float tof<__nv_bfloat16>(__nv_bfloat16 v) { return __bfloat162float(v); }
+__device__ __forceinline__ float tof(float v) { return v; }
+__device__ __forceinline__ float tof(__nv_bfloat16 v) { return __bfloat162float(v); }
 
-template <typename TA, typename TB, int EPI>
-__global__ void __launch_bounds__(256) mlp_gemm_kernel(int M, int N, int K, const TA* __restrict__ A, long long a_i,
-                                                       long long a_k, const TB* __restrict__ B, long long b_k,
-                                                       long long b_j, const float* __restrict__ bias,
-                                                       const __nv_bfloat16* __restrict__ H, long long ldh, void* Cv,
-                                                       long long ldc, int k_per_split) {
-  __shared__ float sA[MK][MT + 1];
-  __shared__ float sB[MK][MT + 1];
+// One operand's stage: entries (r0 + 0..127, k0 + 0..15), zero outside (rows, k1).  8 values per thread.
+template <typename T, bool KC, bool VEC>
+__device__ __forceinline__ void mlp_fetch(float (&v)[8], const T* X, long long ld, int r0, int rows, int k0, int k1) {
+  const int t = threadIdx.x;
+  const int r = KC ? t / 2 : (t % 16) * 8, k = KC ? (t % 2) * 8 : t / 16;  // first of 8 along the contiguous index
+  const T* p = X + (KC ? (long long)(r0 + r) * ld + k0 + k : (long long)(k0 + k) * ld + r0 + r);
+  const bool in = KC ? r0 + r < rows : k0 + k < k1;
+  const int left = in ? (KC ? k1 - (k0 + k) : rows - (r0 + r)) : 0;
+  if (VEC && left >= 8) {
+    if constexpr (sizeof(T) == 2) {
+      const uint4 q = __ldg(reinterpret_cast<const uint4*>(p));
+      const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {  // bf16 is the upper half of an fp32
+        v[2 * e] = __uint_as_float(w[e] << 16);
+        v[2 * e + 1] = __uint_as_float(w[e] & 0xffff0000u);
+      }
+    } else {
+      const float4 a = __ldg(reinterpret_cast<const float4*>(p)), b = __ldg(reinterpret_cast<const float4*>(p) + 1);
+      v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w, v[4] = b.x, v[5] = b.y, v[6] = b.z, v[7] = b.w;
+    }
+  } else {
+#pragma unroll
+    for (int e = 0; e < 8; ++e) v[e] = e < left ? tof(p[e]) : 0.f;
+  }
+}
+template <bool KC>
+__device__ __forceinline__ void mlp_park(float (*s)[MLD], const float (&v)[8]) {
+  const int t = threadIdx.x;
+  if (KC) {
+#pragma unroll
+    for (int e = 0; e < 8; ++e) s[(t % 2) * 8 + e][t / 2] = v[e];
+  } else {
+    float4* d = reinterpret_cast<float4*>(&s[t / 16][(t % 16) * 8]);
+    d[0] = make_float4(v[0], v[1], v[2], v[3]);
+    d[1] = make_float4(v[4], v[5], v[6], v[7]);
+  }
+}
+
+__device__ __forceinline__ unsigned long long pack2(float lo, float hi) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ float2 unpack2(unsigned long long v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+
+template <typename TA, typename TB, bool AK, bool BK, bool VEC, int EPI>
+__global__ void __launch_bounds__(256, 2) mlp_gemm_kernel(int M, int N, int K, const TA* __restrict__ A, long long lda,
+                                                          const TB* __restrict__ B, long long ldb,
+                                                          const float* __restrict__ bias,
+                                                          const __nv_bfloat16* __restrict__ H, void* Cv, long long ldc,
+                                                          int k_per_split) {
+  __shared__ __align__(16) float sA[2][MK][MLD];
+  __shared__ __align__(16) float sB[2][MK][MLD];
   const int i0 = blockIdx.x * MT, j0 = blockIdx.y * MT;
   const int kb = blockIdx.z * k_per_split, ke = min(K, kb + k_per_split);
-  const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-  float acc[4][4] = {};
-  for (int k0 = kb; k0 < ke; k0 += MK) {
+  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+  const int ri = 64 * (warp % 2) + 4 * (lane / 4), cj = 32 * (warp / 2) + 4 * (lane % 4);  // + 32 rows, + 16 columns
+  unsigned long long acc[8][4];  // rows ri + 0..3, ri + 32 + 0..3; column pairs cj + {0,1}, {2,3}, + 16 + {0,1}, {2,3}
 #pragma unroll
-    for (int s = 0; s < 4; ++s) {
-      const int e = threadIdx.x + 256 * s;
-      // walk the unit-stride index fastest for coalesced loads
-      int ii, kk;
-      if (a_k == 1) { kk = e % MK; ii = e / MK; } else { ii = e % MT; kk = e / MT; }
-      const int gi = i0 + ii, gk = k0 + kk;
-      sA[kk][ii] = (gi < M && gk < ke) ? tof(A[gi * a_i + gk * a_k]) : 0.f;
-      int jj, kk2;
-      if (b_k == 1) { kk2 = e % MK; jj = e / MK; } else { jj = e % MT; kk2 = e / MT; }
-      const int gj = j0 + jj, gk2 = k0 + kk2;
-      sB[kk2][jj] = (gj < N && gk2 < ke) ? tof(B[gk2 * b_k + gj * b_j]) : 0.f;
+  for (int a = 0; a < 8; ++a)
+#pragma unroll
+    for (int b = 0; b < 4; ++b) acc[a][b] = 0ull;
+  float va[8], vb[8];
+  mlp_fetch<TA, AK, VEC>(va, A, lda, i0, M, kb, ke);
+  mlp_fetch<TB, BK, VEC>(vb, B, ldb, j0, N, kb, ke);
+  mlp_park<AK>(sA[0], va);
+  mlp_park<BK>(sB[0], vb);
+  __syncthreads();
+  int buf = 0;
+  for (int k0 = kb; k0 < ke; k0 += MK, buf ^= 1) {
+    const bool more = k0 + MK < ke;
+    if (more) {
+      mlp_fetch<TA, AK, VEC>(va, A, lda, i0, M, k0 + MK, ke);
+      mlp_fetch<TB, BK, VEC>(vb, B, ldb, j0, N, k0 + MK, ke);
     }
-    __syncthreads();
 #pragma unroll
     for (int t = 0; t < MK; ++t) {
-      float av[4], bv[4];
+      const float4 a0 = *reinterpret_cast<const float4*>(&sA[buf][t][ri]);
+      const float4 a1 = *reinterpret_cast<const float4*>(&sA[buf][t][ri + 32]);
+      const ulonglong2 b0 = *reinterpret_cast<const ulonglong2*>(&sB[buf][t][cj]);
+      const ulonglong2 b1 = *reinterpret_cast<const ulonglong2*>(&sB[buf][t][cj + 16]);
+      const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+      const unsigned long long bv[4] = {b0.x, b0.y, b1.x, b1.y};
 #pragma unroll
-      for (int a = 0; a < 4; ++a) av[a] = sA[t][ty * 4 + a];
+      for (int a = 0; a < 8; ++a) {
+        const unsigned long long aa = pack2(av[a], av[a]);
 #pragma unroll
-      for (int b = 0; b < 4; ++b) bv[b] = sB[t][tx * 4 + b];
-#pragma unroll
-      for (int a = 0; a < 4; ++a)
-#pragma unroll
-        for (int b = 0; b < 4; ++b) acc[a][b] = fmaf(av[a], bv[b], acc[a][b]);
+        for (int b = 0; b < 4; ++b)
+          asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc[a][b]) : "l"(aa), "l"(bv[b]));
+      }
+    }
+    if (more) {  // the other buffer was last read one stage ago, before the barrier that ended it
+      mlp_park<AK>(sA[buf ^ 1], va);
+      mlp_park<BK>(sB[buf ^ 1], vb);
     }
     __syncthreads();
   }
 #pragma unroll
-  for (int a = 0; a < 4; ++a) {
-    const int i = i0 + ty * 4 + a;
+  for (int a = 0; a < 8; ++a) {
+    const int i = i0 + ri + (a < 4 ? a : 28 + a);
     if (i >= M) continue;
 #pragma unroll
     for (int b = 0; b < 4; ++b) {
-      const int j = j0 + tx * 4 + b;
-      if (j >= N) continue;
-      const float v = acc[a][b];
-      if (EPI == EPI_HIDDEN) {
-        static_cast<__nv_bfloat16*>(Cv)[i * ldc + j] = __float2bfloat16_rn(fmaxf(v + bias[j], 0.f));
-      } else if (EPI == EPI_OUT) {
-        static_cast<float*>(Cv)[i * ldc + j] = v + bias[j];
-      } else if (EPI == EPI_DH) {
-        static_cast<float*>(Cv)[i * ldc + j] = (__bfloat162float(H[i * ldh + j]) > 0.f) ? v : 0.f;
-      } else {
-        atomicAdd(static_cast<float*>(Cv) + i * ldc + j, v);
+      const float2 o = unpack2(acc[a][b]);
+      const int j = j0 + cj + (b < 2 ? 2 * b : 12 + 2 * b);
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        if (j + e >= N) continue;
+        const float v = e ? o.y : o.x;
+        const long long at = i * ldc + j + e;
+        if (EPI == EPI_HIDDEN) {
+          static_cast<__nv_bfloat16*>(Cv)[at] = __float2bfloat16_rn(fmaxf(v + bias[j + e], 0.f));
+        } else if (EPI == EPI_DH) {
+          static_cast<float*>(Cv)[at] = (__bfloat162float(H[at]) > 0.f) ? v : 0.f;
+        } else {
+          atomicAdd(static_cast<float*>(Cv) + at, v);
+        }
       }
     }
+  }
+}
+
+// The output layer (one unit).  Forward: out_i = sum_k H(i, k) w_k + b, one chain per row, a thread per row.
+template <bool VEC>
+__global__ void __launch_bounds__(128) mlp_out_kernel(int m, int K, const __nv_bfloat16* __restrict__ H,
+                                                      const __nv_bfloat16* __restrict__ w, const float* __restrict__ b,
+                                                      float* __restrict__ out) {
+  extern __shared__ float sw[];
+  for (int k = threadIdx.x; k < K; k += blockDim.x) sw[k] = tof(w[k]);
+  __syncthreads();
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= m) return;
+  const __nv_bfloat16* h = H + (long long)i * K;
+  float acc = 0.f;
+  int k = 0;
+  if (VEC) {
+#pragma unroll 4
+    for (; k + 8 <= K; k += 8) {
+      const uint4 q = __ldg(reinterpret_cast<const uint4*>(h + k));
+      const uint32_t u[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        acc = fmaf(__uint_as_float(u[e] << 16), sw[k + 2 * e], acc);
+        acc = fmaf(__uint_as_float(u[e] & 0xffff0000u), sw[k + 2 * e + 1], acc);
+      }
+    }
+  }
+  for (; k < K; ++k) acc = fmaf(tof(h[k]), sw[k], acc);
+  out[i] = acc + *b;
+}
+// Backward of the output layer in one pass over H (m x K): dw_k += sum_i d_i H(i, k), db += sum_i d_i and
+// dX(i, k) = d_i w_k where H(i, k) > 0.  A thread per column k, the rows split over blockIdx.y.
+__global__ void __launch_bounds__(256) mlp_out_backward_kernel(int m, int K, const float* __restrict__ d,
+                                                               const __nv_bfloat16* __restrict__ H,
+                                                               const __nv_bfloat16* __restrict__ w, int rows,
+                                                               float* __restrict__ dX, float* dw, float* db) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  const int r0 = blockIdx.y * rows, r1 = min(m, r0 + rows);
+  if (k < K) {
+    const float wk = tof(w[k]);
+    float s = 0.f;
+#pragma unroll 4
+    for (int i = r0; i < r1; ++i) {
+      const float h = tof(H[(long long)i * K + k]), di = __ldg(d + i);
+      s = fmaf(di, h, s);
+      dX[(long long)i * K + k] = h > 0.f ? di * wk : 0.f;
+    }
+    atomicAdd(dw + k, s);
+  }
+  if (blockIdx.x == 0 && threadIdx.x < 32) {
+    float s = 0.f;
+    for (int i = r0 + threadIdx.x; i < r1; i += 32) s += d[i];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (threadIdx.x == 0) atomicAdd(db, s);
   }
 }
 
@@ -334,13 +460,14 @@ __global__ void mse_kernel(int m, const float* __restrict__ out, const float* __
   for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
   if (threadIdx.x % 32 == 0) atomicAdd(loss, s);
 }
-// g[j] += sum_i dY[i*N + j]
-__global__ void colsum_kernel(int m, int N, const float* __restrict__ dY, float* __restrict__ g) {
-  const int j = blockIdx.x * 32 + threadIdx.x % 32;
+// g[j] += sum_i dY[i*N + j], a thread per column, the rows split over blockIdx.y
+__global__ void __launch_bounds__(256) colsum_kernel(int m, int N, int rows, const float* __restrict__ dY, float* g) {
+  const int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= N) return;
+  const int r1 = min(m, ((int)blockIdx.y + 1) * rows);
   float s = 0.f;
-  for (int i = blockIdx.y * (blockDim.x / 32) + threadIdx.x / 32; i < m; i += gridDim.y * (blockDim.x / 32))
-    s += dY[(long long)i * N + j];
+#pragma unroll 8
+  for (int i = blockIdx.y * rows; i < r1; ++i) s += __ldg(dY + (long long)i * N + j);
   atomicAdd(g + j, s);
 }
 __global__ void adam_kernel(int np, float* __restrict__ w, const float* __restrict__ g, float* __restrict__ m1,
@@ -360,18 +487,24 @@ __global__ void to_bf16_kernel(int np, const float* __restrict__ w, __nv_bfloat1
   for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < np; e += gridDim.x * blockDim.x) wbf[e] = __float2bfloat16_rn(w[e]);
 }
 
-template <typename TA, typename TB, int EPI>
-int mlp_gemm(db200_context* ctx, int M, int N, int K, const TA* A, long long a_i, long long a_k, const TB* B,
-             long long b_k, long long b_j, const float* bias, const __nv_bfloat16* H, long long ldh, void* C,
-             long long ldc, int splits = 1) {
+template <typename TA, typename TB, bool AK, bool BK, int EPI>
+int mlp_gemm(db200_context* ctx, int M, int N, int K, const TA* A, long long lda, const TB* B, long long ldb,
+             const float* bias, const __nv_bfloat16* H, void* C, long long ldc, int splits = 1) {
   if (M <= 0 || N <= 0) return DB200_OK;
   int kps = (K + splits - 1) / splits;
   kps = round_up(kps < MK ? MK : kps, MK);
-  splits = (K + kps - 1) / kps;
-  dim3 grid((M + MT - 1) / MT, (N + MT - 1) / MT, splits < 1 ? 1 : splits);
+  splits = std::max(1, (K + kps - 1) / kps);
+  const dim3 grid((M + MT - 1) / MT, (N + MT - 1) / MT, splits);
   if (grid.y > 65535 || grid.z > 65535) return fail(ctx, DB200_ERR_UNSUPPORTED, "mlp: GEMM too large");
-  mlp_gemm_kernel<TA, TB, EPI><<<grid, 256, 0, ctx->stream>>>(M, N, K, A, a_i, a_k, B, b_k, b_j, bias, H, ldh, C,
-                                                             ldc, kps);
+  // 16-byte pieces: aligned bases and rows
+  const bool vec = reinterpret_cast<uintptr_t>(A) % 16 == 0 && reinterpret_cast<uintptr_t>(B) % 16 == 0 &&
+                   lda * (long long)sizeof(TA) % 16 == 0 && ldb * (long long)sizeof(TB) % 16 == 0;
+  if (vec)
+    mlp_gemm_kernel<TA, TB, AK, BK, true, EPI><<<grid, 256, 0, ctx->stream>>>(M, N, K, A, lda, B, ldb, bias, H, C, ldc,
+                                                                              kps);
+  else
+    mlp_gemm_kernel<TA, TB, AK, BK, false, EPI><<<grid, 256, 0, ctx->stream>>>(M, N, K, A, lda, B, ldb, bias, H, C, ldc,
+                                                                               kps);
   DB200_CUDA(ctx, cudaGetLastError());
   count_launch(ctx);
   return DB200_OK;
@@ -415,12 +548,19 @@ int mlp_forward_impl(db200_context* ctx, db200_mlp* net, int m, const float* F, 
     const int K = net->fan_in[l], N = net->fan_out[l];
     const __nv_bfloat16* W = net->wbf + net->off_w[l];
     const float* b = net->master + net->off_b[l];
-    if (l < net->hidden)
-      st = mlp_gemm<__nv_bfloat16, __nv_bfloat16, EPI_HIDDEN>(ctx, m, N, K, A.h[l], K, 1, W, 1, K, b, nullptr, 0,
-                                                             A.h[l + 1], N);
-    else
-      st = mlp_gemm<__nv_bfloat16, __nv_bfloat16, EPI_OUT>(ctx, m, N, K, A.h[l], K, 1, W, 1, K, b, nullptr, 0,
-                                                          A.out, N);
+    if (l < net->hidden) {
+      st = mlp_gemm<__nv_bfloat16, __nv_bfloat16, true, true, EPI_HIDDEN>(ctx, m, N, K, A.h[l], K, W, K, b, nullptr,
+                                                                         A.h[l + 1], N);
+    } else {
+      const bool vec = K % 8 == 0;  // (A.h is 256-byte aligned)
+      if (vec)
+        mlp_out_kernel<true><<<(m + 127) / 128, 128, sizeof(float) * K, ctx->stream>>>(m, K, A.h[l], W, b, A.out);
+      else
+        mlp_out_kernel<false><<<(m + 127) / 128, 128, sizeof(float) * K, ctx->stream>>>(m, K, A.h[l], W, b, A.out);
+      DB200_CUDA(ctx, cudaGetLastError());
+      count_launch(ctx);
+      st = DB200_OK;
+    }
     if (st) return st;
   }
   return DB200_OK;
@@ -435,22 +575,38 @@ int mlp_backward_impl(db200_context* ctx, db200_mlp* net, int m, const float* ta
   count_launch(ctx);
   float* dY = A.dy0;  // gradient at the output of layer l (m x fan_out[l])
   float* dX = A.dy1;
-  const int splits = std::max(1, std::min(64, m / 512));
+  // rows of one split of the sums over m: enough CTAs for two per SM, at least 64 rows each
+  auto split_rows = [&](long long tiles) -> int {
+    const long long want = std::max(1LL, 2LL * ctx->num_sms / tiles);
+    return (int)std::max(64LL, (m + want - 1) / want);
+  };
   int st;
   for (int l = net->layers - 1; l >= 0; --l) {
     const int K = net->fan_in[l], N = net->fan_out[l];
+    if (l == net->hidden) {  // one unit: its weights' and bias's gradient and dH_{l-1} in one pass
+      const int rows = split_rows((K + 255) / 256);
+      mlp_out_backward_kernel<<<dim3((K + 255) / 256, (m + rows - 1) / rows), 256, 0, ctx->stream>>>(
+          m, K, dY, A.h[l], net->wbf + net->off_w[l], rows, dX, net->grad + net->off_w[l], net->grad + net->off_b[l]);
+      DB200_CUDA(ctx, cudaGetLastError());
+      count_launch(ctx);
+      std::swap(dY, dX);
+      continue;
+    }
     // dW_l (N x K) = dY^T H_l  (sum over the m rows, split with atomics)
-    if ((st = mlp_gemm<float, __nv_bfloat16, EPI_ATOMIC>(ctx, N, K, m, dY, 1, N, A.h[l], K, 1, nullptr, nullptr, 0,
-                                                         net->grad + net->off_w[l], K, splits)))
+    const int wrows = split_rows((long long)((N + MT - 1) / MT) * ((K + MT - 1) / MT));
+    if ((st = mlp_gemm<float, __nv_bfloat16, false, false, EPI_ATOMIC>(ctx, N, K, m, dY, N, A.h[l], K, nullptr, nullptr,
+                                                                       net->grad + net->off_w[l], K,
+                                                                       (m + wrows - 1) / wrows)))
       return st;
-    colsum_kernel<<<dim3((N + 31) / 32, std::max(1, std::min(256, m / 256))), 256, 0, ctx->stream>>>(
-        m, N, dY, net->grad + net->off_b[l]);
+    const int crows = split_rows((N + 255) / 256);
+    colsum_kernel<<<dim3((N + 255) / 256, (m + crows - 1) / crows), 256, 0, ctx->stream>>>(m, N, crows, dY,
+                                                                                         net->grad + net->off_b[l]);
     DB200_CUDA(ctx, cudaGetLastError());
     count_launch(ctx);
     if (l > 0) {
       // dH_{l-1} (m x K) = (dY W_l) masked by ReLU'(H_{l-1})
-      if ((st = mlp_gemm<float, __nv_bfloat16, EPI_DH>(ctx, m, K, N, dY, N, 1, net->wbf + net->off_w[l], K, 1,
-                                                      nullptr, A.h[l], K, dX, K)))
+      if ((st = mlp_gemm<float, __nv_bfloat16, true, false, EPI_DH>(ctx, m, K, N, dY, N, net->wbf + net->off_w[l], K,
+                                                                   nullptr, A.h[l], dX, K)))
         return st;
       std::swap(dY, dX);
     }
