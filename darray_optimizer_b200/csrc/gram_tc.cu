@@ -19,7 +19,14 @@
 //     into M with FP64 atomics (the n dimension is split across CTAs).
 //
 // The result differs from the exact Z~^T Z~ by the dropped groups and the truncation only, about 2e-8, 3e-10,
-// 3e-12, 3e-14 of ||Z~_p|| ||Z~_q|| for KS = 5, 6, 7, 8 (measured), next to FP64 accumulation's ~1e-16 sqrt(n).  The
+// 3e-12, 3e-14 of ||Z~_p|| ||Z~_q|| for KS = 5, 6, 7, 8 (measured), next to FP64 accumulation's ~1e-16 sqrt(n).
+//
+// BITS = 8 (the barrier's and CholeskyQR2's form): seven base-256 digits in [-128, 127] of round(x 2^54), x as above.
+// They carry 54 bits in 7 slices and 28 products instead of 56 bits in 8 slices and 36 products, rounded instead of
+// truncated, and the kept groups end 2^-56 below the first (2^-49 at base 128), so the error is near the FP64 Gram's
+// (4e-16 to 2e-15 where 8 base-128 digits give 3e-15 to 1.5e-14).  The digits of an integer v are the bytes of
+// v + 128 (256^7 - 1) / 255, each less 128: one addition instead of eight shifts and masks.  The s32 sums stay exact:
+// 7 * 16384 * 128^2 < 2^31.  The
 // kernels are instantiated for each KS; the barrier solver
 // still refines each Newton step against the exact FP64 operator and falls back to the FP64 Gram if refinement
 // stalls.
@@ -29,6 +36,7 @@
 #include <algorithm>
 #include <mutex>
 
+#include "barrier.h"
 #include "internal.h"
 #include "ptx.cuh"
 
@@ -50,6 +58,7 @@ constexpr int TMEM_COLS = 512;                 // KS * TN columns of s32 groups 
 constexpr int THREADS = 192;                   // warp 0 TMA, warp 1 MMA, warps 2..5 epilogue
 static_assert(KS_MAX * TN <= TMEM_COLS, "group accumulators exceed TMEM");
 static_assert((long long)KS_MAX * MAX_CHUNKS * KB * 127 * 127 < (1LL << 31), "s32 group sums could overflow");
+static_assert(7LL * MAX_CHUNKS * KB * 128 * 128 < (1LL << 31), "s32 group sums could overflow");
 constexpr int SLICE_CTAS = 4;                  // CTAs (of 256 threads x 16 rows) per scaling chunk
 static_assert(SLICE_CTAS * 256 * 16 == CH && CH / SLICE_CTAS == 256 * 16, "slice_kernel covers a chunk per cluster");
 
@@ -72,7 +81,7 @@ __device__ __forceinline__ int exp_above(double m) {
   return bits == 0 ? 0 : biased - 1022;
 }
 
-template <int KS>
+template <int KS, int BITS>
 __global__ void __launch_bounds__(THREADS, 1)
     gram_i8_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b, GramArgs g) {
   constexpr int STAGE = stage_bytes<KS>();
@@ -197,14 +206,14 @@ __global__ void __launch_bounds__(THREADS, 1)
           tmem_ld16(tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(gi * TN + c0), raw);
           tmem_wait_ld();
 #pragma unroll
-          for (int e = 0; e < 16; ++e) v[e] = v[e] * 0.0078125 + (double)__float_as_int(raw[e]);
+          for (int e = 0; e < 16; ++e) v[e] = v[e] * (1.0 / (1 << BITS)) + (double)__float_as_int(raw[e]);
         }
         if (row < g.r) {
 #pragma unroll
           for (int e = 0; e < 16; ++e) {
             const int col = tj * TN + c0 + e;
             if (col < g.r && row <= col)
-              atomicAdd(g.M + (long long)col * g.ldm + row, ldexp(v[e], ep + ex[col] - 14));
+              atomicAdd(g.M + (long long)col * g.ldm + row, ldexp(v[e], ep + ex[col] - (BITS == 7 ? 14 : 12)));
           }
         }
       }
@@ -222,6 +231,88 @@ __global__ void __launch_bounds__(THREADS, 1)
 // sw[i] = sqrt(w_i) (1 without weights), computed once per Gram.
 __global__ void sqrt_weights_kernel(const double* __restrict__ w, int n, double* __restrict__ sw) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) sw[i] = w ? sqrt(w[i]) : 1.0;
+}
+
+// Largest |.| of a chunk's column from this thread's v: over the CTA, then over the cluster by distributed shared memory.
+__device__ __forceinline__ double chunk_max(double m, double* part, double* cta_max) {
+  namespace cg = cooperative_groups;
+  cg::cluster_group cluster = cg::this_cluster();
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
+  if (threadIdx.x % 32 == 0) part[threadIdx.x / 32] = m;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+#pragma unroll
+    for (int k = 1; k < 8; ++k) m = fmax(m, part[k]);
+    *cta_max = m;
+  }
+  cluster.sync();
+#pragma unroll
+  for (int k = 0; k < SLICE_CTAS; ++k) m = fmax(m, *cluster.map_shared_rank(cta_max, k));
+  cluster.sync();  // every CTA has read the others' maxima before any of them exits
+  return m;
+}
+
+// The base-256 slices (BITS = 8, KS = 7): a cluster per (column p < r, chunk c) as below, a thread four times four
+// neighbouring rows, whose bytes of one slice are one word: no staging, every warp store one whole line.  Columns past r
+// are not written: the tensor maps end at r and their loads read zeros there.  131072 x 528: 214 us; the base-128
+// form, with its digits' shifts and masks and the padding columns, takes 395.
+template <bool VEC>
+__global__ void __cluster_dims__(1, SLICE_CTAS, 1) __launch_bounds__(256)
+    slice256_kernel(const double* __restrict__ Z, long long ldz, const double* __restrict__ sw, int n, int r, int npad,
+                    int rpad, int* __restrict__ exps, int8_t* __restrict__ slices) {
+  constexpr int ROWS = CH / SLICE_CTAS, ROUNDS = ROWS / 1024, KS = 7;
+  __shared__ double part[8];
+  __shared__ double cta_max;
+  const int p = blockIdx.x, c = blockIdx.y / SLICE_CTAS, rank = blockIdx.y % SLICE_CTAS;
+  const int base = c * CH + rank * ROWS;
+  const double* col = Z + (long long)p * ldz;
+  double v[4 * ROUNDS];
+  double m = 0.0;
+#pragma unroll
+  for (int q = 0; q < ROUNDS; ++q) {
+    const int i = base + 1024 * q + 4 * threadIdx.x;
+    if (VEC && i + 4 <= n) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const double2 z = __ldg(reinterpret_cast<const double2*>(col + i) + h);
+        const double2 w = __ldg(reinterpret_cast<const double2*>(sw + i) + h);
+        v[4 * q + 2 * h] = w.x * z.x;
+        v[4 * q + 2 * h + 1] = w.y * z.y;
+      }
+    } else {
+#pragma unroll
+      for (int h = 0; h < 4; ++h) v[4 * q + h] = i + h < n ? sw[i + h] * col[i + h] : 0.0;
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < 4 * ROUNDS; ++j) m = fmax(m, fabs(v[j]));
+  m = chunk_max(m, part, &cta_max);
+  const int e = exp_above(m);
+  if (rank == 0 && threadIdx.x == 0) exps[(size_t)c * rpad + p] = e;
+  const double scale = ldexp(1.0, 54 - e);
+  const size_t slice_bytes = (size_t)r * npad;
+#pragma unroll
+  for (int q = 0; q < ROUNDS; ++q) {
+    const int i = base + 1024 * q + 4 * threadIdx.x;
+    if (i >= npad) break;  // npad is a multiple of 64: four rows are wholly inside or outside
+    uint32_t lo[4], hi[4];
+#pragma unroll
+    for (int h = 0; h < 4; ++h) {
+      const unsigned long long u = (unsigned long long)__double2ll_rn(v[4 * q + h] * scale) + 0x0080808080808080ull;
+      lo[h] = (uint32_t)u ^ 0x80808080u;
+      hi[h] = (uint32_t)(u >> 32) ^ 0x00808080u;
+    }
+    int8_t* dst = slices + (size_t)p * npad + i;
+#pragma unroll
+    for (int s = 0; s < KS; ++s) {  // slice s: byte 6 - s of the four values
+      const int b = (KS - 1 - s) & 3;
+      const uint32_t* w = KS - 1 - s >= 4 ? hi : lo;
+      const uint32_t sel = (uint32_t)b | ((uint32_t)(b + 4) << 4);
+      const uint32_t x = __byte_perm(w[0], w[1], sel), y = __byte_perm(w[2], w[3], sel);
+      *reinterpret_cast<uint32_t*>(dst + s * slice_bytes) = __byte_perm(x, y, 0x5410);
+    }
+  }
 }
 
 // One cluster of SLICE_CTAS CTAs (256 threads, 4096 rows each) per (column p < rpad, chunk c of 16384 rows).
@@ -262,19 +353,7 @@ __global__ void __cluster_dims__(1, SLICE_CTAS, 1) __launch_bounds__(256)
   double m = 0.0;
 #pragma unroll
   for (int j = 0; j < 2 * ROUNDS; ++j) m = fmax(m, fabs(v[j]));
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-  if (threadIdx.x % 32 == 0) part[threadIdx.x / 32] = m;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-#pragma unroll
-    for (int k = 1; k < 8; ++k) m = fmax(m, part[k]);
-    cta_max = m;
-  }
-  cluster.sync();
-#pragma unroll
-  for (int k = 0; k < SLICE_CTAS; ++k) m = fmax(m, *cluster.map_shared_rank(&cta_max, k));
-  cluster.sync();  // every CTA has read the others' maxima before any of them exits
+  m = chunk_max(m, part, &cta_max);
   const int e = exp_above(m);
   if (rank == 0 && threadIdx.x == 0) exps[(size_t)c * rpad + p] = e;
   if (base >= npad) return;
@@ -341,7 +420,7 @@ size_t gram_tc_scratch_bytes(int n, int r) {
 }
 
 namespace {
-template <int KS>
+template <int KS, int BITS>
 int gram_tc_run(db200_context* ctx, int n, int r, const double* Z, long long ldz, const double* w, double* M,
                 int ldm, void* scratch) {
   constexpr int STAGE = stage_bytes<KS>();
@@ -356,16 +435,22 @@ int gram_tc_run(db200_context* ctx, int n, int r, const double* Z, long long ldz
   DB200_CUDA(ctx, cudaGetLastError());
   count_launch(ctx);
   const bool vec = (reinterpret_cast<uintptr_t>(Z) % 16 == 0) && (ldz % 2 == 0);
-  if (vec)
-    slice_kernel<true, KS><<<dim3(rpad, nchunk * SLICE_CTAS), 256, 0, ctx->stream>>>(Z, ldz, sw, n, r, npad, rpad, exps,
+  const int rows = BITS == 8 ? r : rpad;  // columns of Z~ that are sliced; a tensor map reads zeros past them
+  const dim3 sgrid(rows, nchunk * SLICE_CTAS);
+  if (BITS == 8 && vec)
+    slice256_kernel<true><<<sgrid, 256, 0, ctx->stream>>>(Z, ldz, sw, n, r, npad, rpad, exps, slices);
+  else if (BITS == 8)
+    slice256_kernel<false><<<sgrid, 256, 0, ctx->stream>>>(Z, ldz, sw, n, r, npad, rpad, exps, slices);
+  else if (vec)
+    slice_kernel<true, KS><<<sgrid, 256, 0, ctx->stream>>>(Z, ldz, sw, n, r, npad, rpad, exps,
                                                                                 slices);
   else
-    slice_kernel<false, KS><<<dim3(rpad, nchunk * SLICE_CTAS), 256, 0, ctx->stream>>>(Z, ldz, sw, n, r, npad, rpad, exps,
+    slice_kernel<false, KS><<<sgrid, 256, 0, ctx->stream>>>(Z, ldz, sw, n, r, npad, rpad, exps,
                                                                                  slices);
   DB200_CUDA(ctx, cudaGetLastError());
   count_launch(ctx);
   CUtensorMap ta, tb;
-  if (!tmap_slices(&ta, slices, npad, rpad, TM, KS) || !tmap_slices(&tb, slices, npad, rpad, TN, KS))
+  if (!tmap_slices(&ta, slices, npad, rows, TM, KS) || !tmap_slices(&tb, slices, npad, rows, TN, KS))
     return fail(ctx, DB200_ERR_CUDA, "gram_tc: cuTensorMapEncodeTiled failed");
   GramArgs a;
   a.r = r;
@@ -398,11 +483,11 @@ int gram_tc_run(db200_context* ctx, int n, int r, const double* Z, long long ldz
   a.ldm = ldm;
   a.status = ctx->d_status;
   const size_t smem = NSTAGE * STAGE + 512 + 1024;
-  DB200_CUDA(ctx, cudaFuncSetAttribute(gram_i8_kernel<KS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  DB200_CUDA(ctx, cudaFuncSetAttribute(gram_i8_kernel<KS, BITS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   dim3 grid(pairs, splits);
   cudaEvent_t e0 = nullptr;
   prof_begin(ctx, &e0);
-  gram_i8_kernel<KS><<<grid, THREADS, smem, ctx->stream>>>(ta, tb, a);
+  gram_i8_kernel<KS, BITS><<<grid, THREADS, smem, ctx->stream>>>(ta, tb, a);
   DB200_CUDA(ctx, cudaGetLastError());
   prof_end(ctx, e0);
   count_launch(ctx);
@@ -410,15 +495,16 @@ int gram_tc_run(db200_context* ctx, int n, int r, const double* Z, long long ldz
 }
 }  // namespace
 
-// M (upper triangle, FP64, r x r) += Z~^T Z~ with Z~ = diag(sqrt(w)) Z from `slices` int8 digits per value (5..8;
-// error about 2e-8, 3e-10, 3e-12, 3e-14 of ||Z~_p|| ||Z~_q||).  `scratch` holds gram_tc_scratch_bytes.
+// M (upper triangle, FP64, r x r) += Z~^T Z~ with Z~ = diag(sqrt(w)) Z from `slices` int8 digits per value (5..8 base-128
+// ones: error about 2e-8, 3e-10, 3e-12, 3e-14 of ||Z~_p|| ||Z~_q||; kGramBase256: seven base-256 ones, about 1e-15).  `scratch` holds gram_tc_scratch_bytes.
 int gram_tc_weighted(db200_context* ctx, int n, int r, const double* Z, long long ldz, const double* w, double* M,
                      int ldm, void* scratch, int slices) {
   switch (slices) {
-    case 5: return gram_tc_run<5>(ctx, n, r, Z, ldz, w, M, ldm, scratch);
-    case 6: return gram_tc_run<6>(ctx, n, r, Z, ldz, w, M, ldm, scratch);
-    case 7: return gram_tc_run<7>(ctx, n, r, Z, ldz, w, M, ldm, scratch);
-    case 8: return gram_tc_run<8>(ctx, n, r, Z, ldz, w, M, ldm, scratch);
+    case kGramBase256: return gram_tc_run<7, 8>(ctx, n, r, Z, ldz, w, M, ldm, scratch);
+    case 5: return gram_tc_run<5, 7>(ctx, n, r, Z, ldz, w, M, ldm, scratch);
+    case 6: return gram_tc_run<6, 7>(ctx, n, r, Z, ldz, w, M, ldm, scratch);
+    case 7: return gram_tc_run<7, 7>(ctx, n, r, Z, ldz, w, M, ldm, scratch);
+    case 8: return gram_tc_run<8, 7>(ctx, n, r, Z, ldz, w, M, ldm, scratch);
     default: return fail(ctx, DB200_ERR_INVALID, "gram_tc: slices must be 5..8");
   }
 }

@@ -79,14 +79,14 @@ int allreduce_host(db200_context* ctx, double* d_tmp, double* vals, int k, int o
 // when the Gram is not positive definite.  W, Rinv: l x l scratch; R (l x l) receives the factor.
 int cholqr_pass(db200_context* ctx, int n, int l, const double* Yin, int ldin, double* Yout, int ldout, double* R,
                 double* Rinv, double shift_rel, int* d_pair, double* d_scalar, bool tc_gram, bool dist) {
-  // Gram W = Y^T Y (upper triangle).  tc_gram: on the int8 tensor cores, 8 signed 7-bit digits per value, exact
-  // integer products, error ~3e-14 of ||y_p|| ||y_q||; otherwise on the FP64 pipes.  The Cholesky stays FP64.
+  // Gram W = Y^T Y (upper triangle).  tc_gram: on the int8 tensor cores, seven base-256 digits per value, exact
+  // integer products, error ~1e-15 of ||y_p|| ||y_q||; otherwise on the FP64 pipes.  The Cholesky stays FP64.
   int st = DB200_OK;
   if (tc_gram) {
     void* scratch = slot_buffer(ctx, SLOT_SPARE, gram_tc_scratch_bytes(n, l));
     if (!scratch) return DB200_ERR_NOMEM;
     DB200_CUDA(ctx, cudaMemsetAsync(R, 0, sizeof(double) * (size_t)l * l, ctx->stream));
-    if ((st = gram_tc_weighted(ctx, n, l, Yin, ldin, nullptr, R, l, scratch, 8))) return st;
+    if ((st = gram_tc_weighted(ctx, n, l, Yin, ldin, nullptr, R, l, scratch, kGramBase256))) return st;
   } else if ((st = gram<double, double>(ctx, n, l, l, Yin, ldin, Yin, ldin, nullptr, 1.0, 0.0, R, l, true))) {
     return st;
   }
@@ -258,12 +258,12 @@ int svm_barrier_impl(db200_context* ctx, int n, int r, const double* Z, int ldz,
   double* gb = cv.take<double>(n);  // g + nu y (bias mode)
   void* tc_scratch = mixed ? static_cast<void*>(cv.take<char>(tc_bytes)) : nullptr;
   int refine_total = 0, fallbacks_total = 0;
-  // Tensor-core capacity matrix: 8 int8 digits per value (36 products, ~3e-14 of the column norms), after that
-  // the FP64 capacity matrix.  From r = 2048 the Gram (n r^2) outweighs the refinement passes (n r) that a coarser
+  // Tensor-core capacity matrix: seven base-256 int8 digits per value (28 products, ~1e-15 of the column norms), after
+  // that the FP64 capacity matrix.  From r = 2048 the Gram (n r^2) outweighs the refinement passes (n r) that a coarser
   // capacity matrix costs, so there the ladder starts at 6 digits (21 products, ~3e-10) while the refinement
   // converges with it.  (Measured: 6 digits first cut the barrier at n = 524288, r = 2064 from 8.6 to 7.3 s, and
   // lengthened it at r = 528 from 181 to 221 ms and at r = 1040 from 0.83 to 1.28 s.)
-  constexpr int kSlices[2] = {6, 8};
+  constexpr int kSlices[2] = {6, kGramBase256};
   int tc_level = (r >= 2048) ? 0 : 1;  // index into kSlices; 2 = FP64
   bool tc_ok = true;
   int st0 = DB200_OK;
