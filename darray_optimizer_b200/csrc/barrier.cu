@@ -4,8 +4,11 @@
 // arithmetic of tests/testsvm.cpp:243-321, with the Newton system solved as
 //   (Z Z^T + diag(D)) s = -g   ->   (I + Z^T D^-1 Z) u = -Z^T D^-1 g,   s = -D^-1 (g + Z u)
 // instead of the reference's PCG on (Z Z^T + D + n I) x = e_1 (include/dbarrier.h:84-139).
-// Every pass over Z (n x r, column major, FP64) is HBM-bound: one thread per row i reads Z[i + k*ld] for
-// k = 0..r-1, coalesced across the warp; r-vectors live in shared memory.
+// Every pass over Z (n x r, column major, FP64) is HBM-bound.  Row passes (Z times an r-vector) give a CTA 64 rows and
+// each of its 8 warps every eighth column of them (16-byte loads, a warp reads 512 contiguous bytes), the r-vector in
+// shared memory; column passes (Z^T times an n-vector) give a warp four columns of a row range, so that the n-vector
+// is read once for four of them.
+#include <algorithm>
 #include <cfloat>
 
 #include "barrier.h"
@@ -50,18 +53,49 @@ __device__ __forceinline__ void atomic_min_pos(double* p, double v) {
   atomicMin(reinterpret_cast<unsigned long long*>(p), (unsigned long long)__double_as_longlong(v));
 }
 
-__device__ __forceinline__ double row_dot(const double* __restrict__ Z, long long ld, int i, int r,
-                                          const double* s_vec) {
-  double acc = 0.0;
-  const double* zi = Z + i;
+// part[w][i] = sum over the columns k = w (mod 8) of Z(i0 + i, k) s_k for the CTA's 64 rows, then their sum over w in
+// the threads i < 64 (0 past n).  VEC: 16-byte loads.  Thread-per-row passes with 8-byte loads ran at 0.6 to 0.8 of the
+// copy rate (131072 x 528: 106 - 140 us), 3.5 CTAs per SM of one wave.
+constexpr int ROWS = 64;
+template <bool VEC>
+__device__ __forceinline__ double row_dots(const double* __restrict__ Z, long long ld, int i0, int n, int r,
+                                           const double* s, double (*part)[ROWS]) {
+  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+  const int i = i0 + (VEC ? 2 * lane : lane);
+  const double* z = Z + i;
+  double a0 = 0.0, a1 = 0.0;
+  if (VEC && i + 1 < n) {
 #pragma unroll 8
-  for (int k = 0; k < r; ++k) acc = fma(zi[(long long)k * ld], s_vec[k], acc);
-  return acc;
+    for (int k = warp; k < r; k += 8) {
+      const double2 v = __ldg(reinterpret_cast<const double2*>(z + (long long)k * ld));
+      a0 = fma(v.x, s[k], a0);
+      a1 = fma(v.y, s[k], a1);
+    }
+  } else {
+    const int step = VEC ? 1 : 32;  // the second row of this lane
+    const bool p0 = i < n, p1 = i + step < n;
+#pragma unroll 4
+    for (int k = warp; k < r; k += 8) {
+      if (p0) a0 = fma(__ldg(z + (long long)k * ld), s[k], a0);
+      if (p1) a1 = fma(__ldg(z + (long long)k * ld + step), s[k], a1);
+    }
+  }
+  __syncthreads();  // the sums of the row block before have been read
+  part[warp][VEC ? 2 * lane : lane] = a0;
+  part[warp][VEC ? 2 * lane + 1 : lane + 32] = a1;
+  __syncthreads();
+  double sum = 0.0;
+  if (threadIdx.x < ROWS) {
+#pragma unroll
+    for (int w = 0; w < THREADS / 32; ++w) sum += part[w][threadIdx.x];
+  }
+  return sum;
 }
 
 // Gradient and Hessian diagonal at a (Grad_f + Grad_Phi = Grad, Hess_Phi):
 //   zw = Z (Z^T a),  g = zw - 1 + (-1/a + 1/(C - a))/t,  D = (1/a^2 + 1/(C - a)^2)/t,  dinv = 1/D
 // Reductions into red[]: [0] sum(a), [1] sum(log a + log(C - a)), [2] max D, [3] min D.
+template <bool VEC>
 __global__ void __launch_bounds__(THREADS) grad_hess_kernel(int n, int r, const double* __restrict__ Z, long long ld,
                                                             const double* __restrict__ w, const double* __restrict__ a,
                                                             double C, double t, double* __restrict__ g,
@@ -74,9 +108,13 @@ __global__ void __launch_bounds__(THREADS) grad_hess_kernel(int n, int r, const 
   __syncthreads();
   double sums[2] = {0.0, 0.0};
   double dmax = 0.0, dmin = DBL_MAX;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+  __shared__ double part[THREADS / 32][ROWS];
+  for (int i0 = blockIdx.x * ROWS; i0 < n; i0 += gridDim.x * ROWS) {
+    const double dot = zw_in ? 0.0 : row_dots<VEC>(Z, ld, i0, n, r, sw, part);
+    const int i = i0 + threadIdx.x;
+    if (threadIdx.x >= ROWS || i >= n) continue;
     const double ai = a[i], ci = C - ai;
-    const double zw = zw_in ? zw_in[i] : row_dot(Z, ld, i, r, sw);
+    const double zw = zw_in ? zw_in[i] : dot;
     if (zw_out) zw_out[i] = zw;
     g[i] = (zw - 1.0) + ((-1.0 / ai) + (1.0 / ci)) / t;
     const double D = ((1.0 / (ai * ai)) + (1.0 / (ci * ci))) / t;
@@ -101,6 +139,7 @@ __global__ void __launch_bounds__(THREADS) grad_hess_kernel(int n, int r, const 
 
 // Newton direction from u:  s = -dinv * (g + Z u).  Reductions: [0] g.s, [1] sum(s), [2] max feasible step
 // (min over i of -a/s for s < 0 and (C - a)/s for s > 0).
+template <bool VEC>
 __global__ void __launch_bounds__(THREADS) direction_kernel(int n, int r, const double* __restrict__ Z, long long ld,
                                                             const double* __restrict__ u, const double* __restrict__ g,
                                                             const double* __restrict__ dinv,
@@ -111,8 +150,11 @@ __global__ void __launch_bounds__(THREADS) direction_kernel(int n, int r, const 
   __syncthreads();
   double sums[2] = {0.0, 0.0};
   double tmax = DBL_MAX;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const double zu = row_dot(Z, ld, i, r, su);
+  __shared__ double part[THREADS / 32][ROWS];
+  for (int i0 = blockIdx.x * ROWS; i0 < n; i0 += gridDim.x * ROWS) {
+    const double zu = row_dots<VEC>(Z, ld, i0, n, r, su, part);
+    const int i = i0 + threadIdx.x;
+    if (threadIdx.x >= ROWS || i >= n) continue;
     const double gi = g[i];
     const double si = -dinv[i] * (gi + zu);
     s[i] = si;
@@ -128,24 +170,52 @@ __global__ void __launch_bounds__(THREADS) direction_kernel(int n, int r, const 
   if (threadIdx.x % 32 == 0) atomic_min_pos(red + 2, tmax);
 }
 
-// out[k] = sum_i Z[i, k] * (scale_i * v_i)  (scale may be null): Z^T v, one block per group of columns,
-// grid.y splits the rows.  FP64 atomics combine the row splits.
+// out[k] += sign sum_i Z[i, k] * (scale_i * v_i)  (scale may be null): Z^T v.  A warp owns GT_COLS neighbouring columns and
+// the rows of blockIdx.y, whose products scale_i v_i it forms once for all of them; FP64 atomics combine the row
+// splits.  131072 x 528: 86 us (a column per warp, 8-byte loads, the vectors read per column: 106 - 117).
+constexpr int GT_COLS = 4;
+template <bool VEC>
 __global__ void __launch_bounds__(THREADS) gemv_t_kernel(int n, int r, const double* __restrict__ Z, long long ld,
                                                          const double* __restrict__ v, const double* __restrict__ scale,
                                                          double sign, double* out, int rows_per_split) {
-  // 8 warps per block, each warp owns one column at a time; columns strided over blocks
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-  const int r0 = blockIdx.y * rows_per_split;
-  const int r1 = min(n, r0 + rows_per_split);
-  for (int k = blockIdx.x * (THREADS / 32) + warp; k < r; k += gridDim.x * (THREADS / 32)) {
-    const double* zk = Z + (long long)k * ld;
-    double acc = 0.0;
-    for (int i = r0 + lane; i < r1; i += 32) {
-      const double vi = scale ? scale[i] * v[i] : v[i];
-      acc = fma(zk[i], vi, acc);
+  const int k0 = (blockIdx.x * (THREADS / 32) + warp) * GT_COLS;
+  if (k0 >= r) return;
+  const int r0 = blockIdx.y * rows_per_split, r1 = min(n, r0 + rows_per_split);
+  const double* z[GT_COLS];
+  double acc[GT_COLS];
+#pragma unroll
+  for (int c = 0; c < GT_COLS; ++c) {
+    z[c] = Z + (long long)min(k0 + c, r - 1) * ld;  // columns past r repeat the last and are not stored
+    acc[c] = 0.0;
+  }
+  int i = r0 + (VEC ? 2 : 1) * lane;
+  if (VEC) {
+#pragma unroll 2
+    for (; i + 1 < r1; i += 64) {
+      double2 x = __ldg(reinterpret_cast<const double2*>(v + i));
+      if (scale) {
+        const double2 w = __ldg(reinterpret_cast<const double2*>(scale + i));
+        x.x *= w.x;
+        x.y *= w.y;
+      }
+#pragma unroll
+      for (int c = 0; c < GT_COLS; ++c) {
+        const double2 q = __ldg(reinterpret_cast<const double2*>(z[c] + i));
+        acc[c] = fma(q.x, x.x, acc[c]);
+        acc[c] = fma(q.y, x.y, acc[c]);
+      }
     }
-    acc = warp_sum(acc);
-    if (lane == 0) atomicAdd(out + k, sign * acc);
+  }
+  for (; i < r1; i += VEC ? 64 : 32) {  // VEC: an odd last row
+    const double x = scale ? scale[i] * v[i] : v[i];
+#pragma unroll
+    for (int c = 0; c < GT_COLS; ++c) acc[c] = fma(__ldg(z[c] + i), x, acc[c]);
+  }
+#pragma unroll
+  for (int c = 0; c < GT_COLS; ++c) {
+    const double sum = warp_sum(acc[c]);
+    if (lane == 0 && k0 + c < r) atomicAdd(out + k0 + c, sign * sum);
   }
 }
 
@@ -177,6 +247,7 @@ __global__ void __launch_bounds__(THREADS) linesearch_kernel(int n, const double
 
 // gradf = Z w - 1, gradphi = (-1/a + 1/(C-a))/t, grad = gradf + gradphi, D = (1/a^2 + 1/(C-a)^2)/t
 // (include/dbarrier.h:48-81 one by one); red: [0] += sum a, [1] += sum(log a + log(C - a)).
+template <bool VEC>
 __global__ void __launch_bounds__(THREADS) terms_kernel(int n, int r, const double* __restrict__ Z, long long ld,
                                                         const double* __restrict__ w, const double* __restrict__ a,
                                                         double C, double t, double* gf, double* gp, double* g,
@@ -185,9 +256,12 @@ __global__ void __launch_bounds__(THREADS) terms_kernel(int n, int r, const doub
   for (int k = threadIdx.x; k < r; k += blockDim.x) sw[k] = w[k];
   __syncthreads();
   double sums[2] = {0.0, 0.0};
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+  __shared__ double part[THREADS / 32][ROWS];
+  for (int i0 = blockIdx.x * ROWS; i0 < n; i0 += gridDim.x * ROWS) {
+    const double f1 = row_dots<VEC>(Z, ld, i0, n, r, sw, part) - 1.0;
+    const int i = i0 + threadIdx.x;
+    if (threadIdx.x >= ROWS || i >= n) continue;
     const double ai = a[i], ci = C - ai;
-    const double f1 = row_dot(Z, ld, i, r, sw) - 1.0;
     const double p1 = ((-1.0 / ai) + (1.0 / ci)) / t;
     gf[i] = f1;
     gp[i] = p1;
@@ -201,6 +275,7 @@ __global__ void __launch_bounds__(THREADS) terms_kernel(int n, int r, const doub
 
 // Negated residual of the Newton system (Z Z^T + D) s = -g:  res = g + Z v + s / dinv  with v = Z^T s.
 // red: [0] += |res|^2, [1] += |g|^2.
+template <bool VEC>
 __global__ void __launch_bounds__(THREADS) residual_kernel(int n, int r, const double* __restrict__ Z, long long ld,
                                                            const double* __restrict__ v, const double* __restrict__ g,
                                                            const double* __restrict__ dinv,
@@ -210,9 +285,12 @@ __global__ void __launch_bounds__(THREADS) residual_kernel(int n, int r, const d
   for (int k = threadIdx.x; k < r; k += blockDim.x) sv[k] = v[k];
   __syncthreads();
   double sums[2] = {0.0, 0.0};
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+  __shared__ double part[THREADS / 32][ROWS];
+  for (int i0 = blockIdx.x * ROWS; i0 < n; i0 += gridDim.x * ROWS) {
+    const double zv = row_dots<VEC>(Z, ld, i0, n, r, sv, part);
+    const int i = i0 + threadIdx.x;
+    if (threadIdx.x >= ROWS || i >= n) continue;
     const double gi = g[i];
-    const double zv = row_dot(Z, ld, i, r, sv);
     if (zv_out) zv_out[i] = zv;
     const double ri = gi + zv + s[i] / dinv[i];
     res[i] = ri;
@@ -259,6 +337,7 @@ __global__ void axpy_kernel(int n, double alpha, const double* __restrict__ x, d
 }
 
 // Primal value pieces at w = Z^T a:  sum_i max(0, 1 - (Z w)_i)
+template <bool VEC>
 __global__ void __launch_bounds__(THREADS) hinge_kernel(int n, int r, const double* __restrict__ Z, long long ld,
                                                         const double* __restrict__ w, double* red,
                                                         const double* __restrict__ y, double b) {
@@ -266,8 +345,12 @@ __global__ void __launch_bounds__(THREADS) hinge_kernel(int n, int r, const doub
   for (int k = threadIdx.x; k < r; k += blockDim.x) sw[k] = w[k];
   __syncthreads();
   double sums[1] = {0.0};
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-    sums[0] += fmax(0.0, 1.0 - row_dot(Z, ld, i, r, sw) - (y ? y[i] * b : 0.0));
+  __shared__ double part[THREADS / 32][ROWS];
+  for (int i0 = blockIdx.x * ROWS; i0 < n; i0 += gridDim.x * ROWS) {
+    const double zw = row_dots<VEC>(Z, ld, i0, n, r, sw, part);
+    const int i = i0 + threadIdx.x;
+    if (threadIdx.x < ROWS && i < n) sums[0] += fmax(0.0, 1.0 - zw - (y ? y[i] * b : 0.0));
+  }
   block_sum_add<1>(sums, red);
 }
 
@@ -305,6 +388,10 @@ __global__ void dot_kernel(int r, const double* x, const double* y, double* out)
   block_sum_add<1>(v, out);
 }
 
+// grid of the row passes: 64 rows per CTA, up to eight CTAs per SM
+inline int blocks64(db200_context* ctx, int n) { return std::max(1, std::min((n + ROWS - 1) / ROWS, 8 * ctx->num_sms)); }
+inline bool vec_ok(const double* Z, long long ld) { return reinterpret_cast<uintptr_t>(Z) % 16 == 0 && ld % 2 == 0; }
+
 inline int rows_grid(db200_context* ctx, int n) {
   int b = (n + THREADS - 1) / THREADS;
   const int cap = 4 * ctx->num_sms;
@@ -322,8 +409,8 @@ int bar_init_red(db200_context* ctx, double* red, int nsum, int nmax, int nmin) 
 int bar_grad_hess(db200_context* ctx, int n, int r, const double* Z, long long ld, const double* w, const double* a,
                   double C, double t, double* g, double* dinv, double* red, const double* zw_in, double* zw_out) {
   if (r > MAX_R_SMEM) return fail(ctx, DB200_ERR_UNSUPPORTED, "barrier: rank > 4096");
-  grad_hess_kernel<<<rows_grid(ctx, n), THREADS, 0, ctx->stream>>>(n, r, Z, ld, w, a, C, t, g, dinv, red, zw_in,
-                                                                   zw_out);
+  auto k = vec_ok(Z, ld) ? grad_hess_kernel<true> : grad_hess_kernel<false>;
+  k<<<blocks64(ctx, n), THREADS, 0, ctx->stream>>>(n, r, Z, ld, w, a, C, t, g, dinv, red, zw_in, zw_out);
   DB200_CUDA(ctx, cudaGetLastError());
   count_launch(ctx);
   return DB200_OK;
@@ -331,7 +418,8 @@ int bar_grad_hess(db200_context* ctx, int n, int r, const double* Z, long long l
 
 int bar_direction(db200_context* ctx, int n, int r, const double* Z, long long ld, const double* u, const double* g,
                   const double* dinv, const double* a, double C, double* s, double* red) {
-  direction_kernel<<<rows_grid(ctx, n), THREADS, 0, ctx->stream>>>(n, r, Z, ld, u, g, dinv, a, C, s, red);
+  auto k = vec_ok(Z, ld) ? direction_kernel<true> : direction_kernel<false>;
+  k<<<blocks64(ctx, n), THREADS, 0, ctx->stream>>>(n, r, Z, ld, u, g, dinv, a, C, s, red);
   DB200_CUDA(ctx, cudaGetLastError());
   count_launch(ctx);
   return DB200_OK;
@@ -340,13 +428,14 @@ int bar_direction(db200_context* ctx, int n, int r, const double* Z, long long l
 int bar_gemv_t(db200_context* ctx, int n, int r, const double* Z, long long ld, const double* v, const double* scale,
                double sign, double* out) {
   DB200_CUDA(ctx, cudaMemsetAsync(out, 0, sizeof(double) * r, ctx->stream));
-  const int col_blocks = (r + 7) / 8;
-  int splits = (4 * ctx->num_sms + col_blocks - 1) / col_blocks;
-  int rows = (n + splits - 1) / splits;
-  rows = round_up(rows < 32 ? 32 : rows, 32);
+  // about eight CTAs per SM, no split shorter than 128 rows
+  const int per = GT_COLS * THREADS / 32, col_blocks = (r + per - 1) / per;
+  int splits = std::max(1, std::min((n + 127) / 128, 8 * ctx->num_sms / col_blocks));
+  const int rows = round_up((n + splits - 1) / splits, 64);
   splits = (n + rows - 1) / rows;
-  dim3 grid(col_blocks, splits);
-  gemv_t_kernel<<<grid, THREADS, 0, ctx->stream>>>(n, r, Z, ld, v, scale, sign, out, rows);
+  const bool vec = vec_ok(Z, ld) && vec_ok(v, 2) && (!scale || vec_ok(scale, 2));
+  auto k = vec ? gemv_t_kernel<true> : gemv_t_kernel<false>;
+  k<<<dim3(col_blocks, splits), THREADS, 0, ctx->stream>>>(n, r, Z, ld, v, scale, sign, out, rows);
   DB200_CUDA(ctx, cudaGetLastError());
   count_launch(ctx);
   return DB200_OK;
@@ -364,7 +453,8 @@ int bar_linesearch16(db200_context* ctx, int n, const double* a, const double* s
 int bar_terms(db200_context* ctx, int n, int r, const double* Z, long long ld, const double* w, const double* a,
               double C, double t, double* gf, double* gp, double* g, double* D, double* red) {
   if (r > MAX_R_SMEM) return fail(ctx, DB200_ERR_UNSUPPORTED, "barrier: rank > 4096");
-  terms_kernel<<<rows_grid(ctx, n), THREADS, 0, ctx->stream>>>(n, r, Z, ld, w, a, C, t, gf, gp, g, D, red);
+  auto k = vec_ok(Z, ld) ? terms_kernel<true> : terms_kernel<false>;
+  k<<<blocks64(ctx, n), THREADS, 0, ctx->stream>>>(n, r, Z, ld, w, a, C, t, gf, gp, g, D, red);
   DB200_CUDA(ctx, cudaGetLastError());
   count_launch(ctx);
   return DB200_OK;
@@ -372,7 +462,8 @@ int bar_terms(db200_context* ctx, int n, int r, const double* Z, long long ld, c
 
 int bar_residual(db200_context* ctx, int n, int r, const double* Z, long long ld, const double* v, const double* g,
                  const double* dinv, const double* s, double* res, double* red, double* zv_out) {
-  residual_kernel<<<rows_grid(ctx, n), THREADS, 0, ctx->stream>>>(n, r, Z, ld, v, g, dinv, s, res, red, zv_out);
+  auto k = vec_ok(Z, ld) ? residual_kernel<true> : residual_kernel<false>;
+  k<<<blocks64(ctx, n), THREADS, 0, ctx->stream>>>(n, r, Z, ld, v, g, dinv, s, res, red, zv_out);
   DB200_CUDA(ctx, cudaGetLastError());
   count_launch(ctx);
   return DB200_OK;
@@ -417,7 +508,8 @@ int bar_axpy(db200_context* ctx, int n, double alpha, const double* x, double* y
 int bar_hinge(db200_context* ctx, int n, int r, const double* Z, long long ld, const double* w, double* red,
               const double* y, double b) {
   DB200_CUDA(ctx, cudaMemsetAsync(red, 0, sizeof(double), ctx->stream));
-  hinge_kernel<<<rows_grid(ctx, n), THREADS, 0, ctx->stream>>>(n, r, Z, ld, w, red, y, b);
+  auto k = vec_ok(Z, ld) ? hinge_kernel<true> : hinge_kernel<false>;
+  k<<<blocks64(ctx, n), THREADS, 0, ctx->stream>>>(n, r, Z, ld, w, red, y, b);
   DB200_CUDA(ctx, cudaGetLastError());
   count_launch(ctx);
   return DB200_OK;
