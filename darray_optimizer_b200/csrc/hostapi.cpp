@@ -166,7 +166,8 @@ int db200_woodbury_solve(db200_context* ctx, int n, int r, const double* Z, int 
     return fail(ctx, DB200_ERR_INVALID, "woodbury_solve: bad arguments");
   // (Z Z^T + diag(g))^-1 b = g^-1 b - g^-1 Z (I + Z^T g^-1 Z)^-1 Z^T g^-1 b
   const size_t rr = (size_t)r * r;
-  const size_t bytes = 1024 + 2 * align_up((size_t)n * 8, 256) + 2 * align_up(rr * 8, 256) + align_up((size_t)r * 8, 256);
+  const size_t bytes = 1024 + 2 * align_up((size_t)n * 8, 256) + align_up(rr * 8, 256) +
+                       align_up(potrf_inverse_doubles(r) * 8, 256) + align_up((size_t)r * 8, 256);
   char* base = static_cast<char*>(slot_buffer(ctx, SLOT_SPARE, bytes));
   if (!base) return DB200_ERR_NOMEM;
   Carve cv{base};
@@ -175,7 +176,7 @@ int db200_woodbury_solve(db200_context* ctx, int n, int r, const double* Z, int 
   double* ginv = cv.take<double>(n);
   double* nb = cv.take<double>(n);
   double* M = cv.take<double>(rr);
-  double* L = cv.take<double>(rr);
+  double* W = cv.take<double>(potrf_inverse_doubles(r));
   double* u = cv.take<double>(r);
   int st = bar_reciprocal(ctx, n, diag, ginv);
   if (!st) st = gram<double, double>(ctx, n, r, r, Z, ldz, Z, ldz, ginv, 1.0, 0.0, M, r, true);
@@ -183,10 +184,8 @@ int db200_woodbury_solve(db200_context* ctx, int n, int r, const double* Z, int 
   if (!st) st = bar_gemv_t(ctx, n, r, Z, ldz, b, ginv, 1.0, u);  // u = Z^T g^-1 b, solved below for M^-1 Z^T g^-1 b
   if (st) return st;
   DB200_CUDA(ctx, cudaMemsetAsync(pair, 0, 2 * sizeof(int), ctx->stream));
-  if ((st = potrf_upper(ctx, M, r, r, pair, pair + 1))) return st;
-  if ((st = transpose64(ctx, M, r, r, r, L, r))) return st;
-  if ((st = trsv_upper(ctx, M, L, r, r, u, true))) return st;
-  if ((st = trsv_upper(ctx, M, L, r, r, u, false))) return st;
+  if ((st = potrf_upper(ctx, M, r, r, pair, pair + 1, 64, W))) return st;
+  if ((st = trsv_pair(ctx, M, r, r, W, u))) return st;
   // u = M^-1 Z^T g^-1 b now; x = g^-1 (b - Z u) is the direction kernel's -dinv (h + Z u) with h = -b
   if ((st = bar_negate(ctx, n, b, nb))) return st;
   if ((st = bar_init_red(ctx, red, 2, 0, 1))) return st;

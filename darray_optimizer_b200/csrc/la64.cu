@@ -30,7 +30,7 @@ constexpr int GT = 128;
 // trailing matrix (launched after this one).
 template <bool VEC>
 __global__ void __launch_bounds__(P64_THREADS) potrf_block_kernel(double* A, int lda, int k0, int kb, int l,
-                                                                  int* status, int* bad, int* arrivals) {
+                                                                  int* status, int* bad, int* arrivals, double* W) {
   extern __shared__ __align__(16) unsigned char raw[];
   P64Smem& S = *reinterpret_cast<P64Smem*>(raw);
   const int t = threadIdx.x, warp = t / 32;
@@ -62,6 +62,7 @@ __global__ void __launch_bounds__(P64_THREADS) potrf_block_kernel(double* A, int
       const int i = e % P64_NB, j = e / P64_NB;
       if (i < kb) A[(long long)(k0 + j) * lda + k0 + i] = (i <= j) ? S.R[j * P64_RLD + i] : 0.0;
     }
+    if (W) p64_store_inverses(S, W + (long long)k0 * 16, kb);
   }
   if (group >= 4) p64_store<VEC>(acc, A, lda, k0, kb, col, cl);
 }
@@ -156,123 +157,159 @@ __global__ void trinv_clear_kernel(double* X, int ldx, int l, int h) {
     X[(long long)(r0 + e / q) * ldx + r0 + h + e % q] = 0.0;
 }
 
-// Single-CTA triangular solves with an upper factor R (and its transpose L = R^T stored separately so every
-// inner product reads a contiguous column):
-//   mode 0: solve R^T y = b   (forward; row i of R^T = column i of R)
-//   mode 1: solve R x = y     (backward; row i of R = column i of L)
-// x/b in place, FP64, x staged in shared memory (l <= 4096).  Blocks of 32 rows: the 16 warps form the off-block
-// inner products (two rows each; the coefficients of the nearest 256 columns are loaded before the block's
-// barrier, overlapping the previous block's triangle), then warp 0 solves the 32 x 32 triangle from registers it
-// also loaded before the barrier (so the 32 sequential steps carry no memory latency), with the diagonal applied
-// as a reciprocal computed once per block.  Follows triangular_solve (include/blas_like.h:96-140) for one column.
-__global__ void __launch_bounds__(512) trsv_kernel(const double* R, const double* L, int ld, int l, double* x,
-                                                   int mode) {
-  __shared__ double xs[4096];
-  __shared__ double part[32];
-  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-  for (int i = threadIdx.x; i < l; i += blockDim.x) xs[i] = x[i];
-  const int nb = (l + 31) / 32;
-  const double* T = (mode == 0) ? R : L;  // column i0 + lane of T holds this lane's triangle coefficients
-  for (int bb = 0; bb < nb; ++bb) {
-    const int blk = (mode == 0) ? bb : nb - 1 - bb;
-    const int i0 = blk * 32;
-    const int bl = min(32, l - i0);
-    double tri[32];
-    double dinv = 0.0;
+// x <- R^-1 R^-T x for an upper factor R (l <= 4096) with the inverses W = R_bb^-T of its 16 x 16 diagonal blocks, in one
+// CTA: the forward solve R^T z = x (block b needs its columns above the block, a warp per column), then R u = z (block b
+// needs its 16 rows right of the block, 16 contiguous entries per column; no transposed copy).  Per block: the off-block
+// products, their reduction, and y = W r, y += W (r - R_bb^T y), three 16 x 16 products of one warp, instead of 16 dependent
+// substitution steps (the correction keeps the substitution's backward error).  What a block reads depends on nothing
+// computed: every thread holds its part of the next panel (16 x 256) in registers, and warp 0 of the next W and R_bb, loaded
+// one block ahead, so the chain holds no memory latency.  Bound by that chain of l / 16 blocks each way, about 1.5 us a
+// block: l = 528 106 us, l = 138 23 us (shared-memory rings fed by cp.async or bulk copies 121 - 139 and 27, their issue in
+// the chain's way; a global load, a 32-step shuffle chain and a transposed copy per block of 32: 2 x 82 and 2 x 16 us and
+// the copy).
+// Follows triangular_solve (include/blas_like.h:96-140) for one column.
+constexpr int TV_THREADS = 512, TV_NB = 16, TV_LEN = 256, TV_MAX_L = 4096;
+struct TrsvSmem {
+  double x[TV_MAX_L + TV_LEN];
+  double part[16][16];
+  double r[16], e[16];
+};
+
+// One direction's blocks (a template: the addresses of the two differ by constants that the loop then carries as
+// immediates; chosen at run time they made the loop's integer work its bound, 360 instructions per warp and block).
+template <bool FWD>
+__device__ __forceinline__ void trsv_sweep(TrsvSmem& S, const double* __restrict__ R, int ld, int l,
+                                           const double* __restrict__ W, int nb) {
+  const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
+  const int i = lane % 16, h = 8 * (lane / 16);  // warp 0's solve: row i, half h of its products
+  const int first = FWD ? lane : tid / 16;       // this thread's first off-block index, then every 32nd
+  const long long step = FWD ? 32 : 32LL * ld;
+  // forward: rows 0 .. b0 - 1 of column b0 + warp; backward: row b0 + tid % 16 of the columns b0 + 16 .. l - 1
+  auto base = [&](int b) -> const double* {
+    const int b0 = b * TV_NB;
+    return FWD ? R + (long long)min(b0 + warp, l - 1) * ld + first
+               : R + (long long)(b0 + TV_NB + first) * ld + b0 + tid % 16;
+  };
+  auto off_len = [&](int b) -> int { return FWD ? b * TV_NB : l - (b + 1) * TV_NB; };
+  auto load = [&](const double* p, int left, double (&v)[8]) {  // left: entries from `first` of this piece on
+    if (left >= TV_LEN) {
+#pragma unroll
+      for (int u = 0; u < 8; ++u) v[u] = __ldg(p + u * step);
+    } else {
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        v[u] = 0.0;
+        if (first + 32 * u < left) v[u] = __ldg(p + u * step);
+      }
+    }
+  };
+  // forward: W(i, h + k) and R_bb(h + k, i); backward: W(h + k, i) and R_bb(i, h + k)
+  auto load_diag = [&](int b, double (&w)[8], double (&d)[8]) {
+    const int b0 = b * TV_NB;
+    const double* Wb = W + (long long)b * 256 + (FWD ? i * 16 + h : h * 16 + i);
+    const double* Rb = FWD ? R + (long long)min(b0 + i, l - 1) * ld + b0 + h : R + (long long)(b0 + h) * ld + b0 + i;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      w[k] = __ldg(Wb + (FWD ? k : 16 * k));
+      const bool in = FWD ? (h + k <= i && b0 + i < l) : (i <= h + k && b0 + h + k < l);
+      d[k] = in ? __ldg(Rb + (FWD ? k : (long long)k * ld)) : 0.0;
+    }
+  };
+  int b = FWD ? 0 : nb - 1;
+  const double* p = base(b);
+  double nxt[8], wn[8], dn[8];
+  load(p, off_len(b), nxt);
+  if (warp == 0) load_diag(b, wn, dn);
+#pragma unroll 1
+  for (int k = 0; k < nb; ++k) {
+    const int b0 = b * TV_NB, len = off_len(b), bn = FWD ? b + 1 : b - 1;
+    const bool more = k + 1 < nb;
+    double w[8], d[8];
     if (warp == 0) {
-      const double* c = T + (long long)(i0 + lane) * ld + i0;
 #pragma unroll
-      for (int r = 0; r < 32; ++r) tri[r] = (lane < bl && r < bl) ? c[r] : 0.0;
+      for (int q = 0; q < 8; ++q) {
+        w[q] = wn[q];
+        d[q] = dn[q];
+      }
+      if (more) load_diag(bn, wn, dn);
     }
-    // off-block coefficients of rows i0 + warp and i0 + warp + 16: the nearest 32 PF (= 256) columns are loaded
-    // into registers before the barrier (they do not depend on x), so their latency overlaps the previous block's
-    // triangle; a longer range finishes in the loop after the barrier
-    constexpr int PF = 8;
-    double pf[2][PF];
-    int kbeg[2], kend[2];
+    double acc0 = 0.0, acc1 = 0.0;
+    const double* xp = S.x + first + (FWD ? 0 : b0 + TV_NB);
+    int left = len;
+#pragma unroll 1
+    do {
+      double v[8];
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int i = i0 + warp + 16 * h;
-      kbeg[h] = (mode == 0) ? 0 : i0 + 32;
-      kend[h] = (i < l) ? ((mode == 0) ? i0 : l) : kbeg[h];
-      // mode 0 reads the columns just below i0 first (nearest the diagonal), mode 1 those just after i0 + 32
-      const double* col = T + (long long)(i < l ? i : 0) * ld;
-#pragma unroll
-      for (int u = 0; u < PF; ++u) {
-        const int k = (mode == 0) ? kend[h] - 1 - lane - 32 * u : kbeg[h] + lane + 32 * u;
-        pf[h][u] = (k >= kbeg[h] && k < kend[h]) ? col[k] : 0.0;
+      for (int u = 0; u < 8; ++u) v[u] = nxt[u];
+      if (left > TV_LEN) {
+        p += 8 * step;
+        load(p, left - TV_LEN, nxt);
+      } else if (more) {
+        p = base(bn);
+        load(p, off_len(bn), nxt);
       }
-    }
-    __syncthreads();  // xs of the previous block (and the initial staging) visible
+      if (left == len) __syncthreads();  // x of the block before is written
+      // past the end v is zero and x (cleared beyond l) finite
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int i = i0 + warp + 16 * h;
-      double s0 = 0.0, s1 = 0.0;
-#pragma unroll
-      for (int u = 0; u < PF; ++u) {
-        const int k = (mode == 0) ? kend[h] - 1 - lane - 32 * u : kbeg[h] + lane + 32 * u;
-        if (k >= kbeg[h] && k < kend[h]) {
-          if (u & 1)
-            s1 += pf[h][u] * xs[k];
-          else
-            s0 += pf[h][u] * xs[k];
-        }
+      for (int u = 0; u < 8; u += 2) {
+        acc0 = fma(v[u], xp[32 * u], acc0);
+        acc1 = fma(v[u + 1], xp[32 * u + 32], acc1);
       }
-      if (kend[h] - kbeg[h] > 32 * PF) {
-        const double* col = T + (long long)i * ld;
-        if (mode == 0) {
-          for (int k = kbeg[h] + lane; k < kend[h] - 32 * PF; k += 32) s0 += col[k] * xs[k];
-        } else {
-          for (int k = kbeg[h] + 32 * PF + lane; k < kend[h]; k += 32) s1 += col[k] * xs[k];
-        }
-      }
-      double sum = s0 + s1;
+      xp += TV_LEN;
+      left -= TV_LEN;
+    } while (left > 0);
+    acc0 += acc1;
+    acc0 += __shfl_xor_sync(0xffffffffu, acc0, 16);
+    if (FWD) {
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-      if (lane == 0) part[warp + 16 * h] = sum;
+      for (int o = 8; o > 0; o >>= 1) acc0 += __shfl_xor_sync(0xffffffffu, acc0, o);
+      if (lane == 0) S.r[warp] = b0 + warp < l ? S.x[b0 + warp] - acc0 : 0.0;
+    } else {
+      if (lane < 16) S.part[warp][lane] = acc0;
     }
     __syncthreads();
     if (warp == 0) {
-      double dg = 1.0;
+      if (!FWD) {
+        double t = 0.0;
 #pragma unroll
-      for (int r = 0; r < 32; ++r)
-        if (r == lane && lane < bl) dg = tri[r];
-      dinv = (lane < bl) ? 1.0 / dg : 0.0;
-      double v = (lane < bl) ? xs[i0 + lane] - part[lane] : 0.0;
-      if (mode == 0) {
-#pragma unroll
-        for (int r = 0; r < 32; ++r) {
-          const double xr = __shfl_sync(0xffffffffu, v * dinv, r);
-          if (lane == r) v = xr;
-          if (lane > r) v -= tri[r] * xr;
-        }
-      } else {
-#pragma unroll
-        for (int r = 31; r >= 0; --r) {
-          const double xr = __shfl_sync(0xffffffffu, v * dinv, r);
-          if (lane == r) v = xr;
-          if (lane < r) v -= tri[r] * xr;
-        }
+        for (int q = 0; q < 8; ++q) t += S.part[h + q][i];
+        t += __shfl_xor_sync(0xffffffffu, t, 16);
+        if (lane < 16) S.r[i] = b0 + i < l ? S.x[b0 + i] - t : 0.0;
+        __syncwarp();
       }
-      if (lane < bl) xs[i0 + lane] = v;
+      auto apply = [&](const double (&m)[8], const double* v) -> double {
+        double s0 = 0.0, s1 = 0.0;
+#pragma unroll
+        for (int q = 0; q < 8; q += 2) {
+          const double2 z = *reinterpret_cast<const double2*>(v + h + q);
+          s0 = fma(m[q], z.x, s0);
+          s1 = fma(m[q + 1], z.y, s1);
+        }
+        s0 += s1;
+        return s0 + __shfl_xor_sync(0xffffffffu, s0, 16);
+      };
+      double y = apply(w, S.r);
+      if (lane < 16) S.x[b0 + i] = y;
+      __syncwarp();
+      const double ry = apply(d, S.x + b0);
+      if (lane < 16) S.e[i] = S.r[i] - ry;
+      __syncwarp();
+      y += apply(w, S.e);
+      if (lane < 16) S.x[b0 + i] = y;
     }
+    b = bn;
   }
-  __syncthreads();
-  for (int i = threadIdx.x; i < l; i += blockDim.x) x[i] = xs[i];
 }
 
-__global__ void transpose_kernel(const double* A, int lda, int m, int n, double* B, int ldb) {
-  __shared__ double t[32][33];
-  const int bi = blockIdx.x * 32, bj = blockIdx.y * 32;
-  for (int r = threadIdx.y; r < 32; r += blockDim.y) {
-    const int i = bi + threadIdx.x, j = bj + r;
-    if (i < m && j < n) t[r][threadIdx.x] = A[(long long)j * lda + i];
-  }
+__global__ void __launch_bounds__(TV_THREADS, 1) trsv_pair_kernel(const double* __restrict__ R, int ld, int l,
+                                                                  const double* __restrict__ W, double* x) {
+  __shared__ __align__(16) TrsvSmem S;
+  const int nb = (l + TV_NB - 1) / TV_NB;
+  for (int k = threadIdx.x; k < nb * TV_NB + TV_LEN; k += TV_THREADS) S.x[k] = k < l ? x[k] : 0.0;
+  trsv_sweep<true>(S, R, ld, l, W, nb);   // R^T z = x (its first barrier also ends the staging)
+  trsv_sweep<false>(S, R, ld, l, W, nb);  // R u = z
   __syncthreads();
-  for (int r = threadIdx.y; r < 32; r += blockDim.y) {
-    const int j = bj + threadIdx.x, i = bi + r;
-    if (i < m && j < n) B[(long long)i * ldb + j] = t[threadIdx.x][r];
-  }
+  for (int k = threadIdx.x; k < l; k += TV_THREADS) x[k] = S.x[k];
 }
 
 __global__ void scale_kernel(double* C, int ldc, int m, int n, double beta, int upper_only) {
@@ -551,12 +588,12 @@ static int syrk_update(db200_context* ctx, int k, int p, int q, const double* P,
   return dmm_launch<double, double, double, true, true>(ctx, g);
 }
 
-int potrf_upper(db200_context* ctx, double* A, int lda, int l, int* d_status, int* d_bad, int nb) {
-  if (nb < 1 || nb > 64) nb = 64;
+int potrf_upper(db200_context* ctx, double* A, int lda, int l, int* d_status, int* d_bad, int nb, double* W) {
+  if (nb < 1 || nb > 64 || W) nb = 64;
   // up to l = 544 (the barrier's capacity matrices, the CholeskyQR2 and Nystrom Grams) the whole factor is one
   // launch on a thread-block cluster; an explicit smaller block size keeps the multi-kernel path
   if (nb == 64) {
-    const int s = potrf_cluster(ctx, A, lda, l, d_status, d_bad);
+    const int s = potrf_cluster(ctx, A, lda, l, d_status, d_bad, W);
     if (s != DB200_ERR_UNSUPPORTED) return s;
   }
   // (k0 is a multiple of nb: 16-byte loads need an even one too)
@@ -585,10 +622,10 @@ int potrf_upper(db200_context* ctx, double* A, int lda, int l, int* d_status, in
       const unsigned ctas = rest > 64 ? (unsigned)((rest + 63) / 64) : 1u;
       if (vec)
         potrf_block_kernel<true><<<ctas, P64_THREADS, sizeof(P64Smem), ctx->stream>>>(A, lda, k0, kb, l, d_status,
-                                                                                      d_bad, ctx->d_status + 1);
+                                                                                      d_bad, ctx->d_status + 1, W);
       else
         potrf_block_kernel<false><<<ctas, P64_THREADS, sizeof(P64Smem), ctx->stream>>>(A, lda, k0, kb, l, d_status,
-                                                                                       d_bad, ctx->d_status + 1);
+                                                                                       d_bad, ctx->d_status + 1, W);
       count_launch(ctx);
       const int pr = K0 + KB - (k0 + kb);  // rows of this panel below the block
       if (pr > 0) {
@@ -671,17 +708,9 @@ int trinv_upper(db200_context* ctx, const double* R, int ldr, int l, double* X, 
   return DB200_OK;
 }
 
-int trsv_upper(db200_context* ctx, const double* R, const double* L, int ld, int l, double* x, bool transposed) {
-  if (l > 4096) return fail(ctx, DB200_ERR_UNSUPPORTED, "trsv: l > 4096");
-  trsv_kernel<<<1, 512, 0, ctx->stream>>>(R, L, ld, l, x, transposed ? 0 : 1);
-  DB200_CUDA(ctx, cudaGetLastError());
-  count_launch(ctx);
-  return DB200_OK;
-}
-
-int transpose64(db200_context* ctx, const double* A, int lda, int m, int n, double* B, int ldb) {
-  dim3 grid((m + 31) / 32, (n + 31) / 32), block(32, 8);
-  transpose_kernel<<<grid, block, 0, ctx->stream>>>(A, lda, m, n, B, ldb);
+int trsv_pair(db200_context* ctx, const double* R, int ld, int l, const double* W, double* x) {
+  if (l > TV_MAX_L) return fail(ctx, DB200_ERR_UNSUPPORTED, "trsv: l > 4096");
+  trsv_pair_kernel<<<1, TV_THREADS, 0, ctx->stream>>>(R, ld, l, W, x);
   DB200_CUDA(ctx, cudaGetLastError());
   count_launch(ctx);
   return DB200_OK;

@@ -20,8 +20,11 @@ int gemm_tall(db200_context* ctx, int n, int p, int q, const TA* A, long long ld
 
 // In-place upper Cholesky (A = R^T R) with block size nb <= 64; the strictly lower part is zeroed.  A
 // non-positive pivot sets *d_status = DB200_ERR_NOT_SPD and *d_bad = first row of the failing block.
-// Restates cholesky_factorize(A, 'U', n, 0, bs) of include/lapack_like.h:10-56.
-int potrf_upper(db200_context* ctx, double* A, int lda, int l, int* d_status, int* d_bad, int nb = 64);
+// Restates cholesky_factorize(A, 'U', n, 0, bs) of include/lapack_like.h:10-56.  W (may be null; ceil(l / 16) * 256
+// doubles): the inverses R_bb^-T of the 16 x 16 diagonal blocks for trsv_pair (then nb = 64).
+int potrf_upper(db200_context* ctx, double* A, int lda, int l, int* d_status, int* d_bad, int nb = 64,
+                double* W = nullptr);
+inline size_t potrf_inverse_doubles(int l) { return (size_t)((l + 15) / 16) * 256; }
 
 // The same factor in one launch on a thread-block cluster for 1 <= l <= 544 (potrf_cluster.cu); returns
 // DB200_ERR_UNSUPPORTED, launching nothing, where no cluster configuration holds the matrix.  potrf_cluster_init
@@ -29,15 +32,14 @@ int potrf_upper(db200_context* ctx, double* A, int lda, int l, int* d_status, in
 // used for l (0: none).
 void potrf_cluster_init(db200_context* ctx);
 int potrf_cluster_size(const db200_context* ctx, int l);
-int potrf_cluster(db200_context* ctx, double* A, int lda, int l, int* d_status, int* d_bad);
+int potrf_cluster(db200_context* ctx, double* A, int lda, int l, int* d_status, int* d_bad, double* W = nullptr);
 
 // X = R^-1 for upper triangular R.
 int trinv_upper(db200_context* ctx, const double* R, int ldr, int l, double* X, int ldx);
 
-// In-place triangular solve with upper R and its stored transpose L: transposed -> R^T x = b, else R x = b.
-int trsv_upper(db200_context* ctx, const double* R, const double* L, int ld, int l, double* x, bool transposed);
+// x <- R^-1 R^-T x (R upper, l <= 4096) with the diagonal blocks' inverses W that potrf_upper left.
+int trsv_pair(db200_context* ctx, const double* R, int ld, int l, const double* W, double* x);
 
-int transpose64(db200_context* ctx, const double* A, int lda, int m, int n, double* B, int ldb);
 int symmetrize(db200_context* ctx, double* C, int ldc, int l, double shift);
 int mirror_upper(db200_context* ctx, double* C, int ldc, int l);
 template <typename TS, typename TD>

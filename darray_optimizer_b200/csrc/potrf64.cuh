@@ -235,4 +235,11 @@ __device__ __forceinline__ void p64_store(const double (&acc)[8][4], double* A, 
   }
 }
 
+// The inverses W = R_pp^-T of the block's 16 x 16 diagonal blocks (those that hold one of its kb columns), row major 256
+// doubles each, for the triangular solves.
+__device__ __forceinline__ void p64_store_inverses(const P64Smem& S, double* W, int kb) {
+  for (int e = threadIdx.x; e < (kb + 15) / 16 * 256; e += P64_THREADS)
+    W[e] = S.W[e / 256][(e % 256) / 16 * P64_WLD + e % 16];
+}
+
 }  // namespace db200

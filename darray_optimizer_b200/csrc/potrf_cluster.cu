@@ -79,7 +79,7 @@ __device__ __forceinline__ void pc_update_tile(const double* P, double* C, long 
 
 template <bool VEC>
 __global__ void __launch_bounds__(P64_THREADS, 1) potrf_cluster_kernel(double* A, int lda, int l, int* status,
-                                                                       int* bad) {
+                                                                       int* bad, double* W) {
   extern __shared__ __align__(16) unsigned char raw[];
   P64Smem& S = *reinterpret_cast<P64Smem*>(raw);
   const int nc = (int)cluster_nctarank(), c = (int)cluster_ctarank();
@@ -103,11 +103,13 @@ __global__ void __launch_bounds__(P64_THREADS, 1) potrf_cluster_kernel(double* A
     }
     if (group >= 4) p64_store<VEC>(acc, A, lda, c0, kb, col, cl);
     cluster_sync_all();  // the block row is complete; every CTA has read the diagonal block
-    if (step % nc == c)
+    if (step % nc == c) {
+      if (W) p64_store_inverses(S, W + (long long)c0 * 16, kb);
       for (int e = tid; e < kb * P64_NB; e += P64_THREADS) {
         const int i = e % P64_NB, j = e / P64_NB;
         if (i <= j) A[(long long)(c0 + j) * lda + c0 + i] = S.R[j * P64_RLD + i];
       }
+    }
     if (r0 >= l) break;
     // trailing tiles (I <= J), tile number J (J + 1) / 2 + I
     const int tiles = ng * (ng + 1) / 2;
@@ -178,14 +180,14 @@ int potrf_cluster_size(const db200_context* ctx, int l) {
   return 64 * nc >= l - P64_NB ? nc : 0;
 }
 
-int potrf_cluster(db200_context* ctx, double* A, int lda, int l, int* d_status, int* d_bad) {
+int potrf_cluster(db200_context* ctx, double* A, int lda, int l, int* d_status, int* d_bad, double* W) {
   const int nc = potrf_cluster_size(ctx, l);
   if (nc < 1) return DB200_ERR_UNSUPPORTED;
   cudaLaunchAttribute attr[1];
   cudaLaunchConfig_t cfg = pc_config(attr, nc, ctx->stream);
   const bool vec = reinterpret_cast<uintptr_t>(A) % 16 == 0 && lda % 2 == 0;
-  DB200_CUDA(ctx, vec ? cudaLaunchKernelEx(&cfg, potrf_cluster_kernel<true>, A, lda, l, d_status, d_bad)
-                      : cudaLaunchKernelEx(&cfg, potrf_cluster_kernel<false>, A, lda, l, d_status, d_bad));
+  DB200_CUDA(ctx, vec ? cudaLaunchKernelEx(&cfg, potrf_cluster_kernel<true>, A, lda, l, d_status, d_bad, W)
+                      : cudaLaunchKernelEx(&cfg, potrf_cluster_kernel<false>, A, lda, l, d_status, d_bad, W));
   count_launch(ctx);
   return DB200_OK;
 }

@@ -176,6 +176,7 @@ struct FactorSeq {
   const double* dinv;
   double* M;
   double* L;
+  double* W;  // inverses of the factor's diagonal blocks
   int* d_pair;
   int n, r;
   bool use_tc;
@@ -198,7 +199,7 @@ int factor_tail(db200_context* ctx, const FactorSeq& f) {
   DB200_CUDA(ctx, cudaMemcpyAsync(f.L, f.M, sizeof(double) * (size_t)f.r * f.r, cudaMemcpyDeviceToDevice,
                                   ctx->stream));
   DB200_CUDA(ctx, cudaMemsetAsync(f.d_pair, 0, 2 * sizeof(int), ctx->stream));
-  return potrf_upper(ctx, f.M, f.r, f.r, f.d_pair, f.d_pair + 1);
+  return potrf_upper(ctx, f.M, f.r, f.r, f.d_pair, f.d_pair + 1, 64, f.W);
 }
 
 int factor_seq(db200_context* ctx, const FactorSeq& f) {
@@ -223,7 +224,7 @@ size_t barrier_slot_bytes(int n, int r, bool mixed) {
   const size_t rr = (size_t)r * r;
   const size_t tc_bytes = mixed ? gram_tc_scratch_bytes(n, r) : 0;
   return 4096 + 10 * align_up((size_t)n * 8, 256) + 6 * align_up((size_t)r * 8, 256) + 2 * align_up(rr * 8, 256) +
-         align_up(tc_bytes, 256) + 4096;
+         align_up(potrf_inverse_doubles(r) * 8, 256) + align_up(tc_bytes, 256) + 4096;
 }
 
 int svm_barrier_impl(db200_context* ctx, int n, int r, const double* Z, int ldz, const float* y, double C,
@@ -248,7 +249,8 @@ int svm_barrier_impl(db200_context* ctx, int n, int r, const double* Z, int ldz,
   double* v = cv.take<double>(r);
   double* u = cv.take<double>(r);
   double* M = cv.take<double>(rr);
-  double* L = cv.take<double>(rr);
+  double* L = cv.take<double>(rr);  // M before its factorisation, for shifted retries
+  double* W = cv.take<double>(potrf_inverse_doubles(r));
   double* res = cv.take<double>(n);
   double* delta = cv.take<double>(n);
   double* zw = cv.take<double>(n);  // Z w for the current w = Z^T a (valid while zw_ok)
@@ -300,8 +302,7 @@ int svm_barrier_impl(db200_context* ctx, int n, int r, const double* Z, int ldz,
   auto woodbury_body = [&](const double* rhs, double* out, double* rd) -> int {
     int s2;
     if ((s2 = gemv_t(rhs, dinv, -1.0, u))) return s2;
-    if ((s2 = trsv_upper(ctx, M, L, r, r, u, true))) return s2;   // R^T z = rhs
-    if ((s2 = trsv_upper(ctx, M, L, r, r, u, false))) return s2;  // R u = z
+    if ((s2 = trsv_pair(ctx, M, r, r, W, u))) return s2;  // R^T z = rhs, R u = z
     if ((s2 = bar_init_red(ctx, rd, 2, 0, 1))) return s2;
     return bar_direction(ctx, n, r, Z, ldz, u, rhs, dinv, a, C, out, rd);
   };
@@ -365,7 +366,7 @@ int svm_barrier_impl(db200_context* ctx, int n, int r, const double* Z, int ldz,
   // Capacity matrix M = I + Z^T D^-1 Z of the current D and its first Cholesky attempt (status in d_pair), enqueued
   // only: the caller reads the status.
   auto factor_launch = [&](bool use_tc) -> int {
-    const FactorSeq fs{Z, ldz, dinv, M, L, d_pair, n, r, use_tc, kSlices[tc_level], tc_scratch};
+    const FactorSeq fs{Z, ldz, dinv, M, L, W, d_pair, n, r, use_tc, kSlices[tc_level], tc_scratch};
     int s2;
     if (!dist) {
       // Gram, identity, backup, first Cholesky: one graph replay per Newton step (about 17 launches as separate
@@ -421,7 +422,7 @@ int svm_barrier_impl(db200_context* ctx, int n, int r, const double* Z, int ldz,
       // until the relative residual is <= 1e-10; a step that does not get there is recomputed with the FP64
       // capacity matrix.  FP64: the capacity matrix on the FP64 pipes, no refinement.
       bool v_current = false;  // v already holds Z^T s (set by a converged refinement check)
-      // Capacity matrix M = I + Z^T D^-1 Z and its Cholesky factor (upper in M, its transpose in L).
+      // Capacity matrix M = I + Z^T D^-1 Z and its Cholesky factor (upper in M).
       auto factor = [&](bool use_tc) -> int {
         int s2;
         // A capacity matrix with a huge dynamic range (late in the barrier D^-1 spans ~18 orders) can sit on the
@@ -446,9 +447,9 @@ int svm_barrier_impl(db200_context* ctx, int n, int r, const double* Z, int ldz,
           if ((s2 = bar_scale_diag(ctx, M, r, r, 1.0 + eps))) return s2;
           eps *= 10.0;
           DB200_CUDA(ctx, cudaMemsetAsync(d_pair, 0, 2 * sizeof(int), ctx->stream));
-          if ((s2 = potrf_upper(ctx, M, r, r, d_pair, d_pair + 1))) return s2;
+          if ((s2 = potrf_upper(ctx, M, r, r, d_pair, d_pair + 1, 64, W))) return s2;
         }
-        return transpose64(ctx, M, r, r, r, L, r);
+        return DB200_OK;
       };
       // out = -(Z Z^T + D)^-1 rhs by Woodbury on the factored capacity matrix.  With the tensor-core capacity
       // matrix, iterative refinement against the exact FP64 operator (out += H~^-1 (-rhs - H out)) until the
