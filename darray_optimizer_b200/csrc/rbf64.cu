@@ -15,6 +15,11 @@
 //
 // Issued work per 64 rows and 16 points: 8 d/8 distance DMMAs + 8 LT/8 sketch DMMAs per sketch tile; at d = 128,
 // l = 528 (two tiles of 264) that is 1.2x the algorithmic 2 n^2 (d + l) flops (the distance is recomputed per tile).
+//
+// Where the row blocks and tiles leave SMs idle, the points j are cut into ranges (blockIdx.y) whose partial products go
+// to slabs and are summed in a fixed order (r64_splits).  Bound by the DMMAs of a CTA between two barriers: a second
+// CTA on the SM (tiles of up to 144 columns) fills them.
+#include <algorithm>
 #include <cmath>
 
 #include "internal.h"
@@ -60,6 +65,8 @@ struct R64Args {
   double gamma;
   double* Y;
   long long ldy;
+  int per_split;  // stages of a range of j (blockIdx.y)
+  double* slabs;  // [ranges][l][m] partial products without y_i; null: one range, straight to Y
 };
 
 // Shared layout (doubles): Xi [64][dp + 4] | K [2][64][20] | Omega~ [2][lt][20]; Xj (floats) [2][16][dp + 4].
@@ -70,7 +77,7 @@ __host__ __device__ inline size_t r64_smem_bytes(int dp, int lt) {
 
 // NT = n8 column tiles of the CTA's sketch tile (LT = 8 NT); warp half 0 holds tiles [0, H0), half 1 [H0, NT).
 template <int NT>
-__global__ void __launch_bounds__(R64_THREADS, 1) rbf_sketch_f64_kernel(const R64Args a) {
+__global__ void __launch_bounds__(R64_THREADS, NT <= 18 ? 2 : 1) rbf_sketch_f64_kernel(const R64Args a) {
   constexpr int H0 = (NT + 1) / 2, H1 = NT - H0, NB = H0;  // accumulator tiles per warp (half 1 uses H1 <= NB)
   extern __shared__ __align__(16) double smem64[];
   const int dp = a.dp, S = dp + 4, lt = 8 * NT;
@@ -157,15 +164,15 @@ __global__ void __launch_bounds__(R64_THREADS, 1) rbf_sketch_f64_kernel(const R6
 #pragma unroll
     for (int e = 0; e < 4; ++e) acc[b][e] = 0.0;
 
-  const int S_n = a.n_stages;
-  issue_xj(0);
-  if (S_n > 1) issue_xj(1);
-  issue_om(0);
+  const int S_0 = blockIdx.y * a.per_split, S_n = min(a.n_stages, S_0 + a.per_split);
+  issue_xj(S_0);
+  if (S_0 + 1 < S_n) issue_xj(S_0 + 1);
+  issue_om(S_0);
   cp_async_commit();
   cp_async_wait_all();
-  __syncthreads();  // Xi, Xj(0), Xj(1), Omega~(0)
-  distance(0);
-  for (int s = 0; s < S_n; ++s) {
+  __syncthreads();  // Xi, Xj(S_0), Xj(S_0 + 1), Omega~(S_0)
+  distance(S_0);
+  for (int s = S_0; s < S_n; ++s) {
     cp_async_wait_all();  // this thread's copies of Xj(s + 1) and Omega~(s) (issued one iteration ago)
     __syncthreads();      // K(s) complete and every copy visible; every read of stage s - 1 done
     // Xj(s + 2) reuses the buffer distance(s) read (iteration s - 1); Omega~(s + 1) the one sketch(s - 1) read
@@ -197,10 +204,13 @@ __global__ void __launch_bounds__(R64_THREADS, 1) rbf_sketch_f64_kernel(const R6
   }
   cp_async_wait_all();
 
-  // Y(i, c) = y_i acc
+  // Y(i, c) = y_i acc, or the range's slab
   const int ia = i0 + rA, ib = ia + 8;
-  const double ya = (ia < a.m) ? (a.yi ? (double)a.yi[ia] : 1.0) : 0.0;
-  const double yb = (ib < a.m) ? (a.yi ? (double)a.yi[ib] : 1.0) : 0.0;
+  const bool scaled = a.yi && !a.slabs;
+  const double ya = (scaled && ia < a.m) ? (double)a.yi[ia] : 1.0;
+  const double yb = (scaled && ib < a.m) ? (double)a.yi[ib] : 1.0;
+  double* Y = a.slabs ? a.slabs + (long long)blockIdx.y * a.l * a.m : a.Y;
+  const long long ldy = a.slabs ? a.m : a.ldy;
 #pragma unroll
   for (int b = 0; b < NB; ++b) {
     if (b >= nbn) continue;
@@ -208,8 +218,8 @@ __global__ void __launch_bounds__(R64_THREADS, 1) rbf_sketch_f64_kernel(const R6
     for (int e = 0; e < 2; ++e) {
       const int c = c0 + 8 * (nb0 + b) + 2 * t + e;
       if (c >= a.l) continue;
-      if (ia < a.m) a.Y[(long long)c * a.ldy + ia] = ya * acc[b][e];
-      if (ib < a.m) a.Y[(long long)c * a.ldy + ib] = yb * acc[b][2 + e];
+      if (ia < a.m) Y[c * ldy + ia] = ya * acc[b][e];
+      if (ib < a.m) Y[c * ldy + ib] = yb * acc[b][2 + e];
     }
   }
 }
@@ -231,8 +241,23 @@ __global__ void block_omega_kernel(const double* __restrict__ Om, long long ldo,
   }
 }
 
+// Y(i, c) = y_i (slab_0 + slab_1 + ...)(i, c), in that order
+__global__ void __launch_bounds__(256) sum_slabs64_kernel(const R64Args a, int ranges) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= a.m) return;
+  const double y = a.yi ? (double)a.yi[i] : 1.0;
+  const long long stride = (long long)a.l * a.m;
+  for (int c = blockIdx.y; c < a.l; c += gridDim.y) {
+    const double* p = a.slabs + (long long)c * a.m + i;
+    double acc = p[0];
+#pragma unroll 4
+    for (int k = 1; k < ranges; ++k) acc += p[k * stride];
+    a.Y[(long long)c * a.ldy + i] = y * acc;
+  }
+}
+
 template <int NT>
-cudaError_t launch_r64(const R64Args& a, int blocks, size_t smem, cudaStream_t st) {
+cudaError_t launch_r64(const R64Args& a, dim3 blocks, size_t smem, cudaStream_t st) {
   auto k = rbf_sketch_f64_kernel<NT>;
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
@@ -251,6 +276,20 @@ static int r64_tile_cols(int l, int dp) {
   return 264;
 }
 
+// Ranges of j: the least waves x (stages of a range + 8, a CTA's start and end in stages), at least 16 stages each; cut
+// only where that is below 0.9 of the whole, for the slabs' sum.  4096 x 4096, d = 16, l = 138 (64 row blocks): whole,
+// one CTA an SM, 679 us; in 4 ranges, two CTAs an SM, 282.
+static int r64_splits(const db200_context* ctx, int blocks, int per_sm, int n_stages) {
+  const long long slots = (long long)ctx->num_sms * per_sm;
+  const int most = std::max(1, std::min(32, n_stages / 16));
+  auto cost = [&](int s) { return ((blocks * (long long)s + slots - 1) / slots) * ((n_stages + s - 1) / s + 8); };
+  int best = 1;
+  for (int s = 2; s <= most; ++s)
+    if (10 * cost(s) < 9 * cost(1) && cost(s) < cost(best)) best = s;
+  const int per = (n_stages + best - 1) / best;
+  return (n_stages + per - 1) / per;  // no empty range
+}
+
 int rbf_sketch_f64_fused(db200_context* ctx, int m, int n, int d, int l, const float* Xi, int ldxi, const float* Xj,
                          int ldxj, const float* yi, const float* yj, const double* Omega, int ldo, double* Y, int ldy,
                          double gamma) {
@@ -261,7 +300,11 @@ int rbf_sketch_f64_fused(db200_context* ctx, int m, int n, int d, int l, const f
   const int n_stages = (n + R64_KS - 1) / R64_KS;
   const size_t smem = r64_smem_bytes(dp, lt);
   if (smem > R64_SMEM_MAX) return fail(ctx, DB200_ERR_UNSUPPORTED, "rbf_sketch_f64: d too large for the FP64 tile");
-  const size_t bytes = 1024 + align_up((size_t)m * 8, 256) + align_up((size_t)n_stages * R64_KS * 8, 256) +
+  const int blocks = ((m + R64_ROWS - 1) / R64_ROWS) * n_lt;
+  const int per_sm = lt <= 144 && 2 * (smem + 1024) <= 228 * 1024 ? 2 : 1;
+  const int ranges = r64_splits(ctx, blocks, per_sm, n_stages);
+  const size_t slab_doubles = ranges > 1 ? (size_t)ranges * l * m : 0;
+  const size_t bytes = 1024 + align_up(slab_doubles * 8, 256) + align_up((size_t)m * 8, 256) + align_up((size_t)n_stages * R64_KS * 8, 256) +
                        align_up((size_t)n_stages * lpad * R64_KS * 8, 256) + 1024;
   char* base = static_cast<char*>(slot_buffer(ctx, SLOT_SPARE, bytes));
   if (!base) return DB200_ERR_NOMEM;
@@ -269,6 +312,7 @@ int rbf_sketch_f64_fused(db200_context* ctx, int m, int n, int d, int l, const f
   double* si = cv.take<double>(m);
   double* sj = cv.take<double>((size_t)n_stages * R64_KS);
   double* Ob = cv.take<double>((size_t)n_stages * lpad * R64_KS);
+  double* slabs = slab_doubles ? cv.take<double>(slab_doubles) : nullptr;
   DB200_CUDA(ctx, cudaMemsetAsync(sj, 0, sizeof(double) * (size_t)n_stages * R64_KS, ctx->stream));
   int st = rownorm_f64(ctx, Xi, ldxi, m, d, si);
   if (!st) st = rownorm_f64(ctx, Xj, ldxj, n, d, sj);
@@ -302,15 +346,22 @@ int rbf_sketch_f64_fused(db200_context* ctx, int m, int n, int d, int l, const f
   a.gamma = gamma;
   a.Y = Y;
   a.ldy = ldy;
-  const int blocks = ((m + R64_ROWS - 1) / R64_ROWS) * n_lt;
+  a.per_split = (n_stages + ranges - 1) / ranges;
+  a.slabs = slabs;
+  const dim3 grid(blocks, ranges);
   cudaEvent_t e0 = nullptr;
   prof_begin(ctx, &e0);
-  cudaError_t e = (lt == 264)   ? launch_r64<33>(a, blocks, smem, ctx->stream)
-                  : (lt == 144) ? launch_r64<18>(a, blocks, smem, ctx->stream)
-                                : launch_r64<2>(a, blocks, smem, ctx->stream);
+  cudaError_t e = (lt == 264)   ? launch_r64<33>(a, grid, smem, ctx->stream)
+                  : (lt == 144) ? launch_r64<18>(a, grid, smem, ctx->stream)
+                                : launch_r64<2>(a, grid, smem, ctx->stream);
   DB200_CUDA(ctx, e);
   prof_end(ctx, e0);
   count_launch(ctx);
+  if (slabs) {
+    sum_slabs64_kernel<<<dim3((m + 255) / 256, std::min(l, 256)), 256, 0, ctx->stream>>>(a, ranges);
+    DB200_CUDA(ctx, cudaGetLastError());
+    count_launch(ctx);
+  }
   return DB200_OK;
 }
 
