@@ -219,30 +219,38 @@ __global__ void __launch_bounds__(THREADS) gemv_t_kernel(int n, int r, const dou
   }
 }
 
-// Log-barrier sums at T candidate steps: out[k] = sum_i log(a_i + tau_k s_i) + log(C - a_i - tau_k s_i); a
-// candidate that leaves the open box anywhere gets +inf in out[T + k] (infeasible count).
-template <int T>
-__global__ void __launch_bounds__(THREADS) linesearch_kernel(int n, const double* __restrict__ a,
-                                                             const double* __restrict__ s, double C,
-                                                             const double* __restrict__ taus, double* out) {
-  double tau[T];
-#pragma unroll
-  for (int k = 0; k < T; ++k) tau[k] = taus[k];
-  double sums[2 * T];
-#pragma unroll
-  for (int k = 0; k < 2 * T; ++k) sums[k] = 0.0;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+// Log-barrier sums at the 16 candidate steps: out[k] += sum_i log(a_i + tau_k s_i) + log(C - a_i - tau_k s_i); a candidate
+// that leaves the open box anywhere counts its infeasible rows in out[16 + k].  A thread per row and candidate (lane %
+// 16): bound by the logarithms' issue, which needs the warps.  n = 4096: 2.7 us (a thread per row with all 16
+// candidates, 16 CTAs and 32 block sums: 8.9); 131072: 16 us (22).
+__global__ void __launch_bounds__(THREADS) linesearch16_kernel(int n, const double* __restrict__ a,
+                                                               const double* __restrict__ s, double C,
+                                                               const double* __restrict__ taus, double* out) {
+  __shared__ double part[2][THREADS / 32][16];
+  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32, k = lane % 16;
+  const double tau = taus[k];
+  double sum = 0.0, bad = 0.0;
+  for (int i = (blockIdx.x * THREADS + threadIdx.x) / 16; i < n; i += gridDim.x * (THREADS / 16)) {
     const double ai = a[i], si = s[i];
-#pragma unroll
-    for (int k = 0; k < T; ++k) {
-      const double x = fma(tau[k], si, ai), y = C - x;
-      if (x > 0.0 && y > 0.0)
-        sums[k] += log(x) + log(y);
-      else
-        sums[T + k] += 1.0;
-    }
+    const double x = fma(tau, si, ai), y = C - x;
+    if (x > 0.0 && y > 0.0)
+      sum += log(x) + log(y);
+    else
+      bad += 1.0;
   }
-  block_sum_add<2 * T>(sums, out);
+  sum += __shfl_xor_sync(0xffffffffu, sum, 16);
+  bad += __shfl_xor_sync(0xffffffffu, bad, 16);
+  if (lane < 16) {
+    part[0][warp][k] = sum;
+    part[1][warp][k] = bad;
+  }
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    double v = 0.0;
+#pragma unroll
+    for (int w = 0; w < THREADS / 32; ++w) v += part[threadIdx.x / 16][w][k];
+    if (threadIdx.x < 16 || v != 0.0) atomicAdd(out + threadIdx.x, v);
+  }
 }
 
 // gradf = Z w - 1, gradphi = (-1/a + 1/(C-a))/t, grad = gradf + gradphi, D = (1/a^2 + 1/(C-a)^2)/t
@@ -369,22 +377,36 @@ __global__ void init_red_kernel(double* red, int nsum, int nmax, int nmin) {
   else if (i < nsum + nmax + nmin) red[i] = DBL_MAX;
 }
 
-// taus[k] = t0 beta^k (k < 16), t0 = min(1, 0.99 * *step_max), by repeated multiplication (the host forms the
-// same values the same way)
-__global__ void steps16_kernel(const double* step_max, double beta, double* taus) {
-  if (threadIdx.x != 0) return;
-  const double m = 0.99 * *step_max;
-  double t = (m < 1.0) ? m : 1.0;  // as std::min(1.0, m): 1 when m is NaN
-  for (int k = 0; k < 16; ++k) {
-    taus[k] = t;
-    t *= beta;
+// One CTA's scalars of a Newton step in one launch (six nodes of a graph before): wv[0] = w.v, wv[1] = v.v, the line
+// search's sums ls[0..32) cleared, and taus[k] = t0 beta^k (k < 16), t0 = min(1, 0.99 * *step_max), by repeated
+// multiplication (the host forms the same values the same way).
+__global__ void __launch_bounds__(THREADS) step_scalars_kernel(int r, const double* __restrict__ w,
+                                                               const double* __restrict__ v, double* wv,
+                                                               const double* step_max, double beta, double* taus,
+                                                               double* ls) {
+  double s[2] = {0.0, 0.0};
+  for (int k = threadIdx.x; k < r; k += THREADS) {
+    s[0] += w[k] * v[k];
+    s[1] += v[k] * v[k];
   }
+  if (threadIdx.x < 2) wv[threadIdx.x] = 0.0;  // before block_sum_add's barrier, added to after it by the same threads
+  if (threadIdx.x >= 32 && threadIdx.x < 64) ls[threadIdx.x - 32] = 0.0;
+  if (threadIdx.x == 64) {
+    const double m = 0.99 * *step_max;
+    double t = (m < 1.0) ? m : 1.0;  // as std::min(1.0, m): 1 when m is NaN
+    for (int k = 0; k < 16; ++k) {
+      taus[k] = t;
+      t *= beta;
+    }
+  }
+  block_sum_add<2>(s, wv);
 }
 
 __global__ void dot_kernel(int r, const double* x, const double* y, double* out) {
   double s = 0.0;
   for (int k = threadIdx.x; k < r; k += blockDim.x) s += x[k] * y[k];
   double v[1] = {s};
+  if (threadIdx.x == 0) out[0] = 0.0;  // this thread adds the sum to it
   block_sum_add<1>(v, out);
 }
 
@@ -443,8 +465,8 @@ int bar_gemv_t(db200_context* ctx, int n, int r, const double* Z, long long ld, 
 
 int bar_linesearch16(db200_context* ctx, int n, const double* a, const double* s, double C, const double* taus,
                      double* out) {
-  DB200_CUDA(ctx, cudaMemsetAsync(out, 0, sizeof(double) * 32, ctx->stream));
-  linesearch_kernel<16><<<rows_grid(ctx, n), THREADS, 0, ctx->stream>>>(n, a, s, C, taus, out);
+  const int blocks = std::max(1, std::min((n + THREADS / 16 - 1) / (THREADS / 16), 8 * ctx->num_sms));
+  linesearch16_kernel<<<blocks, THREADS, 0, ctx->stream>>>(n, a, s, C, taus, out);
   DB200_CUDA(ctx, cudaGetLastError());
   count_launch(ctx);
   return DB200_OK;
@@ -529,15 +551,15 @@ int bar_scale_diag(db200_context* ctx, double* M, int ldm, int r, double factor)
   return DB200_OK;
 }
 
-int bar_steps16(db200_context* ctx, const double* step_max, double beta, double* taus) {
-  steps16_kernel<<<1, 32, 0, ctx->stream>>>(step_max, beta, taus);
+int bar_step_scalars(db200_context* ctx, int r, const double* w, const double* v, double* wv, const double* step_max,
+                     double beta, double* taus, double* ls) {
+  step_scalars_kernel<<<1, THREADS, 0, ctx->stream>>>(r, w, v, wv, step_max, beta, taus, ls);
   DB200_CUDA(ctx, cudaGetLastError());
   count_launch(ctx);
   return DB200_OK;
 }
 
 int bar_dot(db200_context* ctx, int r, const double* x, const double* y, double* out) {
-  DB200_CUDA(ctx, cudaMemsetAsync(out, 0, sizeof(double), ctx->stream));
   dot_kernel<<<1, THREADS, 0, ctx->stream>>>(r, x, y, out);
   DB200_CUDA(ctx, cudaGetLastError());
   count_launch(ctx);

@@ -18,7 +18,7 @@ int bar_direction(db200_context* ctx, int n, int r, const double* Z, long long l
 // out = sign * Z^T (scale .* v)  (scale may be null); out is zeroed first.
 int bar_gemv_t(db200_context* ctx, int n, int r, const double* Z, long long ld, const double* v, const double* scale,
                double sign, double* out);
-// out[k] = sum log(a + tau_k s) + log(C - a - tau_k s), out[16 + k] = count of coordinates leaving the box.
+// out[k] += sum log(a + tau_k s) + log(C - a - tau_k s), out[16 + k] += count of coordinates leaving the box.
 int bar_linesearch16(db200_context* ctx, int n, const double* a, const double* s, double C, const double* taus,
                      double* out);
 int bar_axpy(db200_context* ctx, int n, double alpha, const double* x, double* y);
@@ -48,7 +48,9 @@ int bar_hinge(db200_context* ctx, int n, int r, const double* Z, long long ld, c
 int bar_add_identity(db200_context* ctx, double* M, int ldm, int r);
 int bar_scale_diag(db200_context* ctx, double* M, int ldm, int r, double factor);
 int bar_dot(db200_context* ctx, int r, const double* x, const double* y, double* out);
-// taus[k] = min(1, 0.99 * *step_max) beta^k for k < 16 (the line search's first candidates, formed on the device)
-int bar_steps16(db200_context* ctx, const double* step_max, double beta, double* taus);
+// wv = {w.v, v.v}, ls[0..32) = 0 and taus[k] = min(1, 0.99 * *step_max) beta^k for k < 16 (the line search's first
+// candidates, formed on the device)
+int bar_step_scalars(db200_context* ctx, int r, const double* w, const double* v, double* wv, const double* step_max,
+                     double beta, double* taus, double* ls);
 
 }  // namespace db200

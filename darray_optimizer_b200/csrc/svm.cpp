@@ -237,11 +237,12 @@ int svm_barrier_impl(db200_context* ctx, int n, int r, const double* Z, int ldz,
   char* base = static_cast<char*>(slot_buffer(ctx, SLOT_BAR, barrier_slot_bytes(n, r, mixed)));
   if (!base) return DB200_ERR_NOMEM;
   Carve cv{base};
+  // one readback: [0..3] row reductions, [8..9] w.w or w.v and v.v, [12] Cholesky status, [16..18] residual, [32..63] ls
   double* red = cv.take<double>(64);
   double* taus = cv.take<double>(16);
-  double* ls = cv.take<double>(32);
-  double* sc = cv.take<double>(8);  // scalars: [0] w.w, [1] w.v, [2] v.v, [3] hinge, [4..6] products with y
-  int* d_pair = cv.take<int>(4);
+  double* ls = red + 32;
+  double* sc = cv.take<double>(8);  // scalars: [0] w.w, [3] hinge, [4..6] products with y
+  int* d_pair = reinterpret_cast<int*>(red + 12);
   double* g = cv.take<double>(n);
   double* dinv = cv.take<double>(n);
   double* s = cv.take<double>(n);
@@ -403,11 +404,7 @@ int svm_barrier_impl(db200_context* ctx, int n, int r, const double* Z, int ldz,
       // the row reductions, w.w and the Cholesky status into red[0..13) for one readback
       if ((st = seq(5, {}, [&]() -> int {
              int s2;
-             if ((s2 = reduce_grad()) || (s2 = bar_dot(ctx, r, w, w, sc))) return s2;
-             DB200_CUDA(ctx, cudaMemcpyAsync(red + 8, sc, sizeof(double), cudaMemcpyDeviceToDevice, ctx->stream));
-             DB200_CUDA(ctx, cudaMemcpyAsync(red + 12, d_pair, 2 * sizeof(int), cudaMemcpyDeviceToDevice,
-                                             ctx->stream));
-             return DB200_OK;
+             return (s2 = reduce_grad()) ? s2 : bar_dot(ctx, r, w, w, red + 8);
            })))
         return st;
       if ((st = fetch(red, 13))) return st;
@@ -575,18 +572,9 @@ int svm_barrier_impl(db200_context* ctx, int n, int r, const double* Z, int ldz,
              int s2;
              if (need_v && (s2 = gemv_t(s, nullptr, 1.0, v))) return s2;
              if ((s2 = reduce(red, 2, DB200_REDUCE_SUM)) || (s2 = reduce(red + 2, 1, DB200_REDUCE_MIN))) return s2;
-             if ((s2 = bar_dot(ctx, r, w, v, sc + 1))) return s2;
-             if ((s2 = bar_dot(ctx, r, v, v, sc + 2))) return s2;
-             DB200_CUDA(ctx, cudaMemcpyAsync(red + 8, sc + 1, 2 * sizeof(double), cudaMemcpyDeviceToDevice,
-                                             ctx->stream));
-             DB200_CUDA(ctx, cudaMemcpyAsync(red + 12, d_pair, 2 * sizeof(int), cudaMemcpyDeviceToDevice,
-                                             ctx->stream));
-             if ((s2 = bar_steps16(ctx, red + 2, P.beta, taus))) return s2;
+             if ((s2 = bar_step_scalars(ctx, r, w, v, red + 8, red + 2, P.beta, taus, ls))) return s2;
              if ((s2 = bar_linesearch16(ctx, n, a, s, C, taus, ls))) return s2;
-             if ((s2 = reduce(ls, 32, DB200_REDUCE_SUM))) return s2;
-             DB200_CUDA(ctx, cudaMemcpyAsync(red + 32, ls, 32 * sizeof(double), cudaMemcpyDeviceToDevice,
-                                             ctx->stream));
-             return DB200_OK;
+             return reduce(ls, 32, DB200_REDUCE_SUM);
            })))
         return st;
       if ((st = fetch(red, 64))) return st;
@@ -612,6 +600,7 @@ int svm_barrier_impl(db200_context* ctx, int n, int r, const double* Z, int ldz,
           double* h_taus = ctx->h_pinned + 256;
           std::memcpy(h_taus, ht, sizeof(ht));
           DB200_CUDA(ctx, cudaMemcpyAsync(taus, h_taus, sizeof(ht), cudaMemcpyHostToDevice, ctx->stream));
+          DB200_CUDA(ctx, cudaMemsetAsync(ls, 0, 32 * sizeof(double), ctx->stream));
           if ((st = bar_linesearch16(ctx, n, a, s, C, taus, ls))) return st;
           if ((st = reduce(ls, 32, DB200_REDUCE_SUM))) return st;
           if ((st = fetch(ls, 32))) return st;
@@ -652,8 +641,7 @@ int svm_barrier_impl(db200_context* ctx, int n, int r, const double* Z, int ldz,
     if ((st = bar_grad_hess(ctx, n, r, Z, ldz, w, a, C, t, g, dinv, red, nullptr, zw))) return st;
     if ((st = reduce_grad())) return st;
     zw_ok = true;
-    if ((st = bar_dot(ctx, r, w, w, sc))) return st;
-    DB200_CUDA(ctx, cudaMemcpyAsync(red + 8, sc, sizeof(double), cudaMemcpyDeviceToDevice, ctx->stream));
+    if ((st = bar_dot(ctx, r, w, w, sc)) || (st = bar_dot(ctx, r, w, w, red + 8))) return st;
     if ((st = fetch(red, 9))) return st;
     suma_now = h[0];
     fa = 0.5 * h[8] - suma_now;
