@@ -9,7 +9,9 @@
 //   nl_scan_kernel     exclusive prefix of the chunk counts, the line count
 //   nl_starts_kernel   byte offset of the start of every line < n     (block-wide ranks of the newlines)
 //   parse_kernel       one warp per line: a 512-byte window staged in shared memory (the next one already in
-//                      flight), token starts by ballot, one token per lane parsed in one pass
+//                      flight), token starts by ballot, one token per lane parsed in one pass.  Bound by instruction
+//                      issue: 16384 x 128 dense decimals 84 us (109 with rounds that ended with the window, 39 of 64
+//                      lanes busy, 64-bit digit loops and byte-wise delimiter masks)
 //
 // Values are converted exactly as glibc's strtod does (correctly rounded to double; for float output the double
 // is then rounded to float, as the reference's `T value = atof(...)`).  Short decimals take Clinger's fast path
@@ -61,18 +63,15 @@ __device__ __forceinline__ uint4 load_seg(const unsigned char* text, long long b
   return make_uint4(w[0], w[1], w[2], w[3]);
 }
 
-// bit k set when byte k of the 16-byte segment is '\n'
-__device__ __forceinline__ uint32_t nl_mask(uint4 v) {
+// bit k set when byte k of the 16-byte segment equals the byte that `c` repeats
+__device__ __forceinline__ uint32_t byte_mask(uint4 v, uint32_t c) {
   const uint32_t w[4] = {v.x, v.y, v.z, v.w};
   uint32_t m = 0;
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const uint32_t r = __vcmpeq4(w[i], 0x0a0a0a0au);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) m |= ((r >> (8 * j + 7)) & 1u) << (4 * i + j);
-  }
+  for (int i = 0; i < 4; ++i) m |= (((__vcmpeq4(w[i], c) & 0x08040201u) * 0x01010101u) >> 24) << (4 * i);
   return m;
 }
+__device__ __forceinline__ uint32_t nl_mask(uint4 v) { return byte_mask(v, 0x0a0a0a0au); }
 
 __device__ __forceinline__ int block_sum(int v, int* red) {
 #pragma unroll
@@ -89,10 +88,12 @@ __device__ __forceinline__ int block_sum(int v, int* red) {
   return t;  // valid in thread 0
 }
 
+// Also clears the call's partial-line count meta[2] and error word meta[3] for the kernels that follow.
 template <bool AL>
 __global__ void __launch_bounds__(NL_THREADS) nl_count_kernel(const unsigned char* text, long long bytes,
-                                                              int* counts) {
+                                                              int* counts, long long* meta) {
   __shared__ int red[NL_THREADS / 32];
+  if (blockIdx.x == 0 && threadIdx.x < 2) meta[2 + threadIdx.x] = threadIdx.x == 0 ? 0 : -1;
   const long long base = (long long)blockIdx.x * CHUNK;
   int c = 0;
 #pragma unroll
@@ -400,11 +401,17 @@ __device__ __forceinline__ unsigned parse_value(const LineBytes L, int q, double
     if (c_hex(c2) || (c2 == '.' && c_hex(L.at(q + 3)))) return E_HEX;
   }
   uint64_t w_hi = 0, w_lo = 0;
+  uint32_t w9 = 0;  // the first nine significant digits, in 32 bits; w_hi takes over at the tenth
   int nsig = 0, e10 = 0;
-  bool any = false, dropped = false;
+  bool any = c_digit(c), dropped = false;
+  while (c_digit(c) && nsig < 9) {
+    w9 = w9 * 10 + (c - '0');
+    nsig += w9 != 0;
+    c = L.at(++q);
+  }
+  if (c_digit(c)) w_hi = w9;
   while (c_digit(c)) {
     const unsigned dg = c - '0';
-    any = true;
     if (nsig == 0 && dg == 0) {
     } else if (nsig < MAX_SIG) {
       if (nsig < 19) w_hi = w_hi * 10 + dg;
@@ -418,9 +425,16 @@ __device__ __forceinline__ unsigned parse_value(const LineBytes L, int q, double
   }
   if (c == '.') {
     c = L.at(++q);
+    any |= c_digit(c);
+    while (c_digit(c) && nsig < 9) {
+      w9 = w9 * 10 + (c - '0');
+      nsig += w9 != 0;
+      --e10;
+      c = L.at(++q);
+    }
+    if (c_digit(c) && w_hi == 0) w_hi = w9;
     while (c_digit(c)) {
       const unsigned dg = c - '0';
-      any = true;
       if (nsig == 0 && dg == 0) {
         --e10;
       } else if (nsig < MAX_SIG) {
@@ -435,6 +449,7 @@ __device__ __forceinline__ unsigned parse_value(const LineBytes L, int q, double
     }
   }
   if (!any) return E_NONE;  // no conversion
+  if (w_hi == 0) w_hi = w9;
   if ((c | 0x20u) == 'e') {
     int r = q + 1;
     unsigned cr = L.at(r);
@@ -488,7 +503,7 @@ __device__ __forceinline__ void report(unsigned long long* err, long long line, 
 // Parse one "index:value" token of line i starting at `pos`, in one pass over its bytes; returns the index
 // written (0 when none).
 template <typename T>
-__device__ __forceinline__ long long feature_token(const LineBytes L, int q, long long i, int d, T* X, long long ldx,
+__device__ __forceinline__ int feature_token(const LineBytes L, int q, long long i, int d, T* X, long long ldx,
                                                    unsigned long long* err) {
   const int start = q;
   unsigned c = L.at(q);
@@ -498,7 +513,12 @@ __device__ __forceinline__ long long feature_token(const LineBytes L, int q, lon
     neg = (c == '-');
     c = L.at(++q);
   }
-  long long idx = 0;
+  uint32_t i9 = 0;  // nine digits in 32 bits, any others in 64
+  for (int k = 0; k < 9 && c_digit(c); ++k) {
+    i9 = i9 * 10 + (c - '0');
+    c = L.at(++q);
+  }
+  long long idx = i9;
   while (c_digit(c)) {
     if (idx < (1ll << 40)) idx = idx * 10 + (c - '0');
     c = L.at(++q);
@@ -517,7 +537,7 @@ __device__ __forceinline__ long long feature_token(const LineBytes L, int q, lon
     return 0;
   }
   X[i * ldx + (idx - 1)] = to_t<T>(v);
-  return idx;
+  return (int)idx;
 }
 
 // 16 bytes of the text at offset o (aligned to 16 when AL), blanks outside the line [s, e).
@@ -553,33 +573,26 @@ __global__ void __launch_bounds__(PARSE_THREADS) parse_kernel(const unsigned cha
     const long long e = (i + 1 <= nl) ? starts[i + 1] : bytes;
     bool prev_space = true;  // the line start acts as a delimiter
     long long tok = 0;       // tokens of this line seen so far
-    long long maxidx = 0;    // largest feature index written so far
+    int maxidx = 0;          // largest feature index written so far
     bool simple = true;      // indices strictly increasing: no two tokens write one element
     long long named = 0;     // feature tokens written (distinct while `simple`)
     // Windows of 512 bytes on 16-byte boundaries of the text, bytes outside [s, e) read as blanks.  The next
     // window's segment is loaded into registers before the current window is parsed, so its memory latency hides
-    // behind the token work; tokens that cross a window's end read the rest through L1.
+    // behind the token work; tokens that cross a window's end read the rest through L1.  Tokens are parsed 32 at a
+    // time: where the line goes on, a window's tokens past the last 32 are left to the next one, which then starts at
+    // the first of them (its lines are in L1), so that rounds are full.
     uint4 vn = line_seg<AL>(text, bytes, (s & ~15ll) + 16 * lane, s, e);
-    for (long long w0 = s & ~15ll; w0 < e; w0 += WIN) {
+    long long w0 = s & ~15ll;
+    while (w0 < e) {
       const uint4 v = vn;
       reinterpret_cast<uint4*>(stage)[lane] = v;
       if (w0 + WIN < e) vn = line_seg<AL>(text, bytes, w0 + WIN + 16 * lane, s, e);
-      const uint32_t wv[4] = {v.x, v.y, v.z, v.w};
       // The reference sees a line as a C string that a NUL byte would end: reject such text.
-      bool has_nul = false;
-#pragma unroll
-      for (int k = 0; k < 16; ++k) has_nul |= ((wv[k >> 2] >> (8 * (k & 3))) & 0xffu) == 0u;
-      if (__any_sync(0xffffffffu, has_nul) && lane == 0) report(err, i, E_NUL);
-      const unsigned last = (wv[3] >> 24) & 0xffu;
-      const unsigned prev_last = (unsigned)__shfl_up_sync(0xffffffffu, (int)last, 1);
-      bool pb = lane == 0 ? prev_space : (prev_last == ' ');
-      uint32_t m = 0;
-#pragma unroll
-      for (int k = 0; k < 16; ++k) {
-        const bool sp = ((wv[k >> 2] >> (8 * (k & 3))) & 0xffu) == ' ';
-        if (!sp && pb) m |= 1u << k;
-        pb = sp;
-      }
+      if (__any_sync(0xffffffffu, byte_mask(v, 0u) != 0u) && lane == 0) report(err, i, E_NUL);
+      const uint32_t sp = byte_mask(v, 0x20202020u);
+      const unsigned prev_last = __shfl_up_sync(0xffffffffu, sp >> 15, 1);
+      const uint32_t pb = lane == 0 ? (prev_space ? 1u : 0u) : prev_last;
+      const uint32_t m = ~sp & ((sp << 1) | pb) & 0xffffu;
       const int c = __popc(m);
       int x = c;
 #pragma unroll
@@ -597,10 +610,12 @@ __global__ void __launch_bounds__(PARSE_THREADS) parse_kernel(const unsigned cha
       }
       __syncwarp();
       const LineBytes L{stage, (unsigned)WIN, w0, text, e};
-      for (int t0 = 0; t0 < total; t0 += 32) {
+      const bool rebase = w0 + WIN < e && total > 32 && (total & 31) != 0;
+      const int use = rebase ? total & ~31 : total;
+      for (int t0 = 0; t0 < use; t0 += 32) {
         const int t = t0 + lane;
-        long long widx = 0;
-        if (t < total) {
+        int widx = 0;
+        if (t < use) {
           const int q = sh[t];
           if (tok + t == 0) {
             double lv64;
@@ -613,22 +628,36 @@ __global__ void __launch_bounds__(PARSE_THREADS) parse_kernel(const unsigned cha
           }
         }
         // every written index must exceed all earlier ones (token order = lane order within a round)
-        long long incl = widx;
+        const int left = __shfl_up_sync(0xffffffffu, widx, 1);
+        if (__all_sync(0xffffffffu, widx > (lane == 0 ? maxidx : left))) {  // a full round in order
+          named += 32;
+          maxidx = __shfl_sync(0xffffffffu, widx, 31);
+          continue;
+        }
+        int incl = widx;
 #pragma unroll
         for (int off = 1; off < 32; off <<= 1) {
-          const long long yv = __shfl_up_sync(0xffffffffu, incl, off);
+          const int yv = __shfl_up_sync(0xffffffffu, incl, off);
           if (lane >= off) incl = incl > yv ? incl : yv;
         }
-        long long before = __shfl_up_sync(0xffffffffu, incl, 1);
+        int before = __shfl_up_sync(0xffffffffu, incl, 1);
         if (lane == 0) before = 0;
         before = before > maxidx ? before : maxidx;
         if (__any_sync(0xffffffffu, widx > 0 && widx <= before)) simple = false;
         named += __popc(__ballot_sync(0xffffffffu, widx > 0));
-        const long long rmax = __shfl_sync(0xffffffffu, incl, 31);
+        const int rmax = __shfl_sync(0xffffffffu, incl, 31);
         maxidx = rmax > maxidx ? rmax : maxidx;
       }
-      tok += total;
-      prev_space = __shfl_sync(0xffffffffu, last == ' ' ? 1 : 0, 31) != 0;
+      tok += use;
+      if (rebase) {
+        const long long from = w0 + sh[use];  // bytes before it read as blanks
+        w0 = from & ~15ll;
+        vn = line_seg<AL>(text, bytes, w0 + 16 * lane, from, e);
+        prev_space = true;
+      } else {
+        w0 += WIN;
+        prev_space = __shfl_sync(0xffffffffu, sp >> 15, 31) != 0;
+      }
       __syncwarp();  // the stage is rewritten by the next window
     }
     if (tok == 0 && lane == 0) report(err, i, E_NOLABEL);
@@ -667,15 +696,13 @@ int parse_impl(db200_context* ctx, const unsigned char* text, long long bytes, i
   int* counts = cv.take<int>((size_t)nchunks + 1);
   long long* prefix = cv.take<long long>((size_t)nchunks + 1);
   long long* starts = cv.take<long long>((size_t)n + 2);
-  long long* meta = cv.take<long long>(3);
-  unsigned long long* err = cv.take<unsigned long long>(1);
-  DB200_CUDA(ctx, cudaMemsetAsync(meta, 0, 3 * sizeof(long long), ctx->stream));
-  DB200_CUDA(ctx, cudaMemsetAsync(err, 0xff, sizeof(unsigned long long), ctx->stream));
+  long long* meta = cv.take<long long>(4);  // newlines, lines, partial lines, first error: one readback
+  unsigned long long* err = reinterpret_cast<unsigned long long*>(meta + 3);
   const bool al = (reinterpret_cast<uintptr_t>(text) & 15u) == 0;
   if (nchunks > 0) {
     if (nchunks > 0x7fffffffLL) return fail(ctx, DB200_ERR_TOO_LARGE, "libsvm: text too large");
-    if (al) nl_count_kernel<true><<<(unsigned)nchunks, NL_THREADS, 0, ctx->stream>>>(text, bytes, counts);
-    else nl_count_kernel<false><<<(unsigned)nchunks, NL_THREADS, 0, ctx->stream>>>(text, bytes, counts);
+    if (al) nl_count_kernel<true><<<(unsigned)nchunks, NL_THREADS, 0, ctx->stream>>>(text, bytes, counts, meta);
+    else nl_count_kernel<false><<<(unsigned)nchunks, NL_THREADS, 0, ctx->stream>>>(text, bytes, counts, meta);
     DB200_CUDA(ctx, cudaGetLastError());
     nl_scan_kernel<<<1, 1024, 0, ctx->stream>>>(counts, (int)nchunks, prefix, text, bytes, n, meta);
     DB200_CUDA(ctx, cudaGetLastError());
@@ -683,7 +710,7 @@ int parse_impl(db200_context* ctx, const unsigned char* text, long long bytes, i
     else nl_starts_kernel<false><<<(unsigned)nchunks, NL_THREADS, 0, ctx->stream>>>(text, bytes, prefix, n, starts);
     DB200_CUDA(ctx, cudaGetLastError());
     long long blocks = ((long long)n + PARSE_THREADS / 32 - 1) / (PARSE_THREADS / 32);
-    const long long cap = (long long)ctx->num_sms * 8;
+    const long long cap = (long long)ctx->num_sms * 64;  // a line per warp up to there: lines differ in length
     if (blocks > cap) blocks = cap;
     if (blocks < 1) blocks = 1;
     if (al)
@@ -694,11 +721,12 @@ int parse_impl(db200_context* ctx, const unsigned char* text, long long bytes, i
                                                                                  ldx, y, err);
     DB200_CUDA(ctx, cudaGetLastError());
     count_launch(ctx, 4);
+  } else {
+    DB200_CUDA(ctx, cudaMemsetAsync(meta, 0, 3 * sizeof(long long), ctx->stream));
+    DB200_CUDA(ctx, cudaMemsetAsync(err, 0xff, sizeof(unsigned long long), ctx->stream));
   }
   // readback: lines parsed and the first error (pinned staging)
-  DB200_CUDA(ctx, cudaMemcpyAsync(ctx->h_pinned, meta, 3 * sizeof(long long), cudaMemcpyDeviceToHost, ctx->stream));
-  DB200_CUDA(ctx, cudaMemcpyAsync(reinterpret_cast<char*>(ctx->h_pinned) + 24, err, sizeof(unsigned long long),
-                                  cudaMemcpyDeviceToHost, ctx->stream));
+  DB200_CUDA(ctx, cudaMemcpyAsync(ctx->h_pinned, meta, 4 * sizeof(long long), cudaMemcpyDeviceToHost, ctx->stream));
   DB200_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   long long hm[3];
   unsigned long long he;
