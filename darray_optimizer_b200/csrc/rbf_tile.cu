@@ -930,7 +930,8 @@ __global__ void __launch_bounds__(256) sum_slabs_kernel(const TileInst* __restri
 // patterns): block maxima, then one atomicMax per block into *out, which the caller zeroes first.  A set without gaps
 // is passed as one row; otherwise a warp walks a row.  vec: 16-byte loads (aligned base, and ld when rows > 1).  Bound
 // by reading the set once (131072 x 128: 67 MB, 19 us; with a 64-bit division per element it took 87 us).
-__global__ void __launch_bounds__(256) absmax_points_kernel(const float* __restrict__ X, long long rows, long long cols,
+// A single CTA stores the maximum and clears out[1..4) itself.
+__global__ void __launch_bounds__(1024) absmax_points_kernel(const float* __restrict__ X, long long rows, long long cols,
                                                             long long ld, int vec, unsigned* __restrict__ out) {
   float mx = 0.f;
   auto take = [&](float x) {
@@ -955,12 +956,16 @@ __global__ void __launch_bounds__(256) absmax_points_kernel(const float* __restr
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-  __shared__ float wmax[8];
+  __shared__ float wmax[32];
   if ((threadIdx.x & 31) == 0) wmax[threadIdx.x / 32] = mx;
   __syncthreads();
-  if (threadIdx.x == 0) {
+  if (threadIdx.x >= 32) return;
+  mx = threadIdx.x < blockDim.x / 32 ? wmax[threadIdx.x] : 0.f;
 #pragma unroll
-    for (int w = 1; w < 8; ++w) mx = fmaxf(mx, wmax[w]);
+  for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  if (gridDim.x == 1) {
+    if (threadIdx.x < 4) out[threadIdx.x] = threadIdx.x == 0 ? __float_as_uint(mx) : 0u;
+  } else if (threadIdx.x == 0) {
     atomicMax(out, __float_as_uint(mx));
   }
 }
@@ -1191,17 +1196,20 @@ int pack_points(db200_context* ctx, const float* X, int ldx, int layout, int n, 
   const bool point_major = layout == DB200_POINT_MAJOR;
   const bool aligned = reinterpret_cast<uintptr_t>(X) % 16 == 0;
   unsigned* mx = reinterpret_cast<unsigned*>(norms + npad);
-  DB200_CUDA(ctx, cudaMemsetAsync(mx, 0, 4 * sizeof(unsigned), ctx->stream));  // max |x|, scale, lo flag
+  long long rows = point_major ? n : d, cols = point_major ? d : n;
+  if (ldx == cols) {
+    cols *= rows;
+    rows = 1;
+  }
+  // mx: max |x|, scale, lo flag.  A small set takes one CTA, which clears them itself: 1024 x 32, 3.6 us; eight CTAs 2.3
+  // behind a clear of 1.0 and its gap of 2 (the whole sketch of 64 columns 28.9 and 30.6 us).
+  const bool one = n > 0 && rows <= 256 && rows * cols <= 32768;
+  if (!one) DB200_CUDA(ctx, cudaMemsetAsync(mx, 0, 4 * sizeof(unsigned), ctx->stream));
   if (n > 0) {
-    long long rows = point_major ? n : d, cols = point_major ? d : n;
-    if (ldx == cols) {
-      cols *= rows;
-      rows = 1;
-    }
     const bool vec = aligned && (rows == 1 || ldx % 4 == 0);
     const long long work = rows == 1 ? (cols + 4095) / 4096 : (rows + 7) / 8;  // 16 elements a thread, a row a warp
-    const unsigned blocks = (unsigned)std::max(1LL, std::min(work, 8LL * ctx->num_sms));
-    absmax_points_kernel<<<blocks, 256, 0, ctx->stream>>>(X, rows, cols, ldx, vec ? 1 : 0, mx);
+    const unsigned blocks = one ? 1u : (unsigned)std::max(1LL, std::min(work, 8LL * ctx->num_sms));
+    absmax_points_kernel<<<blocks, one ? 1024 : 256, 0, ctx->stream>>>(X, rows, cols, ldx, vec ? 1 : 0, mx);
     DB200_CUDA(ctx, cudaGetLastError());
     count_launch(ctx);
   }
