@@ -603,7 +603,7 @@ int potrf_upper(db200_context* ctx, double* A, int lda, int l, int* d_status, in
   // the diagonal-block kernel's arrival counter starts every factorisation at zero
   DB200_CUDA(ctx, cudaMemsetAsync(ctx->d_status + 1, 0, sizeof(int), ctx->stream));
   // A trailing matrix of at least one wave of 128 x 128 upper tiles takes its update on the FP64 tensor cores
-  // (gram_kernel, alpha = -1, added in place).  While the matrix beyond the next 8 nb columns is that large, the
+  // (dmm_kernel, alpha = -1, added in place).  While the matrix beyond the next 8 nb columns is that large, the
   // factor goes by outer panels of 8 nb columns: each nb-block of the panel is factored (potrf_block_kernel, which
   // also solves its row to the last column), the panel's own later rows are updated at once (a strip of at most
   // 7 nb rows), and the trailing matrix takes one rank-8 nb update per panel instead of eight rank-nb ones

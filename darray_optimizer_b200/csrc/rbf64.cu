@@ -277,7 +277,7 @@ static int r64_tile_cols(int l, int dp) {
 }
 
 // Ranges of j: the least waves x (stages of a range + 8, a CTA's start and end in stages), at least 16 stages each; cut
-// only where that is below 0.9 of the whole, for the slabs' sum.  4096 x 4096, d = 16, l = 138 (64 row blocks): whole,
+// only where that is below 0.9 of the whole, for the slabs' sum.  4096 x 4096, d = 32, l = 138 (64 row blocks): whole,
 // one CTA an SM, 679 us; in 4 ranges, two CTAs an SM, 282.
 static int r64_splits(const db200_context* ctx, int blocks, int per_sm, int n_stages) {
   const long long slots = (long long)ctx->num_sms * per_sm;

@@ -162,7 +162,7 @@ DB200_API int db200_lra_host(db200_context* ctx, int n, int d, int k, const floa
 
 /* In-place upper Cholesky A = R^T R of the n x n matrix A (only the upper triangle is read; the strictly lower
  * part is zeroed), blocked right-looking with block size nb (<= 64; 0 = 64).  With nb = 64 and n <= 544 the whole
- * factor is one kernel on a thread-block cluster, in 32-column steps (the failing block named below is then the
+ * factor is one kernel on a thread-block cluster, in 64-column steps (the failing block named below is then the
  * 32-row block).  A non-positive pivot returns
  * DB200_ERR_NOT_SPD (db200_last_error names the failing block).  Replaces cholesky_factorize(A, 'U', n, 0, bs)
  * and cholesky_factorize_recursive (include/lapack_like.h:10-90), in FP64.  Synchronous. */
@@ -205,9 +205,9 @@ typedef struct db200_barrier_params {
  *   promoted fp32 accumulation (range finder DB200_SKETCH_COMPENSATED_PROMOTED_COARSE, final pass
  *   DB200_SKETCH_COMPENSATED_PROMOTED), which keeps the dual objective within ~5e-7 of the FP64 path's; the
  *   Woodbury capacity matrix
- *   I + Z^T D^-1 Z formed in integers on the int8 tensor cores from 8 signed 7-bit slices of every column (Ozaki
- *   scheme, error ~3e-14 of the column norms; from r = 2048 first 6 slices, ~3e-10, while refinement converges
- *   with them) and factored in FP64 while each Newton step refined
+ *   I + Z^T D^-1 Z formed in integers on the int8 tensor cores from seven base-256 digits of every value (Ozaki
+ *   scheme, error ~1e-15 of the column norms; from r = 2048 first 6 signed 7-bit digits, ~3e-10, while refinement
+ *   converges with them) and factored in FP64 while each Newton step refined
  *   against the exact FP64 operator (Z Z^T + D) reaches relative residual 1e-10, the FP64 capacity matrix after;
  *   objective, gradients, gap and line search in FP64.
  * DB200_FP64: plain FP64 everywhere (FP64 kernel blocks and products, FP64 capacity matrix): the comparator.
