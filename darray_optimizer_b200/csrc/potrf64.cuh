@@ -5,13 +5,13 @@
 // group, rows 8 b + 2 t and + 1 in d0, d1; column g + 8 in d2, d3), which are at once the A fragments of a product
 // over those rows (the pairing k = 2t, 2t + 1 inside the instruction is free).  Warps 0..3 hold the block's own column
 // groups, the others column groups of the block row.  In four steps p of 16 rows:
-//   warp p factors its 16 x 16 diagonal block (factor16): one warp, lane = column, with the 16 columns of the identity
-//     in the other half-warp, so the elimination also leaves W = R_pp^-T;
+//   warp p factors its 16 x 16 diagonal block (factor16, whose elimination keeps the factor's backward error at a few u):
+//     one warp, lane = column, with the 16 columns of the identity in the other half-warp, so it also leaves W = R_pp^-T;
 //   every later group solves its rows p, X = W B, then X += W (B - R_pp^T X): the correction makes the solve as
 //     backward stable as substitution, whose 16 dependent steps it replaces by three 16 x 16 products;
 //   every later group subtracts R_pr^T X_p from its rows r > p.
-// What bounds it is the chain of 64 pivots, taken two at a time (a shuffle, a reciprocal and some products per pair):
-// 23.6 k cycles for a full block with 64 columns of its block row, of which the four 16 x 16 factors take 16 k.  One
+// What bounds it is the chain of 64 pivots, taken two at a time (a shuffle, a reciprocal, the reduced row through shared
+// memory and some products per pair): 23.6 k cycles for a full block with 64 columns of its block row, of which the four 16 x 16 factors take 16 k.  One
 // 64-column step of the blocked factor takes 21.5 us; with a barrier, a division and a strip update per pivot, and the
 // block row solved by 64 dependent shuffle steps, it took 38.8 us.
 #pragma once
@@ -53,54 +53,62 @@ __device__ __forceinline__ void p64_mma_tile(double* d, const double* a, double 
 // Factor of the staged 16 x 16 block D (upper entries) by one warp: R into Rb (column major, ld P64_RLD, zeros below
 // the diagonal), W = R^-T; returns false on a non-positive or NaN pivot (the same answer in every lane).  Rows are
 // eliminated unscaled and divided by the square roots of their pivots at the end, two at a time: with the 2 x 2
-// pivot [p q; q r], det = p r - q^2, the rows below lose [a_im a_i+1,m] [p q; q r]^-1 [a_i; a_i+1], so that one reciprocal
-// (of det) sits on the chain per two columns; the second pivot is det / p.
+// pivot [p q; q r], det = p r - q^2 and the second row reduced by the first, u = a_i+1 - (q / p) a_i, the rows below lose
+// a_im a_i / p + u_m u (p / det), so that one reciprocal's latency (1 / p and 1 / det are independent) sits on the chain
+// per two columns; the second pivot is det / p.  Applying [p q; q r]^-1 to the unreduced rows instead is shorter by a
+// shared-memory round trip, but its errors grow by 1 / (1 - rho^2) for columns i, i + 1 of correlation rho, where
+// eliminating one row at a time (and this form) leaves a few u |A| whatever the matrix.
+// The block is first scaled symmetrically by powers of two to diagonal entries in [1, 4), exactly, so that det neither
+// overflows nor underflows for any range of the entries, and R and W are scaled back at the end.
 static __device__ __noinline__ bool p64_factor16(P64Smem& S, double* Rb, double* Wb) {
   const int lane = threadIdx.x % 32, j = lane & 15;
   const bool unit = lane >= 16;  // a column of the identity
+  const int k2 = (((__double2hiint(S.D[j * P64_DLD + j]) >> 20) & 0x7ff) - 1023) >> 1;
+  const double s = __hiloint2double((1023 - k2) << 20, 0), s_inv = __hiloint2double((1023 + k2) << 20, 0);
+  if (!unit) S.rs[j] = s;
+  __syncwarp();
   double a[16];
 #pragma unroll
   for (int m = 0; m < 16; m += 2) {
     const double2 v = *reinterpret_cast<const double2*>(S.D + j * P64_DLD + m);
-    a[m] = unit ? (m == j ? 1.0 : 0.0) : v.x;
-    a[m + 1] = unit ? (m + 1 == j ? 1.0 : 0.0) : v.y;
+    const double2 sm = *reinterpret_cast<const double2*>(S.rs + m);
+    a[m] = unit ? (m == j ? 1.0 : 0.0) : v.x * sm.x * s;
+    a[m + 1] = unit ? (m + 1 == j ? 1.0 : 0.0) : v.y * sm.y * s;
   }
   double dg = 1.0;
   bool ok = true;
 #pragma unroll
   for (int i = 0; i < 16; i += 2) {
     double* rb = S.row + (i & 2) * 16;
-    if (!unit) {
-      rb[j] = a[i];
-      rb[16 + j] = a[i + 1];
-    }
+    if (!unit) rb[j] = a[i];
     const double p = __shfl_sync(0xffffffffu, a[i], i), q = __shfl_sync(0xffffffffu, a[i], i + 1);
     const double r = __shfl_sync(0xffffffffu, a[i + 1], i + 1);
     const double det = fma(p, r, -q * q);
     const double ip = 1.0 / p, id = 1.0 / det;
-    ok = ok && p > 0.0 && det > 0.0;
-    const double y0 = (r * a[i] - q * a[i + 1]) * id, y1 = (p * a[i + 1] - q * a[i]) * id;
+    a[i + 1] = fma(-q * ip, a[i], a[i + 1]);
+    if (!unit) rb[16 + j] = a[i + 1];
+    const double y0 = a[i] * ip, y1 = a[i + 1] * (p * id), second = det * ip;
+    ok = ok && p > 0.0 && second > 0.0;
     __syncwarp();
 #pragma unroll
     for (int m = i + 2; m < 16; ++m) a[m] = fma(-rb[m], y0, fma(-rb[16 + m], y1, a[m]));
-    a[i + 1] = fma(-q * ip, a[i], a[i + 1]);
     if (lane == i) dg = p;
-    if (lane == i + 1) dg = det * ip;
+    if (lane == i + 1) dg = second;
   }
   if (!ok) return false;
-  const double sq = sqrt(dg);
+  const double sq = sqrt(dg), back = unit ? s : s_inv;
   if (!unit) S.rs[j] = 1.0 / sq;
   __syncwarp();
 #pragma unroll
   for (int i = 0; i < 16; i += 2) {
     const double2 rs = *reinterpret_cast<const double2*>(S.rs + i);
-    const double v0 = a[i] * rs.x, v1 = a[i + 1] * rs.y;
+    const double v0 = a[i] * rs.x * back, v1 = a[i + 1] * rs.y * back, d = sq * back;
     if (unit) {
       Wb[i * P64_WLD + j] = (i >= j) ? v0 : 0.0;
       Wb[(i + 1) * P64_WLD + j] = (i + 1 >= j) ? v1 : 0.0;
     } else {
       *reinterpret_cast<double2*>(Rb + j * P64_RLD + i) =
-          make_double2(i < j ? v0 : (i == j ? sq : 0.0), i + 1 < j ? v1 : (i + 1 == j ? sq : 0.0));
+          make_double2(i < j ? v0 : (i == j ? d : 0.0), i + 1 < j ? v1 : (i + 1 == j ? d : 0.0));
     }
   }
   return true;
