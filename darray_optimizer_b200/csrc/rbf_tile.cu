@@ -1145,11 +1145,13 @@ cudaLaunchConfig_t launch_config(cudaLaunchAttribute* attr, int clusters, size_t
 }
 
 // Persistent grid size: as many CTA pairs as can be resident at once, no more than there are items.  Not
-// stream-ordered (so launches can be captured in a CUDA graph afterwards).
+// stream-ordered (so launches can be captured in a CUDA graph afterwards).  The kernel's shared-memory limit is the
+// device's, whatever this plan takes: it belongs to the function, so a limit of this plan's size would refuse the launch
+// of a larger plan prepared before it (a batch's two kinds of pass) or by another thread.
 template <int MODE, bool LEAN>
 cudaError_t plan_clusters(size_t smem, int max_clusters, int n_items, int* clusters) {
   auto k = rbf_tile_kernel<MODE, LEAN>;
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_LIMIT);
   if (e != cudaSuccess) return e;
   cudaLaunchAttribute attr[1];
   cudaLaunchConfig_t cfg = launch_config(attr, max_clusters, smem, nullptr);
