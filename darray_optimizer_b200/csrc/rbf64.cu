@@ -256,10 +256,13 @@ __global__ void __launch_bounds__(256) sum_slabs64_kernel(const R64Args a, int r
   }
 }
 
+constexpr size_t R64_SMEM_MAX = 227 * 1024;
+
 template <int NT>
 cudaError_t launch_r64(const R64Args& a, dim3 blocks, size_t smem, cudaStream_t st) {
   auto k = rbf_sketch_f64_kernel<NT>;
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  // the most any call takes: the limit belongs to the function, which other threads launch with other sizes
+  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)R64_SMEM_MAX);
   if (e != cudaSuccess) return e;
   k<<<blocks, R64_THREADS, smem, st>>>(a);
   return cudaGetLastError();
@@ -269,7 +272,6 @@ cudaError_t launch_r64(const R64Args& a, dim3 blocks, size_t smem, cudaStream_t 
 
 // Sketch tile width: up to 264 columns (33 n8 tiles) per CTA; small sketches, and wide points whose Xi tile
 // leaves too little shared memory, take narrower tiles.
-constexpr size_t R64_SMEM_MAX = 227 * 1024;
 static int r64_tile_cols(int l, int dp) {
   if (l <= 16 || r64_smem_bytes(dp, 144) > R64_SMEM_MAX) return 16;
   if (l <= 144 || r64_smem_bytes(dp, 264) > R64_SMEM_MAX) return 144;
