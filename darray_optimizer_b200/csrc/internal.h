@@ -179,7 +179,8 @@ size_t sketch_slab_floats(const SketchPlan& plan, int npad_i, int npad_j, int l,
 // A prepared launch: the instance table is on the device; launch_rbf_plan only launches (graph-capturable).
 struct TilePlan {
   int mode = 0, count = 0, n_items = 0, nsx = 0, nso = 0, nkc_max = 0, panel_max = 0, om_mult = 1, kblock = 0, yacc = 0;
-  int red_m = 0, red_l = 0;  // largest split sketch (0: none): its ranges are summed after the tile launch
+  int sum_list = 0;        // > 0, or sum_grid.z > 0: split sketches, whose ranges are summed after the tile launch
+  dim3 sum_grid{0, 0, 0};
   int clusters = 0;  // persistent grid: CTA pairs resident at once (at most one per item)
   bool lean = false; // SKETCH with the single product and no promotion in every instance: the lean kernel
   size_t smem = 0;

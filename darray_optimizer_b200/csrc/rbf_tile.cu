@@ -909,19 +909,34 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) rbf_tile_kernel(const __grid_c
   if (warp == 1) tmem_dealloc_pair(tmem_base, TMEM_COLS);
 }
 
-// Y(i, c) = the sum over the ranges of the j tiles, in their order, of the partial sums in the slabs (blockIdx.z: the
-// instance; those of one range wrote Y themselves).
-__global__ void __launch_bounds__(256) sum_slabs_kernel(const TileInst* __restrict__ inst) {
-  const TileInst* I = inst + blockIdx.z;
-  const int S = I->n_splits, i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (S <= 1 || i >= I->m) return;
-  const long long stride = I->split_stride, ldo = I->ldo, ldy = I->red_ldo;
-  for (int c = blockIdx.y; c < I->l; c += gridDim.y) {
-    const float* p = I->out + c * ldo + i;
-    float acc = p[0];
+// Y(i, c) = the sum over the ranges of the j tiles, in their order, of the partial sums in the slabs, for every instance
+// that has several (those of one range wrote Y themselves), in pieces of 256 rows of a column.  GRID: a CTA per piece of
+// the largest instance and instance (blockIdx.z), for few instances of like size.  Otherwise the CTAs walk one list of all
+// instances' pieces: that grid was 4 million CTAs, almost all empty, for a batch of 64 (10 ms of a pass of 110).
+template <bool GRID>
+__global__ void __launch_bounds__(256) sum_slabs_kernel(const TileInst* __restrict__ inst, int count) {
+  int u = blockIdx.x;  // !GRID: this CTA's next piece, counted from the instance's first (slabs: fewer than 2^31 bytes)
+  for (int b = GRID ? blockIdx.z : 0; b < (GRID ? (int)blockIdx.z + 1 : count); ++b) {
+    const TileInst* I = inst + b;
+    const int S = I->n_splits, m = I->m, l = I->l;
+    if (S <= 1) continue;
+    const long long stride = I->split_stride, ldo = I->ldo, ldy = I->red_ldo;
+    auto piece = [&](int i, int c) {
+      if (i >= m) return;
+      const float* p = I->out + c * ldo + i;
+      float acc = p[0];
 #pragma unroll 4
-    for (int k = 1; k < S; ++k) acc += p[k * stride];
-    I->red_out[c * ldy + i] = acc;
+      for (int k = 1; k < S; ++k) acc += p[k * stride];
+      I->red_out[c * ldy + i] = acc;
+    };
+    if (GRID) {
+      for (int c = blockIdx.y; c < l; c += gridDim.y) piece(blockIdx.x * 256 + threadIdx.x, c);
+    } else {
+      const unsigned rows = (unsigned)(m + 255) / 256, pieces = rows * (unsigned)l;
+      for (; u < (int)pieces; u += gridDim.x)
+        piece((int)((unsigned)u % rows) * 256 + (int)threadIdx.x, (int)((unsigned)u / rows));
+      u -= (int)pieces;
+    }
   }
 }
 
@@ -1240,7 +1255,8 @@ int prepare_rbf_tiles(db200_context* ctx, int mode, const TileJob* jobs, int cou
                       size_t table_capacity, TilePlan* plan) {
   if (count < 1 || !jobs || !plan) return fail(ctx, DB200_ERR_INVALID, "rbf tiles: empty job list");
   std::vector<TileInst> host((size_t)count);
-  int items = 0, nkc_max = 1, panel_max = 16, om_mult = 1, red_m = 0, red_l = 0;
+  int items = 0, nkc_max = 1, panel_max = 16, om_mult = 1, sum_rows = 0, sum_cols = 0;
+  long long pieces = 0;  // of split sketches, for the sum of their ranges
   int kblock = (mode == RBF_MODE_KBLOCK || mode == RBF_MODE_KNN) ? 1 : 0;
   for (int b = 0; b < count; ++b) {
     const TileJob& J = jobs[b];
@@ -1327,8 +1343,10 @@ int prepare_rbf_tiles(db200_context* ctx, int mode, const TileJob* jobs, int cou
       I.out = J.slab;
       I.ldo = J.slab_ld;
       I.split_stride = J.slab_stride;
-      red_m = std::max(red_m, I.m);
-      red_l = std::max(red_l, I.l);
+      const int rows = (I.m + 255) / 256;
+      pieces += (long long)rows * I.l;
+      sum_rows = std::max(sum_rows, rows);
+      sum_cols = std::max(sum_cols, std::min(I.l, 256));
     }
     items += I.n_itiles * I.n_panels * I.n_splits;
     nkc_max = std::max(nkc_max, I.nkc);
@@ -1338,8 +1356,10 @@ int prepare_rbf_tiles(db200_context* ctx, int mode, const TileJob* jobs, int cou
   T.mode = mode;
   T.count = count;
   T.n_items = items;
-  T.red_m = red_m;
-  T.red_l = red_l;
+  if (pieces > 0 && (long long)sum_rows * sum_cols * count <= 2 * pieces && count <= 65535)
+    T.sum_grid = dim3((unsigned)sum_rows, (unsigned)sum_cols, (unsigned)count);
+  else if (pieces > 0)
+    T.sum_list = (int)std::min<long long>(pieces, 32LL * ctx->num_sms);
   T.nkc_max = nkc_max;
   T.panel_max = panel_max;
   T.nso = (mode == RBF_MODE_SKETCH) ? MAX_NSO : 0;
@@ -1432,9 +1452,10 @@ int launch_rbf_plan(db200_context* ctx, const TilePlan& T) {
   DB200_CUDA(ctx, err);
   prof_end(ctx, e0);
   count_launch(ctx);
-  if (T.red_m > 0) {
-    const dim3 grid((unsigned)((T.red_m + 255) / 256), (unsigned)std::min(T.red_l, 256), (unsigned)T.count);
-    sum_slabs_kernel<<<grid, 256, 0, ctx->stream>>>(static_cast<const TileInst*>(T.table));
+  if (T.sum_list > 0 || T.sum_grid.z > 0) {
+    const TileInst* inst = static_cast<const TileInst*>(T.table);
+    if (T.sum_list > 0) sum_slabs_kernel<false><<<T.sum_list, 256, 0, ctx->stream>>>(inst, T.count);
+    else sum_slabs_kernel<true><<<T.sum_grid, 256, 0, ctx->stream>>>(inst, T.count);
     DB200_CUDA(ctx, cudaGetLastError());
     count_launch(ctx);
   }
