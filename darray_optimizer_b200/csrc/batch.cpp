@@ -115,31 +115,46 @@ int db200_rbf_sketch_batched(db200_context* ctx, int count, const db200_sketch_j
   if (!ctx) return DB200_ERR_INVALID;
   if (count < 0 || (count > 0 && !jobs)) return fail(ctx, DB200_ERR_INVALID, "rbf_sketch_batched: bad arguments");
   if (count == 0) return DB200_OK;
-  size_t bytes = 4096;
+  // Ranges of the points j, as db200_rbf_sketch cuts each problem alone: its partial sums are added in the same order, so
+  // a problem gives the same result alone and in a batch.  A batch that leaves CTA pairs idle takes them as work items of
+  // their own, with slabs; one that fills the GPU lets each row block walk its ranges, its accumulation chunk one range
+  // (a second launch takes the problems that have one range, in the leaner kernel).  Whole call, ms: 64 problems of 2048
+  // points (l = 144) walked 1.34, split 1.61, 16 of them 0.36 and 0.41; 64 of 1024 to 4096 points 1.59 and 1.85; 64 of
+  // 4096 points (l = 272) 2.24 and 2.65; one of 2048 points split 0.039, whole 0.049.
+  size_t bytes = 4096, slab_bytes = 0;
   std::vector<SketchPlan> plans((size_t)count);
+  std::vector<int> split((size_t)count);
+  TileLoad walked, whole, all;
   for (int b = 0; b < count; ++b) {
     const db200_sketch_job& J = jobs[b];
     if (J.m < 1 || J.n < 1 || J.d < 1 || J.d > 128 || J.l < 1 || !J.Xi || !J.Xj || J.ldxi < J.d || J.ldxj < J.d ||
         !J.Omega || J.ldo < J.n || !J.Y || J.ldy < J.m)
       return fail(ctx, DB200_ERR_INVALID, "rbf_sketch_batched: bad job " + std::to_string(b));
-    plans[(size_t)b] = job_plan(J.l, J.n_panels, J.panel, J.g_bufs);
-    bytes += packed_bytes(J.m, J.n, J.d, J.Xi == J.Xj && J.ldxi == J.ldxj && J.m == J.n, plans[(size_t)b]);
+    SketchPlan& P = plans[(size_t)b];
+    P = job_plan(J.l, J.n_panels, J.panel, J.g_bufs);
+    bytes += packed_bytes(J.m, J.n, J.d, J.Xi == J.Xj && J.ldxi == J.ldxj && J.m == J.n, P);
     const int mp = point_pad(J.m), np = point_pad(J.n);
-    bytes += align_up(sketch_slab_floats(plans[(size_t)b], mp, np, J.l, sketch_split(ctx, plans[(size_t)b], mp, np, J.l)) *
-                          4,
-                      256);
+    split[(size_t)b] = sketch_split(ctx, P, mp, np, J.l);
+    slab_bytes += align_up(sketch_slab_floats(P, mp, np, J.l, split[(size_t)b]) * 4, 256);
+    const SketchLoad L = sketch_load(P, mp, np, split[(size_t)b]);
+    all.add(L.split);
+    if (L.ranges > 1) walked.add(L.walked);
+    else whole.add(L.whole);
   }
+  const bool slabs =
+      slab_bytes <= MAX_BATCH_SLABS && (count == 1 || all.time(ctx) < walked.time(ctx) + whole.time(ctx));
+  if (slabs) bytes += slab_bytes;
   void* ws = workspace(ctx, bytes);
   if (!ws) return DB200_ERR_NOMEM;
   Carve cv{static_cast<char*>(ws)};
-  std::vector<TileJob> tj((size_t)count);
+  std::vector<TileJob> tj[2];  // [1]: problems that walk their ranges
   for (int b = 0; b < count; ++b) {
     const db200_sketch_job& J = jobs[b];
     Packed P;
     int st = pack_problem(ctx, J.m, J.n, J.d, J.Xi, J.ldxi, J.Xj, J.ldxj, plans[(size_t)b], cv, &P);
     if (!st) st = pack_sketch(ctx, J.Omega, J.ldo, J.yj, J.n, J.l, P.npad_j, P.plan.lrows, P.op);
     if (st) return st;
-    TileJob& T = tj[(size_t)b];
+    TileJob T;
     T.pi = P.pi;
     T.pj = P.pj;
     T.yi = J.yi;
@@ -150,14 +165,19 @@ int db200_rbf_sketch_batched(db200_context* ctx, int count, const db200_sketch_j
     T.gamma = J.gamma;
     T.out = J.Y;
     T.ldo = J.ldy;
-    const int split = sketch_split(ctx, P.plan, P.npad_i, P.npad_j, J.l);
-    const size_t slab = sketch_slab_floats(P.plan, P.npad_i, P.npad_j, J.l, split);
-    if (slab) T.set_split(split, cv.take<float>(slab));
+    const size_t slab = sketch_slab_floats(P.plan, P.npad_i, P.npad_j, J.l, split[(size_t)b]);
+    if (slab && slabs) T.set_split(split[(size_t)b], cv.take<float>(slab));
+    if (slab && !slabs) T.plan.promote = split[(size_t)b];
+    tj[slab && !slabs].push_back(T);
   }
-  TilePlan plan;
-  int st = prepare_rbf_tiles(ctx, RBF_MODE_SKETCH, tj.data(), count, nullptr, 0, &plan);
-  if (st) return st;
-  return launch_rbf_plan(ctx, plan);
+  for (const std::vector<TileJob>& list : tj) {
+    if (list.empty()) continue;
+    TilePlan plan;
+    int st = prepare_rbf_tiles(ctx, RBF_MODE_SKETCH, list.data(), (int)list.size(), nullptr, 0, &plan);
+    if (!st) st = launch_rbf_plan(ctx, plan);
+    if (st) return st;
+  }
+  return DB200_OK;
 }
 
 int db200_svm_solve_batched(db200_context* ctx, int count, const db200_svm_instance* inst, int q,
@@ -194,6 +214,13 @@ int db200_svm_solve_batched(db200_context* ctx, int count, const db200_svm_insta
     const int np = point_pad(I.n);
     return sketch_slab_floats(p, np, np, I.l, sketch_split(ctx, p, np, np, I.l));
   };
+  // A pass is one launch per group of instances: those without slabs and as many of the others as MAX_BATCH_SLABS holds,
+  // then more of the others on the same slabs.  (Row blocks kept whole instead would need none, but another order of the
+  // fp32 sums moves a solve's objective by up to 4e-6 against the single solve's.)
+  std::vector<int> group((size_t)count, 0);
+  std::vector<size_t> slab_at((size_t)count);
+  size_t slab_used = 0, slab_area = 0;
+  int groups = 1;
   size_t wbytes = 4096, pbytes = 4096 + (size_t)workers * 256;  // + the final pass's instance table, below
   int njobs = 0;  // tile-engine instances: default multi-panel plans split into exact-width panels
   for (int b = 0; b < count; ++b) {
@@ -205,12 +232,21 @@ int db200_svm_solve_batched(db200_context* ctx, int count, const db200_svm_insta
     slab_floats[(size_t)b] = pass_slab(plans[(size_t)b], I, false);
     if (plans[(size_t)b].comp == 2)
       slab_floats[(size_t)b] = std::max(slab_floats[(size_t)b], pass_slab(plans[(size_t)b], I, true));
-    wbytes += align_up(slab_floats[(size_t)b] * 4, 256);
+    if (const size_t bytes = align_up(slab_floats[(size_t)b] * 4, 256)) {
+      if (slab_used > 0 && slab_used + bytes > MAX_BATCH_SLABS) {
+        ++groups;
+        slab_used = 0;
+      }
+      group[(size_t)b] = groups - 1;
+      slab_at[(size_t)b] = slab_used;
+      slab_used += bytes;
+      slab_area = std::max(slab_area, slab_used);
+    }
     njobs += (I.n_panels <= 0) ? plans[(size_t)b].n_panels : 1;
     const size_t nl = (size_t)I.n * I.l, ll = (size_t)I.l * I.l;
     pbytes += 2 * align_up(nl * 4, 256) + align_up(nl * 8, 256) + 2 * align_up(ll * 8, 256);
   }
-  wbytes += align_up(tile_table_bytes(njobs), 256);
+  wbytes += slab_area + 2 * (tile_table_bytes(njobs) + (size_t)groups * 256);
   void* ws = workspace(ctx, wbytes);
   char* base = static_cast<char*>(slot_buffer(ctx, SLOT_PIPE, pbytes + 4096));
   if (!ws || !base) return DB200_ERR_NOMEM;
@@ -245,8 +281,8 @@ int db200_svm_solve_batched(db200_context* ctx, int count, const db200_svm_insta
   // Tile-engine instances.  A default plan of several panels is split into exact-width panels and ranges of the points j,
   // as the single-problem path splits it, so each instance's passes are the single solve's to the bit; an explicit
   // (autotuned) plan is kept as one instance of equal panels.
-  std::vector<TileJob> tj;
-  tj.reserve((size_t)njobs);
+  std::vector<std::vector<TileJob>> tj((size_t)groups);
+  char* slabs = slab_area ? cw.take<char>(slab_area) : nullptr;
   for (int b = 0; b < count; ++b) {
     TileJob T;
     T.pi = pk[(size_t)b].pi;
@@ -261,35 +297,38 @@ int db200_svm_solve_batched(db200_context* ctx, int count, const db200_svm_insta
     T.ldo = inst[b].n;
     const int np = T.pi.npad;
     if (slab_floats[(size_t)b])
-      T.set_split(sketch_split(ctx, T.plan, np, np, T.l), cw.take<float>(slab_floats[(size_t)b]));
+      T.set_split(sketch_split(ctx, T.plan, np, np, T.l), reinterpret_cast<float*>(slabs + slab_at[(size_t)b]));
     if (T.plan.comp == 2) {  // the final pass's ranges: the same slabs, multiples of its own chunks
       SketchPlan pf = T.plan;
       pf.promote = 2;
       T.split_final = T.slab ? sketch_split(ctx, pf, np, np, T.l) : 0;
     }
-    if (inst[b].n_panels <= 0) exact_panel_jobs(T, tj);
-    else tj.push_back(T);
+    std::vector<TileJob>& list = tj[(size_t)group[(size_t)b]];
+    if (inst[b].n_panels <= 0) exact_panel_jobs(T, list);
+    else list.push_back(T);
   }
-  const int nj = (int)tj.size();
-  TilePlan tplan, tplan_final;
-  if ((st = prepare_rbf_tiles(ctx, RBF_MODE_SKETCH, tj.data(), nj, nullptr, 0, &tplan))) return st;
-  // the final pass (Y = K Q, contracted into the Nystrom core, whose scale the accumulation's truncation would
-  // shrink) promotes every two j tiles, as db200_lowrank's final pass does; its instance table is in the workspace
-  for (TileJob& T : tj)
-    if (T.plan.comp == 2) {
-      T.plan.promote = 2;
-      T.split_tiles = T.split_final;
+  // [0]: the range-finder passes; [1]: the final pass (Y = K Q, contracted into the Nystrom core, whose scale the
+  // accumulation's truncation would shrink) promotes every two j tiles, as db200_lowrank's final pass does
+  std::vector<TilePlan> pass_plans[2];
+  for (std::vector<TilePlan>& plist : pass_plans) {
+    for (std::vector<TileJob>& list : tj) {
+      const int nj = (int)list.size();
+      if (&plist == &pass_plans[1])
+        for (TileJob& T : list)
+          if (T.plan.comp == 2) {
+            T.plan.promote = 2;
+            T.split_tiles = T.split_final;
+          }
+      TilePlan plan;
+      void* table = cw.take<char>(tile_table_bytes(nj));
+      if ((st = prepare_rbf_tiles(ctx, RBF_MODE_SKETCH, list.data(), nj, table, tile_table_bytes(nj), &plan))) return st;
+      plist.push_back(plan);
     }
-  {
-    void* table_final = cw.take<char>(tile_table_bytes(nj));
-    if ((st = prepare_rbf_tiles(ctx, RBF_MODE_SKETCH, tj.data(), nj, table_final, tile_table_bytes(nj),
-                                &tplan_final)))
-      return st;
   }
 
   // ---- one kernel pass over every instance: pack each test matrix (Omega, or Q from the previous pass), then one
-  // persistent launch.  After the first Q pass the sequence is captured once and replayed.
-  auto enqueue_pass = [&](bool from_omega, const TilePlan& tp) -> int {
+  // persistent launch per group.  After the first Q pass the sequence is captured once and replayed.
+  auto enqueue_pass = [&](bool from_omega, bool final_pass) -> int {
     for (int b = 0; b < count; ++b) {
       const db200_svm_instance& I = inst[b];
       const float* src = from_omega ? I.Omega : Qf[(size_t)b];
@@ -298,10 +337,13 @@ int db200_svm_solve_batched(db200_context* ctx, int count, const db200_svm_insta
                            pk[(size_t)b].op, pk[(size_t)b].plan.comp);
       if (s2) return s2;
     }
-    return launch_rbf_plan(ctx, tp);
+    for (const TilePlan& plan : pass_plans[final_pass ? 1 : 0])
+      if (int s2 = launch_rbf_plan(ctx, plan)) return s2;
+    return DB200_OK;
   };
   cudaStream_t cs = nullptr;
   cudaGraphExec_t graphs[2] = {nullptr, nullptr};  // the range-finder Q pass and the final pass
+  int graph_launches[2] = {0, 0};
   cudaEvent_t ev = nullptr;
   auto cleanup = [&]() {
     for (cudaGraphExec_t& g : graphs)
@@ -310,8 +352,7 @@ int db200_svm_solve_batched(db200_context* ctx, int count, const db200_svm_insta
     if (ev) cudaEventDestroy(ev);
   };
   auto q_pass = [&](bool final_pass) -> int {
-    const TilePlan& tp = final_pass ? tplan_final : tplan;
-    if (!use_graph) return enqueue_pass(false, tp);
+    if (!use_graph) return enqueue_pass(false, final_pass);
     cudaGraphExec_t& gx = graphs[final_pass ? 1 : 0];
     if (!gx) {
       // capture on a private stream (the context's stream may be the legacy default stream)
@@ -328,12 +369,13 @@ int db200_svm_solve_batched(db200_context* ctx, int count, const db200_svm_insta
       if (cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
         s2 = fail(ctx, DB200_ERR_CUDA, "svm_solve_batched: begin capture");
       } else {
-        s2 = enqueue_pass(false, tp);
+        s2 = enqueue_pass(false, final_pass);
         const cudaError_t e = cudaStreamEndCapture(cs, &g);
         if (!s2 && e != cudaSuccess) s2 = cuda_fail(ctx, e, "cudaStreamEndCapture");
       }
       ctx->stream = keep;
       ctx->profiling = prof;
+      graph_launches[final_pass ? 1 : 0] = (int)(ctx->launches - launches);
       ctx->launches = launches;
       if (!s2 && cudaGraphInstantiate(&gx, g, 0) != cudaSuccess)
         s2 = fail(ctx, DB200_ERR_CUDA, "svm_solve_batched: graph instantiate");
@@ -346,7 +388,7 @@ int db200_svm_solve_batched(db200_context* ctx, int count, const db200_svm_insta
     DB200_CUDA(ctx, cudaGraphLaunch(gx, cs));
     DB200_CUDA(ctx, cudaEventRecord(ev, cs));
     DB200_CUDA(ctx, cudaStreamWaitEvent(ctx->stream, ev, 0));
-    count_launch(ctx, count + 1);
+    count_launch(ctx, graph_launches[final_pass ? 1 : 0]);
     R.graph_replays += 1;
     return DB200_OK;
   };
@@ -443,7 +485,7 @@ int db200_svm_solve_batched(db200_context* ctx, int count, const db200_svm_insta
   };
   {
     Timer t(ctx->stream);
-    st = enqueue_pass(true, tplan);
+    st = enqueue_pass(true, false);
     R.kernel_passes += 1;
     if (!st) R.ms_sketch += t.stop();
   }

@@ -1,5 +1,6 @@
 // Internal host-side interfaces shared by the .cu translation units of libdarray_b200.
 #pragma once
+#include <algorithm>
 #include <cstddef>
 #include <cstdint>
 #include <functional>
@@ -176,6 +177,28 @@ int tile_split(const db200_context* ctx, int row_blocks, int n_jtiles, int unit,
                int max_ranges = 32);
 int sketch_split(const db200_context* ctx, const SketchPlan& plan, int npad_i, int npad_j, int l);
 size_t sketch_slab_floats(const SketchPlan& plan, int npad_i, int npad_j, int l, int split_tiles);
+// Work items of a launch in units of one tile's time, and the time they are expected to take on the CTA pairs.
+struct TileLoad {
+  double sum = 0.0;
+  int longest = 0;
+  void add(double items, int tiles) {
+    sum += items * tiles;
+    longest = std::max(longest, tiles);
+  }
+  void add(const TileLoad& o) {
+    sum += o.sum;
+    longest = std::max(longest, o.longest);
+  }
+  double time(const db200_context* ctx) const;
+};
+// One sketch's load with its row blocks whole, walking their ranges of split_tiles j tiles one after the other (a chunk
+// drained per range), and split into an item per range.
+struct SketchLoad {
+  TileLoad whole, walked, split;
+  int ranges = 1;
+};
+SketchLoad sketch_load(const SketchPlan& plan, int npad_i, int npad_j, int split_tiles);
+constexpr size_t MAX_BATCH_SLABS = (size_t)512 << 20;  // bytes of the slabs of one batched launch
 // A prepared launch: the instance table is on the device; launch_rbf_plan only launches (graph-capturable).
 struct TilePlan {
   int mode = 0, count = 0, n_items = 0, nsx = 0, nso = 0, nkc_max = 0, panel_max = 0, om_mult = 1, kblock = 0, yacc = 0;

@@ -69,7 +69,8 @@ constexpr float LOG2E = 1.4426950408889634f;
 // A sketch item's fill and drain in units of one tile's time (promoted items drain while they compute, single-product ones
 // store their whole panel at the end), and the summation of split ranges.  Fitted to 59 to 158 items of 157 to 470 tiles
 // cut into 1 to 16 ranges.
-constexpr int SKETCH_ITEM_TILES = 8, PROMOTED_ITEM_TILES = 2, SKETCH_SPLIT_TILES = 4;
+// WALKED_RANGE_TILES: the drain at the end of a range that its row block walks (2048 points, ranges of two tiles: 2.9 us).
+constexpr int SKETCH_ITEM_TILES = 8, PROMOTED_ITEM_TILES = 2, SKETCH_SPLIT_TILES = 4, WALKED_RANGE_TILES = 4;
 
 // One instance of the tile engine.  A launch walks a work list over a table of instances in global memory (one
 // instance for the single-problem entry points, many for the batched one); work item k belongs to the instance
@@ -1365,8 +1366,10 @@ int prepare_rbf_tiles(db200_context* ctx, int mode, const TileJob* jobs, int cou
   T.nso = (mode == RBF_MODE_SKETCH) ? MAX_NSO : 0;
   T.lean = (mode == RBF_MODE_SKETCH);
   int chunk = 0;  // shortest promoted chunk
+  bool compensated = false;
   for (int b = 0; b < count; ++b) {
     const int p = host[(size_t)b].promote;
+    compensated = compensated || host[(size_t)b].comp > 0;
     if (p > 0) chunk = chunk > 0 ? std::min(chunk, p) : p;
   }
   for (int b = 0; b < count; ++b) T.lean = T.lean && host[(size_t)b].comp == 0 && host[(size_t)b].promote == 0;
@@ -1375,14 +1378,15 @@ int prepare_rbf_tiles(db200_context* ctx, int mode, const TileJob* jobs, int cou
   // Promoted chunks are summed in shared memory where the panel's sums leave room for the rings: two Omega stages and 3
   // Xj stages for chunks of two tiles (256 points; 40000 x 40000, d = 128, l = 528: 10.0 -> 8.9 ms; l = 256, five stages:
   // 5.9 -> 4.4 ms), 6 for longer ones, which drain seldom and need their rings more (with 3 stages 6.9 -> 7.7 ms).  The
-  // Xj ring takes whatever is left.
+  // Xj ring takes whatever is left.  Chunks of a single product are ranges that their row block walks: added into Y as the
+  // sum of their slabs would be, scaled first.
   auto ring = [&](int yacc, int nso) -> int {
     const SmemLayout L0 = make_layout(nkc_max, panel_max, 0, nso, om_mult, T.kblock, yacc);
     const long long left = (long long)SMEM_LIMIT - 1024 - (long long)L0.total;
     return left < 0 ? 0 : (int)std::min<long long>(MAX_NSX, left / XJ_CHUNK);
   };
   T.yacc = 0;
-  if (chunk > 0)
+  if (chunk > 0 && compensated)
     for (int nso = MAX_NSO; nso >= 2 && !T.yacc; --nso)
       if (ring(1, nso) >= (chunk <= 2 ? 3 : 6)) {
         T.yacc = 1;
@@ -1498,6 +1502,24 @@ int sketch_split(const db200_context* ctx, const SketchPlan& plan, int npad_i, i
   return tile_split(ctx, npad_i / PAIR_M * plan.n_panels, npad_j / BN, plan.promote ? plan.promote : 1,
                     plan.promote ? PROMOTED_ITEM_TILES : SKETCH_ITEM_TILES, SKETCH_SPLIT_TILES,
                     (int)std::max(1LL, std::min(32LL, most)));
+}
+
+// A launch cannot end before its longest item, and on average half of one is left over when the others have ended.
+double TileLoad::time(const db200_context* ctx) const {
+  return std::max<double>(longest, sum / std::max(1, ctx->num_sms / 2) + 0.5 * longest);
+}
+
+SketchLoad sketch_load(const SketchPlan& plan, int npad_i, int npad_j, int split_tiles) {
+  const int items = npad_i / PAIR_M * plan.n_panels, tiles = npad_j / BN;
+  const int ranges = (tiles + split_tiles - 1) / split_tiles;
+  SketchLoad L;
+  L.ranges = ranges;
+  L.whole.add(items, tiles + (plan.promote ? PROMOTED_ITEM_TILES : SKETCH_ITEM_TILES));
+  L.walked.add(items, tiles + PROMOTED_ITEM_TILES + WALKED_RANGE_TILES * ranges);
+  L.split.add((double)items * ranges, std::min(split_tiles, tiles) +
+                                          (plan.promote ? PROMOTED_ITEM_TILES : SKETCH_ITEM_TILES));
+  if (ranges > 1) L.split.sum += SKETCH_SPLIT_TILES * (double)items;
+  return L;
 }
 
 size_t sketch_slab_floats(const SketchPlan& plan, int npad_i, int npad_j, int l, int split_tiles) {
