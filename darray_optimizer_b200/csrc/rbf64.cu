@@ -278,12 +278,14 @@ static int r64_tile_cols(int l, int dp) {
   return 264;
 }
 
-// Ranges of j: the least waves x (stages of a range + 8, a CTA's start and end in stages), at least 16 stages each; cut
-// only where that is below 0.9 of the whole, for the slabs' sum.  4096 x 4096, d = 32, l = 138 (64 row blocks): whole,
-// one CTA an SM, 679 us; in 4 ranges, two CTAs an SM, 282.
-static int r64_splits(const db200_context* ctx, int blocks, int per_sm, int n_stages) {
+// Ranges of j: the least waves x (stages of a range + 8, a CTA's start and end in stages), at least 16 stages each and
+// slabs of at most 128 MB (thousands of row blocks gain a part of one wave by them); cut only where that is below 0.9 of
+// the whole, for the slabs' sum.  4096 x 4096, d = 32, l = 138 (64 row blocks): whole, one CTA an SM, 679 us; in 4 ranges,
+// two CTAs an SM, 282.
+static int r64_splits(const db200_context* ctx, int blocks, int per_sm, int n_stages, size_t slab_doubles) {
   const long long slots = (long long)ctx->num_sms * per_sm;
-  const int most = std::max(1, std::min(32, n_stages / 16));
+  const int room = (int)std::min<size_t>(32, ((size_t)128 << 20) / (8 * slab_doubles));
+  const int most = std::max(1, std::min(room, n_stages / 16));
   auto cost = [&](int s) { return ((blocks * (long long)s + slots - 1) / slots) * ((n_stages + s - 1) / s + 8); };
   int best = 1;
   for (int s = 2; s <= most; ++s)
@@ -304,17 +306,25 @@ int rbf_sketch_f64_fused(db200_context* ctx, int m, int n, int d, int l, const f
   if (smem > R64_SMEM_MAX) return fail(ctx, DB200_ERR_UNSUPPORTED, "rbf_sketch_f64: d too large for the FP64 tile");
   const int blocks = ((m + R64_ROWS - 1) / R64_ROWS) * n_lt;
   const int per_sm = lt <= 144 && 2 * (smem + 1024) <= 228 * 1024 ? 2 : 1;
-  const int ranges = r64_splits(ctx, blocks, per_sm, n_stages);
-  const size_t slab_doubles = ranges > 1 ? (size_t)ranges * l * m : 0;
-  const size_t bytes = 1024 + align_up(slab_doubles * 8, 256) + align_up((size_t)m * 8, 256) + align_up((size_t)n_stages * R64_KS * 8, 256) +
-                       align_up((size_t)n_stages * lpad * R64_KS * 8, 256) + 1024;
-  char* base = static_cast<char*>(slot_buffer(ctx, SLOT_SPARE, bytes));
+  int ranges = r64_splits(ctx, blocks, per_sm, n_stages, (size_t)l * m);
+  auto scratch = [&]() -> char* {
+    return static_cast<char*>(slot_buffer(
+        ctx, SLOT_SPARE, 2048 + align_up(ranges > 1 ? (size_t)ranges * l * m * 8 : 0, 256) + align_up((size_t)m * 8, 256) +
+                             align_up((size_t)n_stages * R64_KS * 8, 256) +
+                             align_up((size_t)n_stages * lpad * R64_KS * 8, 256)));
+  };
+  char* base = scratch();
+  if (!base && ranges > 1) {  // no room for the slabs
+    cudaGetLastError();
+    ranges = 1;
+    base = scratch();
+  }
   if (!base) return DB200_ERR_NOMEM;
   Carve cv{base};
   double* si = cv.take<double>(m);
   double* sj = cv.take<double>((size_t)n_stages * R64_KS);
   double* Ob = cv.take<double>((size_t)n_stages * lpad * R64_KS);
-  double* slabs = slab_doubles ? cv.take<double>(slab_doubles) : nullptr;
+  double* slabs = ranges > 1 ? cv.take<double>((size_t)ranges * l * m) : nullptr;
   DB200_CUDA(ctx, cudaMemsetAsync(sj, 0, sizeof(double) * (size_t)n_stages * R64_KS, ctx->stream));
   int st = rownorm_f64(ctx, Xi, ldxi, m, d, si);
   if (!st) st = rownorm_f64(ctx, Xj, ldxj, n, d, sj);
