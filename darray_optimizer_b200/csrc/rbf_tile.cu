@@ -944,11 +944,16 @@ __global__ void __launch_bounds__(256) sum_slabs_kernel(const TileInst* __restri
 // ------------------------------------------------------------------ packing kernels
 // Largest |x| of `rows` rows of `cols` contiguous floats, ld apart (non-negative floats order like their bit
 // patterns): block maxima, then one atomicMax per block into *out, which the caller zeroes first.  A set without gaps
-// is passed as one row; otherwise a warp walks a row.  vec: 16-byte loads (aligned base, and ld when rows > 1).  Bound
-// by reading the set once (131072 x 128: 67 MB, 19 us; with a 64-bit division per element it took 87 us).
+// is passed as one row; otherwise a warp walks rows, cut into pieces by blockIdx.y (feature-major sets have few rows, and long
+// ones: 131072 x 8 with gaps took a warp each, 60 us, and 180 unaligned).  vec: 16-byte loads (aligned base, and ld when
+// rows > 1).  Bound by reading the set once (131072 x 128: 67 MB, 19 us; with a 64-bit division per element 87 us).
 // A single CTA stores the maximum and clears out[1..4) itself.
+constexpr int ABSMAX_PIECE = 1024;
 __global__ void __launch_bounds__(1024) absmax_points_kernel(const float* __restrict__ X, long long rows, long long cols,
-                                                            long long ld, int vec, unsigned* __restrict__ out) {
+                                                            long long ld, long long piece, int vec,
+                                                            unsigned* __restrict__ out) {
+  X += blockIdx.y * piece;
+  cols = min(piece, cols - blockIdx.y * piece);
   float mx = 0.f;
   auto take = [&](float x) {
     const float a = fabsf(x);
@@ -968,6 +973,7 @@ __global__ void __launch_bounds__(1024) absmax_points_kernel(const float* __rest
       take(v.z);
       take(v.w);
     }
+#pragma unroll 8
     for (long long c = 4 * c4 + lane; c < cols; c += step) take(__ldg(row + c));
   }
 #pragma unroll
@@ -979,7 +985,7 @@ __global__ void __launch_bounds__(1024) absmax_points_kernel(const float* __rest
   mx = threadIdx.x < blockDim.x / 32 ? wmax[threadIdx.x] : 0.f;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-  if (gridDim.x == 1) {
+  if (gridDim.x * gridDim.y == 1) {
     if (threadIdx.x < 4) out[threadIdx.x] = threadIdx.x == 0 ? __float_as_uint(mx) : 0u;
   } else if (threadIdx.x == 0) {
     atomicMax(out, __float_as_uint(mx));
@@ -1225,9 +1231,13 @@ int pack_points(db200_context* ctx, const float* X, int ldx, int layout, int n, 
   if (!one) DB200_CUDA(ctx, cudaMemsetAsync(mx, 0, 4 * sizeof(unsigned), ctx->stream));
   if (n > 0) {
     const bool vec = aligned && (rows == 1 || ldx % 4 == 0);
+    // (65535 pieces at most; a multiple of four keeps their alignment)
+    const long long piece = rows == 1 ? cols : std::max<long long>(one ? cols : ABSMAX_PIECE, (cols + 65534) / 65535 * 4);
+    const long long pieces = (cols + piece - 1) / piece;
     const long long work = rows == 1 ? (cols + 4095) / 4096 : (rows + 7) / 8;  // 16 elements a thread, a row a warp
-    const unsigned blocks = one ? 1u : (unsigned)std::max(1LL, std::min(work, 8LL * ctx->num_sms));
-    absmax_points_kernel<<<blocks, one ? 1024 : 256, 0, ctx->stream>>>(X, rows, cols, ldx, vec ? 1 : 0, mx);
+    const long long blocks = one ? 1 : std::max(1LL, std::min(work, 8LL * ctx->num_sms / pieces));
+    absmax_points_kernel<<<dim3((unsigned)blocks, (unsigned)pieces), one ? 1024 : 256, 0, ctx->stream>>>(
+        X, rows, cols, ldx, piece, vec ? 1 : 0, mx);
     DB200_CUDA(ctx, cudaGetLastError());
     count_launch(ctx);
   }
