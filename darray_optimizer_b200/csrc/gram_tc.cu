@@ -21,10 +21,13 @@
 // The result differs from the exact Z~^T Z~ by the dropped groups and the truncation only, about 2e-8, 3e-10,
 // 3e-12, 3e-14 of ||Z~_p|| ||Z~_q|| for KS = 5, 6, 7, 8 (measured), next to FP64 accumulation's ~1e-16 sqrt(n).
 //
-// BITS = 8 (the barrier's and CholeskyQR2's form): seven base-256 digits in [-128, 127] of round(x 2^54), x as above.
-// They carry 54 bits in 7 slices and 28 products instead of 56 bits in 8 slices and 36 products, rounded instead of
-// truncated, and the kept groups end 2^-56 below the first (2^-49 at base 128), so the error is near the FP64 Gram's
-// (4e-16 to 2e-15 where 8 base-128 digits give 3e-15 to 1.5e-14).  The digits of an integer v are the bytes of
+// BITS = 8 (the barrier's and CholeskyQR2's form): seven base-256 digits in [-128, 127] of round(x 2^55), x as above (of
+// round(x 2^54), e one larger, where the chunk's largest |x| is above 0.996 and its digits would not fit).  They hold an
+// entry to 2^-56 of 2^e, as 8 truncated base-128 digits do, in 7 slices and 28 products instead of 36, and what the dropped
+// groups can add up to is less: 6 x 128^2 x 2^-70 a row against 7 x 127^2 x 2^-70.  Mean error against 64-bit sums, in
+// ||Z~_p|| ||Z~_q||, this form and 8 base-128 digits (4096 rows, restated on the CPU): Gaussian columns 6e-18 and 1.4e-17,
+// the diagonal 3e-18 and 4e-16, entries over six decades 5e-17 and 8e-17, over eighteen 4e-17 and 8e-17, a spike on a
+// column of 1e-6 of it 1.3e-15 and 2.1e-15 (with 54 bits 2e-16, 2e-16 and 5e-15 in these three).  The digits of an integer v are the bytes of
 // v + 128 (256^7 - 1) / 255, each less 128: one addition instead of eight shifts and masks.  The s32 sums stay exact:
 // 7 * 16384 * 128^2 < 2^31.  The
 // kernels are instantiated for each KS; the barrier solver
@@ -213,7 +216,7 @@ __global__ void __launch_bounds__(THREADS, 1)
           for (int e = 0; e < 16; ++e) {
             const int col = tj * TN + c0 + e;
             if (col < g.r && row <= col)
-              atomicAdd(g.M + (long long)col * g.ldm + row, ldexp(v[e], ep + ex[col] - (BITS == 7 ? 14 : 12)));
+              atomicAdd(g.M + (long long)col * g.ldm + row, ldexp(v[e], ep + ex[col] - 14));
           }
         }
       }
@@ -257,6 +260,7 @@ __device__ __forceinline__ double chunk_max(double m, double* part, double* cta_
 // neighbouring rows, whose bytes of one slice are one word: no staging, every warp store one whole line.  Columns past r
 // are not written: the tensor maps end at r and their loads read zeros there.  131072 x 528: 214 us; the base-128
 // form, with its digits' shifts and masks and the padding columns, takes 395.
+constexpr double SLICE256_MAX = (double)0x7f7f7f7f7f7f70ll;  // largest double within seven digits of 127
 template <bool VEC>
 __global__ void __cluster_dims__(1, SLICE_CTAS, 1) __launch_bounds__(256)
     slice256_kernel(const double* __restrict__ Z, long long ldz, const double* __restrict__ sw, int n, int r, int npad,
@@ -288,9 +292,10 @@ __global__ void __cluster_dims__(1, SLICE_CTAS, 1) __launch_bounds__(256)
 #pragma unroll
   for (int j = 0; j < 4 * ROUNDS; ++j) m = fmax(m, fabs(v[j]));
   m = chunk_max(m, part, &cta_max);
-  const int e = exp_above(m);
+  int e = exp_above(m);
+  if (ldexp(m, 55 - e) > SLICE256_MAX) ++e;
   if (rank == 0 && threadIdx.x == 0) exps[(size_t)c * rpad + p] = e;
-  const double scale = ldexp(1.0, 54 - e);
+  const double scale = ldexp(1.0, 55 - e);
   const size_t slice_bytes = (size_t)r * npad;
 #pragma unroll
   for (int q = 0; q < ROUNDS; ++q) {

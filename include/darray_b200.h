@@ -78,6 +78,11 @@ DB200_API int db200_selftest_wait_timeout(db200_context* ctx, int limit_ms);
  * returns DB200_ERR_TIMEOUT and clears it. */
 DB200_API int db200_selftest_grid_barrier_timeout(db200_context* ctx, int limit_ms);
 
+/* Test hook: db200_gram_weighted in the form the mixed solves use (seven base-256 int8 digits per value).  Stream-
+ * ordered. */
+DB200_API int db200_selftest_solver_gram(db200_context* ctx, int n, int r, const double* Z, int ldz, const double* w,
+                                         double* M, int ldm);
+
 /* Enable (1) or disable (0) CUDA-event timing of every tcgen05 tile-kernel launch on the context's stream;
  * db200_profile_read() returns the summed kernel time (ms) and the number of timed launches since the last
  * read, then clears them.  Both synchronize the stream. */
