@@ -203,6 +203,7 @@ int db200_gram_weighted(db200_context* ctx, int n, int r, const double* Z, int l
   if (!ctx) return DB200_ERR_INVALID;
   if (n < 1 || r < 1 || !Z || ldz < n || !M || ldm < r) return fail(ctx, DB200_ERR_INVALID, "gram_weighted: bad arguments");
   if (!use_tensor_cores) return gram<double, double>(ctx, n, r, r, Z, ldz, Z, ldz, w, 1.0, 0.0, M, ldm, true);
+  if (use_tensor_cores > 8) return fail(ctx, DB200_ERR_INVALID, "gram_weighted: slices must be 5..8");
   void* scratch = slot_buffer(ctx, SLOT_SPARE, gram_tc_scratch_bytes(n, r));
   if (!scratch) return DB200_ERR_NOMEM;
   DB200_CUDA(ctx, cudaMemset2DAsync(M, sizeof(double) * ldm, 0, sizeof(double) * r, r, ctx->stream));

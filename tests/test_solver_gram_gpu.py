@@ -7,6 +7,8 @@ dropped digit groups add up to less than 6.1 x 2^-56 2^(e_p + e_q) a row, and th
 import numpy as np
 import pytest
 
+from darray_optimizer_b200._lib import DB200Error
+
 pytestmark = pytest.mark.gpu
 U = 2.0 ** -53
 CHUNK = 16384
@@ -74,3 +76,9 @@ def test_no_further_off_than_eight_base128_digits(gpu_ctx, kind):
     up = np.triu(np.ones((r, r), bool), 1)  # the truncated digits' bias adds up on the diagonal: compare beside it
     rms = [np.sqrt(np.mean(((grams(gpu_ctx, Z, w, 1, k) - ref).astype(float) / s[:, None] / s)[up] ** 2)) for k in (None, 8)]
     assert rms[0] <= rms[1]
+
+
+@pytest.mark.parametrize("slices", [9, 255, 256])
+def test_unknown_slice_counts_are_refused(gpu_ctx, slices):
+    with pytest.raises(DB200Error):
+        grams(gpu_ctx, np.ones((64, 2)), None, 0, slices)
