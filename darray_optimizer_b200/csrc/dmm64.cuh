@@ -35,8 +35,9 @@ constexpr int DMM_THREADS = 256;
 constexpr int DMM_BM = 128;     // rows of C per CTA (8 warps x 16)
 constexpr int DMM_KS = 32;      // k per stage
 constexpr int DMM_STAGES = 2;
+static_assert(DMM_BM % DMM_KS == 0, "tri_a starts a tile's reduction at its first row");
 
-enum DmmEpi { DMM_STORE = 0, DMM_ADD = 1, DMM_ATOMIC = 2, DMM_RBF = 3 };
+enum DmmEpi { DMM_STORE = 0, DMM_ADD = 1, DMM_ATOMIC = 2, DMM_RBF = 3, DMM_FROM = 4 };
 
 struct DmmArgs {
   int m = 0, q = 0, p = 0;
@@ -52,11 +53,15 @@ struct DmmArgs {
   int kps = 0;                // reduction length of one split (grid.y), a multiple of DMM_KS
   int upper = 0;              // only C(i, j) with i <= j
   int tri = kFullB;            // kUpperB: op(B)(k, j) = 0 for k > j; kLowerB: for k < j
+  int tri_a = 0;               // op(A)(i, k) = 0 for k < i
   int epi = DMM_STORE;
   // batches along grid.z (the block pairs of a triangular inverse of order bl, halves of bs): the z-th pair's second
   // half has min(bs, bl - (2 z + 1) bs) rows, which replaces m and p (vary = 1) or q (vary = 2)
   long long sA = 0, sB = 0, sC = 0;
   int vary = 0, bl = 0, bs = 0;
+  // DMM_FROM: C = S + alpha op(A) op(B), S FP64 (null: the identity)
+  const double* S = nullptr;
+  long long lds = 0;
   // DMM_RBF: C(i, j) = yi_i yj_j exp(-gamma max(si_i + sj_j - 2 G, 0))
   const double* si = nullptr;
   const double* sj = nullptr;
@@ -186,6 +191,7 @@ __global__ void __launch_bounds__(DMM_THREADS, 2) dmm_kernel(const DmmArgs g) {
   int kb = blockIdx.y * g.kps, ke = min(p, kb + g.kps);
   if (g.tri == kUpperB) ke = min(ke, j0 + BN);
   if (g.tri == kLowerB) kb = max(kb, j0 / DMM_KS * DMM_KS);
+  if (g.tri_a) kb = max(kb, i0);
   const int nst = ke > kb ? (ke - kb + DMM_KS - 1) / DMM_KS : 0;
 
   const int lane = threadIdx.x % 32, warp = threadIdx.x / 32;
@@ -270,6 +276,9 @@ __global__ void __launch_bounds__(DMM_THREADS, 2) dmm_kernel(const DmmArgs g) {
           if constexpr (sizeof(TC) == 8) atomicAdd(dst, (TC)(g.alpha * v));
         } else if (g.epi == DMM_ADD) {
           *dst = (TC)((double)*dst + g.alpha * v);
+        } else if (g.epi == DMM_FROM) {
+          const double s = g.S ? g.S[(long long)j * g.lds + i] : (i == j ? 1.0 : 0.0);
+          *dst = (TC)(s + g.alpha * v);
         } else {
           double x = g.alpha * v;
           if (g.beta != 0.0) x += g.beta * (double)*dst;

@@ -115,6 +115,15 @@ __global__ void zero_lower_kernel(double* A, int lda, int l) {
   }
 }
 
+// U <- the upper triangle of R, zeros below.
+__global__ void copy_upper_kernel(const double* R, int ldr, int l, double* U, int ldu) {
+  const long long total = (long long)l * l;
+  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total; e += (long long)gridDim.x * blockDim.x) {
+    const int i = (int)(e % l), j = (int)(e / l);
+    U[(long long)j * ldu + i] = i <= j ? R[(long long)j * ldr + i] : 0.0;
+  }
+}
+
 // Diagonal blocks of X = R^-1 (upper triangular, l x l): one warp per 32 x 32 block, lane j holding column j of the
 // block's inverse in registers (column-oriented back substitution; R's columns are read from shared memory as
 // broadcasts).  Rows and columns past l behave as identity and are not stored.
@@ -150,7 +159,7 @@ __global__ void __launch_bounds__(32 * TI_WARPS) trinv_diag_kernel(const double*
   }
 }
 
-// Clears the rows below the diagonal of every block pair (blockIdx.y) of trinv_upper's level h.
+// Clears the rows below the diagonal of every block pair (blockIdx.y) of trinv_doubling's level h.
 __global__ void trinv_clear_kernel(double* X, int ldx, int l, int h) {
   const int r0 = 2 * h * (int)blockIdx.y, q = min(h, l - r0 - h);
   for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < q * h; e += gridDim.x * blockDim.x)
@@ -658,13 +667,11 @@ int potrf_upper(db200_context* ctx, double* A, int lda, int l, int* d_status, in
   return DB200_OK;
 }
 
-// X = R^-1 by block doubling: the 32 x 32 diagonal blocks, then for half = 32, 64, 128, ... every pair of inverted
-// blocks X11, X22 (the second one possibly shorter) becomes one with X12 = -X11 R12 X22, two batched products per
+// X = R^-1 by block doubling: the 32 x 32 diagonal blocks by substitution, then for half = 32, 64, 128, ... every pair of
+// inverted blocks X11, X22 (the second one possibly shorter) becomes one with X12 = -X11 R12 X22, two batched products per
 // level on the FP64 tensor cores.  The first product is kept transposed, T^T = (R12 X22)^T, in the pair's place
-// below the diagonal (q x half, exactly its shape), cleared before the next level reads the blocks.  One warp per column doing its own
-// back substitution over global memory (the form before) took 1.01 ms at l = 528 and 3.4 ms at l = 1024, a chain of l
-// dependent memory round trips; the levels are log2(l / 32) pairs of launches.
-int trinv_upper(db200_context* ctx, const double* R, int ldr, int l, double* X, int ldx) {
+// below the diagonal (q x half, exactly its shape), cleared before the next level reads the blocks.
+static int trinv_doubling(db200_context* ctx, const double* R, int ldr, int l, double* X, int ldx) {
   trinv_diag_kernel<<<(l + TI * TI_WARPS - 1) / (TI * TI_WARPS), 32 * TI_WARPS, 0, ctx->stream>>>(R, ldr, l, X, ldx);
   DB200_CUDA(ctx, cudaGetLastError());
   count_launch(ctx);
@@ -705,6 +712,48 @@ int trinv_upper(db200_context* ctx, const double* R, int ldr, int l, double* X, 
     DB200_CUDA(ctx, cudaGetLastError());
     count_launch(ctx);
   }
+  return DB200_OK;
+}
+
+// X = R^-1: the inverse X0 by block doubling and one correction, X = X0 + X0 (I - R X0).  The doubling's right residual
+// R X - I grows at every level by that of X11: 4 to 8 times column substitution's for factors of condition 1e4 to 1e8, and
+// 2e-7 against 1e-12 for the factor of an RBF kernel of 528 sorted points + 1e-7 I (against |R| |X| 2e-10 and 2e-16).  The
+// correction brings it to substitution's (2e-16; a correction of every level's X12 does no better and takes five times
+// the launches).  Bound by the launches' latency and the longest tile's reduction: db200_trsm_lutn of one column takes
+// 266 us at l = 528 and 341 at l = 1024, of which the correction 62 and 112.  One warp per column doing its own back
+// substitution over global memory, a chain of l dependent memory round trips, took 1.01 and 3.4 ms for the inverse alone.
+int trinv_upper(db200_context* ctx, const double* R, int ldr, int l, double* X, int ldx, double* X0, double* D) {
+  int st = trinv_doubling(ctx, R, ldr, l, X0, l);
+  if (st) return st;
+  // D = I - R X0 and X = X0 + X0 D, zeros below the diagonal included
+  DmmArgs g;
+  g.m = g.q = g.p = l;
+  g.tri = kUpperB;
+  g.tri_a = 1;
+  g.epi = DMM_FROM;
+  g.A = R;
+  g.lda = ldr;
+  g.B = X0;
+  g.ldb = l;
+  g.alpha = -1.0;
+  g.C = D;
+  g.ldc = l;
+  if ((st = dmm_launch<double, double, double, false, true>(ctx, g))) return st;
+  g.A = X0;
+  g.lda = l;
+  g.B = D;
+  g.alpha = 1.0;
+  g.S = X0;
+  g.lds = l;
+  g.C = X;
+  g.ldc = ldx;
+  return dmm_launch<double, double, double, false, true>(ctx, g);
+}
+
+int copy_upper(db200_context* ctx, const double* R, int ldr, int l, double* U, int ldu) {
+  copy_upper_kernel<<<grid_for((long long)l * l, 256, 1024), 256, 0, ctx->stream>>>(R, ldr, l, U, ldu);
+  DB200_CUDA(ctx, cudaGetLastError());
+  count_launch(ctx);
   return DB200_OK;
 }
 

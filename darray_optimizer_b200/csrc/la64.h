@@ -34,8 +34,10 @@ void potrf_cluster_init(db200_context* ctx);
 int potrf_cluster_size(const db200_context* ctx, int l);
 int potrf_cluster(db200_context* ctx, double* A, int lda, int l, int* d_status, int* d_bad, double* W = nullptr);
 
-// X = R^-1 for upper triangular R.
-int trinv_upper(db200_context* ctx, const double* R, int ldr, int l, double* X, int ldx);
+// X = R^-1 for upper triangular R with exact zeros below the diagonal; X0, D: l x l scratch.
+int trinv_upper(db200_context* ctx, const double* R, int ldr, int l, double* X, int ldx, double* X0, double* D);
+// U <- the upper triangle of R, zeros below
+int copy_upper(db200_context* ctx, const double* R, int ldr, int l, double* U, int ldu);
 
 // x <- R^-1 R^-T x (R upper, l <= 4096) with the diagonal blocks' inverses W that potrf_upper left.
 int trsv_pair(db200_context* ctx, const double* R, int ld, int l, const double* W, double* x);

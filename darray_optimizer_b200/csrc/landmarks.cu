@@ -745,13 +745,15 @@ int db200_ridge_leverage(db200_context* ctx, int n, int r, const double* Z, int 
   if (!ctx) return DB200_ERR_INVALID;
   if (n < 1 || r < 1 || ldz < n || !Z || !lev || !(lambda > 0)) return fail(ctx, DB200_ERR_INVALID, "ridge_leverage: bad arguments");
   const size_t rr = (size_t)r * r;
-  const size_t bytes = 1024 + 2 * align_up(rr * 8, 256) + align_up((size_t)n * r * 8, 256);
+  const size_t bytes = 1024 + 4 * align_up(rr * 8, 256) + align_up((size_t)n * r * 8, 256);
   char* base = static_cast<char*>(slot_buffer(ctx, SLOT_SPARE, bytes));
   if (!base) return DB200_ERR_NOMEM;
   Carve cv{base};
   int* d_pair = cv.take<int>(4);
   double* G = cv.take<double>(rr);
   double* Xi = cv.take<double>(rr);
+  double* X0 = cv.take<double>(rr);
+  double* D = cv.take<double>(rr);
   double* W = cv.take<double>((size_t)n * r);
   // (Z^T Z + lambda I) = R^T R;  lev_i = ||z_i^T R^-1||^2
   int st = gram<double, double>(ctx, n, r, r, Z, ldz, Z, ldz, nullptr, 1.0, 0.0, G, r, true);
@@ -764,7 +766,7 @@ int db200_ridge_leverage(db200_context* ctx, int n, int r, const double* Z, int 
   DB200_CUDA(ctx, cudaMemcpyAsync(hs, d_pair, 2 * sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
   DB200_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   if (hs[0]) return fail(ctx, DB200_ERR_NOT_SPD, "ridge_leverage: Z^T Z + lambda I not positive definite");
-  if ((st = trinv_upper(ctx, G, r, r, Xi, r))) return st;
+  if ((st = trinv_upper(ctx, G, r, r, Xi, r, X0, D))) return st;
   if ((st = gemm_tall<double, double>(ctx, n, r, r, Z, ldz, Xi, r, false, 0.0, W, n, 1.0, kUpperB))) return st;
   row_sumsq64_kernel<<<blocks_for(n, 256, 4096), 256, 0, ctx->stream>>>(n, r, W, n, lev);
   DB200_CUDA(ctx, cudaGetLastError());
@@ -990,7 +992,7 @@ template <typename TC>
 static int landmark_factor_impl(db200_context* ctx, int n, int d, const float* X, int ldx, const float* y,
                                 float gamma, int r, const int* idx, double* Z, int ldz, double* nu_out) {
   const size_t rr = (size_t)r * r;
-  const size_t bytes = 4096 + align_up((size_t)n * r * sizeof(TC), 256) + 3 * align_up(rr * 8, 256) +
+  const size_t bytes = 4096 + align_up((size_t)n * r * sizeof(TC), 256) + 4 * align_up(rr * 8, 256) +
                        align_up((size_t)r * d * 4, 256) + align_up((size_t)r * 4, 256);
   char* base = static_cast<char*>(slot_buffer(ctx, SLOT_PIPE, bytes));
   if (!base) return DB200_ERR_NOMEM;
@@ -1001,6 +1003,7 @@ static int landmark_factor_impl(db200_context* ctx, int n, int d, const float* X
   double* W = cv.take<double>(rr);
   double* R = cv.take<double>(rr);
   double* Xinv = cv.take<double>(rr);
+  double* D = cv.take<double>(rr);
   float* XL = cv.take<float>((size_t)r * d);
   float* yL = cv.take<float>(r);
   gather_rows_f32_kernel<<<blocks_for((long long)r * d, 256, 4096), 256, 0, ctx->stream>>>(X, ldx, idx, r, d, XL);
@@ -1037,7 +1040,7 @@ static int landmark_factor_impl(db200_context* ctx, int n, int d, const float* X
   }
   if (!ok) return fail(ctx, DB200_ERR_NOT_SPD, "landmark_factor: K(L, L) + nu I not positive definite after 12 shifts");
   // Z = C R^-1
-  if ((st = trinv_upper(ctx, R, r, r, Xinv, r))) return st;
+  if ((st = trinv_upper(ctx, R, r, r, Xinv, r, W, D))) return st;
   if ((st = gemm_tall<TC, double>(ctx, n, r, r, Cm, n, Xinv, r, false, 0.0, Z, ldz, 1.0, kUpperB))) return st;
   if (nu_out) *nu_out = nu;
   return db200_synchronize(ctx);

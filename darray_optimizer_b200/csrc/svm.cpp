@@ -76,9 +76,9 @@ int allreduce_host(db200_context* ctx, double* d_tmp, double* vals, int k, int o
 }
 
 // One CholeskyQR pass Yout = Yin R^-1 with R = chol(Yin^T Yin + shift I); returns NOT_SPD without touching Yout
-// when the Gram is not positive definite.  W, Rinv: l x l scratch; R (l x l) receives the factor.
+// when the Gram is not positive definite.  Rinv, S0, S1: l x l scratch; R (l x l) receives the factor.
 int cholqr_pass(db200_context* ctx, int n, int l, const double* Yin, int ldin, double* Yout, int ldout, double* R,
-                double* Rinv, double shift_rel, int* d_pair, double* d_scalar, bool tc_gram, bool dist) {
+                double* Rinv, double* S0, double* S1, double shift_rel, int* d_pair, double* d_scalar, bool tc_gram, bool dist) {
   // Gram W = Y^T Y (upper triangle).  tc_gram: on the int8 tensor cores, seven base-256 digits per value, exact
   // integer products, error ~1e-15 of ||y_p|| ||y_q||; otherwise on the FP64 pipes.  The Cholesky stays FP64.
   int st = DB200_OK;
@@ -106,7 +106,7 @@ int cholqr_pass(db200_context* ctx, int n, int l, const double* Yin, int ldin, d
   if ((st = read_status(ctx, d_pair, &pst, &bad))) return st;
   if (pst) return fail(ctx, DB200_ERR_NOT_SPD, "CholeskyQR: Gram matrix not positive definite at row " +
                                                    std::to_string(bad));
-  if ((st = trinv_upper(ctx, R, l, l, Rinv, l))) return st;
+  if ((st = trinv_upper(ctx, R, l, l, Rinv, l, S0, S1))) return st;
   return gemm_tall<double, double>(ctx, n, l, l, Yin, ldin, Rinv, l, false, 0.0, Yout, ldout, 1.0, kUpperB);
 }
 
@@ -132,7 +132,7 @@ int cholqr2_impl(db200_context* ctx, int n, int l, double* Y, int ldy, double* R
   double* R3 = cv.take<double>(ll);
   double* Rinv = cv.take<double>(ll);
   double* Racc = cv.take<double>(ll);
-  int st = cholqr_pass(ctx, n, l, Y, ldy, T, n, R1, Rinv, 0.0, d_pair, d_scalar, tc_gram, dist);
+  int st = cholqr_pass(ctx, n, l, Y, ldy, T, n, R1, Rinv, R3, Racc, 0.0, d_pair, d_scalar, tc_gram, dist);
   bool shifted = false;
   if (st == DB200_ERR_NOT_SPD) {
     // shifted CholeskyQR3 (Fukaya, Kannan, Nakatsukasa, Yamamoto, Yanagisawa 2020): first pass with
@@ -141,17 +141,17 @@ int cholqr2_impl(db200_context* ctx, int n, int l, double* Y, int ldy, double* R
     if (dist && (st = allreduce_host(ctx, d_scalar, &rows, 1, DB200_REDUCE_SUM))) return st;
     const double u = 1.1102230246251565e-16;
     const double rel = 11.0 * (rows * l + (double)l * (l + 1)) * u;
-    st = cholqr_pass(ctx, n, l, Y, ldy, T, n, R1, Rinv, rel, d_pair, d_scalar, tc_gram, dist);
+    st = cholqr_pass(ctx, n, l, Y, ldy, T, n, R1, Rinv, R3, Racc, rel, d_pair, d_scalar, tc_gram, dist);
     shifted = true;
   }
   if (st) return st;
   // second pass T -> Y
-  if ((st = cholqr_pass(ctx, n, l, T, n, Y, ldy, R2, Rinv, 0.0, d_pair, d_scalar, tc_gram, dist))) return st;
+  if ((st = cholqr_pass(ctx, n, l, T, n, Y, ldy, R2, Rinv, R3, Racc, 0.0, d_pair, d_scalar, tc_gram, dist))) return st;
   // R = R2 R1 (upper * upper)
   if ((st = gemm_tall<double, double>(ctx, l, l, l, R2, l, R1, l, false, 0.0, Racc, l, 1.0, kUpperB))) return st;
   if (shifted) {
     // third pass Y -> T, then copy back; R = R3 (R2 R1)
-    if ((st = cholqr_pass(ctx, n, l, Y, ldy, T, n, R3, Rinv, 0.0, d_pair, d_scalar, tc_gram, dist))) return st;
+    if ((st = cholqr_pass(ctx, n, l, Y, ldy, T, n, R3, Rinv, R1, R2, 0.0, d_pair, d_scalar, tc_gram, dist))) return st;
     DB200_CUDA(ctx, cudaMemcpy2DAsync(Y, sizeof(double) * ldy, T, sizeof(double) * n, sizeof(double) * n, l,
                                       cudaMemcpyDeviceToDevice, ctx->stream));
     if ((st = gemm_tall<double, double>(ctx, l, l, l, R3, l, Racc, l, false, 0.0, R1, l, 1.0, kUpperB))) return st;
@@ -881,14 +881,19 @@ int db200_trsm_lutn(db200_context* ctx, int m, int n, const double* R, int ldr, 
   if (!ctx) return DB200_ERR_INVALID;
   if (m < 0 || n < 0 || !R || !B || ldr < m || ldb < m) return fail(ctx, DB200_ERR_INVALID, "trsm: bad arguments");
   if (m == 0 || n == 0) return DB200_OK;
-  // B <- (R^-1)^T B:  X = R^-1 (triangular inverse), then B = X^T B through the Gram kernel into scratch
-  const size_t bytes = 1024 + align_up((size_t)m * m * 8, 256) + align_up((size_t)m * n * 8, 256);
+  // B <- (R^-1)^T B:  X = R^-1 (triangular inverse, of a copy: what is below R's diagonal is not read), then B = X^T B
+  // through the Gram kernel into scratch
+  const size_t bytes = 1024 + 4 * align_up((size_t)m * m * 8, 256) + align_up((size_t)m * n * 8, 256);
   char* base = static_cast<char*>(slot_buffer(ctx, SLOT_SPARE, bytes));
   if (!base) return DB200_ERR_NOMEM;
   Carve cv{base};
   double* Xi = cv.take<double>((size_t)m * m);
+  double* U = cv.take<double>((size_t)m * m);
+  double* X0 = cv.take<double>((size_t)m * m);
+  double* D = cv.take<double>((size_t)m * m);
   double* T = cv.take<double>((size_t)m * n);
-  int st = trinv_upper(ctx, R, ldr, m, Xi, m);
+  int st = copy_upper(ctx, R, ldr, m, U, m);
+  if (!st) st = trinv_upper(ctx, U, m, m, Xi, m, X0, D);
   if (!st) st = gram<double, double>(ctx, m, m, n, Xi, m, B, ldb, nullptr, 1.0, 0.0, T, m, false);
   if (st) return st;
   DB200_CUDA(ctx, cudaMemcpy2DAsync(B, sizeof(double) * ldb, T, sizeof(double) * m, sizeof(double) * m, n,
