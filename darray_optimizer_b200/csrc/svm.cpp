@@ -367,7 +367,8 @@ int svm_barrier_impl(db200_context* ctx, int n, int r, const double* Z, int ldz,
   // Capacity matrix M = I + Z^T D^-1 Z of the current D and its first Cholesky attempt (status in d_pair), enqueued
   // only: the caller reads the status.
   auto factor_launch = [&](bool use_tc) -> int {
-    const FactorSeq fs{Z, ldz, dinv, M, L, W, d_pair, n, r, use_tc, kSlices[tc_level], tc_scratch};
+    const int slices = kSlices[std::min(tc_level, 1)];  // unused from level 2 on (FP64)
+    const FactorSeq fs{Z, ldz, dinv, M, L, W, d_pair, n, r, use_tc, slices, tc_scratch};
     int s2;
     if (!dist) {
       // Gram, identity, backup, first Cholesky: one graph replay per Newton step (about 17 launches as separate
