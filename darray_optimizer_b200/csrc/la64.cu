@@ -723,6 +723,7 @@ static int trinv_doubling(db200_context* ctx, const double* R, int ldr, int l, d
 // 266 us at l = 528 and 341 at l = 1024, of which the correction 62 and 112.  One warp per column doing its own back
 // substitution over global memory, a chain of l dependent memory round trips, took 1.01 and 3.4 ms for the inverse alone.
 int trinv_upper(db200_context* ctx, const double* R, int ldr, int l, double* X, int ldx, double* X0, double* D) {
+  if (l <= TI) return trinv_doubling(ctx, R, ldr, l, X, ldx);  // one block, by substitution
   int st = trinv_doubling(ctx, R, ldr, l, X0, l);
   if (st) return st;
   // D = I - R X0 and X = X0 + X0 D, zeros below the diagonal included
