@@ -968,7 +968,12 @@ __global__ void __launch_bounds__(1024) absmax_points_kernel(const float* __rest
   const long long r0 = rows == 1 ? 0 : (long long)blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
   for (long long r = r0; r < rows; r += (long long)gridDim.x * (blockDim.x / 32)) {
     const float* row = X + r * ld;
-    const long long c4 = vec ? cols / 4 : 0;
+    if (!vec) {
+#pragma unroll 8
+      for (long long c = lane; c < cols; c += step) take(__ldg(row + c));
+      continue;
+    }
+    const long long c4 = cols / 4;
 #pragma unroll 4
     for (long long c = lane; c < c4; c += step) {
       const float4 v = __ldg(reinterpret_cast<const float4*>(row) + c);
@@ -977,7 +982,7 @@ __global__ void __launch_bounds__(1024) absmax_points_kernel(const float* __rest
       take(v.z);
       take(v.w);
     }
-#pragma unroll 8
+#pragma unroll 1
     for (long long c = 4 * c4 + lane; c < cols; c += step) take(__ldg(row + c));
   }
 #pragma unroll
@@ -1229,9 +1234,11 @@ int pack_points(db200_context* ctx, const float* X, int ldx, int layout, int n, 
     cols *= rows;
     rows = 1;
   }
-  // mx: max |x|, scale, lo flag.  A small set takes one CTA, which clears them itself: 1024 x 32, 3.6 us; eight CTAs 2.3
-  // behind a clear of 1.0 and its gap of 2 (the whole sketch of 64 columns 28.9 and 30.6 us).
-  const bool one = n > 0 && rows <= 256 && rows * cols <= 32768;
+  // mx: max |x|, scale, lo flag.  A small set takes one CTA, which clears them itself, without a clear and its gap before
+  // several CTAs.  A sketch of 16 columns, one CTA and several, us: 2048 values 23.6 and 25.6, 32768 27.3 and 28.6, 49152
+  // 28.5 and 29.1, 65536 to 98304 the same, 131072 31.5 to 38 and 29.7.  Rows with gaps take a warp each, so one CTA has
+  // fewer loads in flight: 64 rows of 128 23.6 and 24.9, 128 rows 25.7 both, 256 rows of 64 27.3 and 25.6.
+  const bool one = n > 0 && (rows == 1 ? cols <= 32768 : rows <= 64 && rows * cols <= 32768);
   if (!one) DB200_CUDA(ctx, cudaMemsetAsync(mx, 0, 4 * sizeof(unsigned), ctx->stream));
   if (n > 0) {
     const bool vec = aligned && (rows == 1 || ldx % 4 == 0);
