@@ -114,10 +114,10 @@ static __device__ __noinline__ bool p64_factor16(P64Smem& S, double* Rb, double*
   return true;
 }
 
-// The four steps for this warp's column group (0..3: the block's own columns; above: block row; group < 0: none) held
-// in acc.  Every thread of the CTA calls it.  Returns false, in every thread, when a pivot fails (S.fail says where).
+// The steps over the block's kb columns for this warp's column group (0..3: the block's own columns; above: block row;
+// group < 0: none) held in acc.  Every thread of the CTA calls it.  Returns false, in every thread, when a pivot fails (S.fail says where).
 // On return acc holds the group's rows of R (own columns: rows of the earlier groups; the block itself is in S.R).
-__device__ __forceinline__ bool p64_run(P64Smem& S, double (&acc)[8][4], int group) {
+__device__ __forceinline__ bool p64_run(P64Smem& S, double (&acc)[8][4], int group, int kb) {
   const int lane = threadIdx.x % 32, g = lane / 4, t = lane % 4;
   if (threadIdx.x == 0) S.fail = 0;
 #pragma unroll
@@ -163,7 +163,7 @@ __device__ __forceinline__ bool p64_run(P64Smem& S, double (&acc)[8][4], int gro
                 make_double2(x[n][2 * h], x[n][2 * h + 1]);
       }
     }
-    if (p == 3) break;
+    if (p == 3 || 16 * (p + 1) >= kb) break;  // no columns left: what follows is the padding's identity
     __syncthreads();
     if (group > p) {
 #pragma unroll

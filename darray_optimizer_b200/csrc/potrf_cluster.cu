@@ -97,7 +97,7 @@ __global__ void __launch_bounds__(P64_THREADS, 1) potrf_cluster_kernel(double* A
       cl = l;
     }
     if (group >= 0) p64_load<VEC>(acc, A, lda, c0, kb, col, cl, warp < 4 ? warp : -1);
-    if (!p64_run(S, acc, group)) {
+    if (!p64_run(S, acc, group, kb)) {
       if (c == 0 && tid == 0 && atomicCAS(status, 0, DB200_ERR_NOT_SPD) == 0) *bad = (c0 + S.fail - 1) / 32 * 32;
       return;
     }
