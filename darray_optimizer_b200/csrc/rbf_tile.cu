@@ -914,34 +914,42 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) rbf_tile_kernel(const __grid_c
   if (warp == 1) tmem_dealloc_pair(tmem_base, TMEM_COLS);
 }
 
-// Y(i, c) = the sum over the ranges of the j tiles, in their order, of the partial sums in the slabs, for every instance
-// that has several (those of one range wrote Y themselves), in pieces of 256 rows of a column.  GRID: a CTA per piece of
-// the largest instance and instance (blockIdx.z), for few instances of like size.  Otherwise the CTAs walk one list of all
-// instances' pieces: that grid was 4 million CTAs, almost all empty, for a batch of 64 (10 ms of a pass of 110).
-template <bool GRID>
-__global__ void __launch_bounds__(256) sum_slabs_kernel(const TileInst* __restrict__ inst, int count) {
-  int u = blockIdx.x;  // !GRID: this CTA's next piece, counted from the instance's first (slabs: fewer than 2^31 bytes)
-  for (int b = GRID ? blockIdx.z : 0; b < (GRID ? (int)blockIdx.z + 1 : count); ++b) {
+// Y(i, c) = the sum over the ranges of the j tiles, in their order, of the partial sums in the slabs (blockIdx.z: the
+// instance; those of one range wrote Y themselves).  For few instances of like size.
+__global__ void __launch_bounds__(256) sum_slabs_kernel(const TileInst* __restrict__ inst) {
+  const TileInst* I = inst + blockIdx.z;
+  const int S = I->n_splits, i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (S <= 1 || i >= I->m) return;
+  const long long stride = I->split_stride, ldo = I->ldo, ldy = I->red_ldo;
+  for (int c = blockIdx.y; c < I->l; c += gridDim.y) {
+    const float* p = I->out + c * ldo + i;
+    float acc = p[0];
+#pragma unroll 4
+    for (int k = 1; k < S; ++k) acc += p[k * stride];
+    I->red_out[c * ldy + i] = acc;
+  }
+}
+
+// The same for a batch: the CTAs walk one list of all instances' pieces (256 rows of a column).  The grid above was 4
+// million CTAs, almost all empty, for a batch of 64 (10 ms of a pass of 110); for one instance the list takes 1 us more.
+__global__ void __launch_bounds__(256) sum_slab_list_kernel(const TileInst* __restrict__ inst, int count) {
+  int u = blockIdx.x;  // this CTA's next piece, counted from the instance's first (slabs hold fewer than 2^31 bytes)
+  for (int b = 0; b < count; ++b) {
     const TileInst* I = inst + b;
     const int S = I->n_splits, m = I->m, l = I->l;
     if (S <= 1) continue;
     const long long stride = I->split_stride, ldo = I->ldo, ldy = I->red_ldo;
-    auto piece = [&](int i, int c) {
-      if (i >= m) return;
+    const unsigned rows = (unsigned)(m + 255) / 256, pieces = rows * (unsigned)l;
+    for (; u < (int)pieces; u += gridDim.x) {
+      const int c = (int)((unsigned)u / rows), i = (int)((unsigned)u % rows) * 256 + (int)threadIdx.x;
+      if (i >= m) continue;
       const float* p = I->out + c * ldo + i;
       float acc = p[0];
 #pragma unroll 4
       for (int k = 1; k < S; ++k) acc += p[k * stride];
       I->red_out[c * ldy + i] = acc;
-    };
-    if (GRID) {
-      for (int c = blockIdx.y; c < l; c += gridDim.y) piece(blockIdx.x * 256 + threadIdx.x, c);
-    } else {
-      const unsigned rows = (unsigned)(m + 255) / 256, pieces = rows * (unsigned)l;
-      for (; u < (int)pieces; u += gridDim.x)
-        piece((int)((unsigned)u % rows) * 256 + (int)threadIdx.x, (int)((unsigned)u / rows));
-      u -= (int)pieces;
     }
+    u -= (int)pieces;
   }
 }
 
@@ -1479,8 +1487,8 @@ int launch_rbf_plan(db200_context* ctx, const TilePlan& T) {
   count_launch(ctx);
   if (T.sum_list > 0 || T.sum_grid.z > 0) {
     const TileInst* inst = static_cast<const TileInst*>(T.table);
-    if (T.sum_list > 0) sum_slabs_kernel<false><<<T.sum_list, 256, 0, ctx->stream>>>(inst, T.count);
-    else sum_slabs_kernel<true><<<T.sum_grid, 256, 0, ctx->stream>>>(inst, T.count);
+    if (T.sum_list > 0) sum_slab_list_kernel<<<T.sum_list, 256, 0, ctx->stream>>>(inst, T.count);
+    else sum_slabs_kernel<<<T.sum_grid, 256, 0, ctx->stream>>>(inst);
     DB200_CUDA(ctx, cudaGetLastError());
     count_launch(ctx);
   }
