@@ -51,7 +51,7 @@ __global__ void __launch_bounds__(P64_THREADS) potrf_block_kernel(double* A, int
     __threadfence();
   }
   if (*(volatile int*)status) return;  // an earlier block column failed (checked after counting in)
-  const bool ok = p64_run(S, acc, group, kb);
+  const bool ok = p64_run(S, acc, group, P64_NB);  // (a constant: a bound here costs each of many full blocks 0.4 us)
   const bool writer = S.flag != 0;  // visible: p64_run passed a barrier
   if (!ok) {
     if (writer && t == 0 && atomicCAS(status, 0, DB200_ERR_NOT_SPD) == 0) *bad = k0;
