@@ -72,6 +72,14 @@ SketchPlan comp_plan(const SketchPlan& p, int l) {
   return c;
 }
 
+// Ranges of the points j that a problem alone takes: those of its default plan, whatever tile plan the instance has, since
+// they fix the order of its sums.
+int single_split(db200_context* ctx, const SketchPlan& plan, int npad_i, int npad_j, int l) {
+  SketchPlan p = plan_sketch(l, plan.comp);
+  p.promote = plan.promote;
+  return sketch_split(ctx, p, npad_i, npad_j, l);
+}
+
 int pack_problem(db200_context* ctx, int m, int n, int d, const float* Xi, int ldxi, const float* Xj, int ldxj,
                  const SketchPlan& plan, Carve& cv, Packed* P) {
   const int dp = feature_pad(d), mpad = point_pad(m), npad = point_pad(n);
@@ -134,7 +142,7 @@ int db200_rbf_sketch_batched(db200_context* ctx, int count, const db200_sketch_j
     P = job_plan(J.l, J.n_panels, J.panel, J.g_bufs);
     bytes += packed_bytes(J.m, J.n, J.d, J.Xi == J.Xj && J.ldxi == J.ldxj && J.m == J.n, P);
     const int mp = point_pad(J.m), np = point_pad(J.n);
-    split[(size_t)b] = sketch_split(ctx, P, mp, np, J.l);
+    split[(size_t)b] = single_split(ctx, P, mp, np, J.l);
     slab_bytes += align_up(sketch_slab_floats(P, mp, np, J.l, split[(size_t)b]) * 4, 256);
     const SketchLoad L = sketch_load(P, mp, np, split[(size_t)b]);
     all.add(L.split);
@@ -212,11 +220,11 @@ int db200_svm_solve_batched(db200_context* ctx, int count, const db200_svm_insta
   auto pass_slab = [&](SketchPlan p, const db200_svm_instance& I, bool final_pass) -> size_t {
     if (final_pass) p.promote = 2;
     const int np = point_pad(I.n);
-    return sketch_slab_floats(p, np, np, I.l, sketch_split(ctx, p, np, np, I.l));
+    return sketch_slab_floats(p, np, np, I.l, single_split(ctx, p, np, np, I.l));
   };
   // A pass is one launch per group of instances: those without slabs and as many of the others as MAX_BATCH_SLABS holds,
   // then more of the others on the same slabs.  (Row blocks kept whole instead would need none, but another order of the
-  // fp32 sums moves a solve's objective by up to 4e-6 against the single solve's.)
+  // fp32 sums moves a solve's objective by 1.4e-7 against the single solve's, where 1e-7 is promised.)
   std::vector<int> group((size_t)count, 0);
   std::vector<size_t> slab_at((size_t)count);
   size_t slab_used = 0, slab_area = 0;
@@ -297,11 +305,11 @@ int db200_svm_solve_batched(db200_context* ctx, int count, const db200_svm_insta
     T.ldo = inst[b].n;
     const int np = T.pi.npad;
     if (slab_floats[(size_t)b])
-      T.set_split(sketch_split(ctx, T.plan, np, np, T.l), reinterpret_cast<float*>(slabs + slab_at[(size_t)b]));
+      T.set_split(single_split(ctx, T.plan, np, np, T.l), reinterpret_cast<float*>(slabs + slab_at[(size_t)b]));
     if (T.plan.comp == 2) {  // the final pass's ranges: the same slabs, multiples of its own chunks
       SketchPlan pf = T.plan;
       pf.promote = 2;
-      T.split_final = T.slab ? sketch_split(ctx, pf, np, np, T.l) : 0;
+      T.split_final = T.slab ? single_split(ctx, pf, np, np, T.l) : 0;
     }
     std::vector<TileJob>& list = tj[(size_t)group[(size_t)b]];
     if (inst[b].n_panels <= 0) exact_panel_jobs(T, list);

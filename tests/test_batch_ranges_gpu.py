@@ -97,3 +97,22 @@ def test_more_problems_than_a_grid_dimension(gpu_ctx):
     gpu_ctx.rbf_sketch(n, n, d, l, ptr(X), d, ptr(X), d, 0, None, None, ptr(Om), n, ptr(one), n, 0.5)
     gpu_ctx.sync()
     assert torch.equal(Y, one.expand(count, n))
+
+
+@pytest.mark.parametrize("plan", [(1, 272, 1), (2, 144, 2), (3, 96, 2), (6, 48, 2)])
+@pytest.mark.parametrize("n,copies", [(1500, 1), (2048, 1), (4096, 1), (2048, 24)])
+def test_explicit_plans_keep_the_ranges(gpu_ctx, n, copies, plan):
+    """An instance's tile plan (the autotuner's) does not change its ranges, so nor its bits."""
+    import torch
+    from darray_optimizer_b200._lib import SketchJob
+    d, l = 64, 272
+    g = torch.Generator(device="cuda").manual_seed(n)
+    X = torch.rand(n, d, device="cuda", generator=g)
+    Om = torch.randn(l, n, device="cuda", generator=g)
+    Y = torch.empty(copies, l, n, device="cuda")
+    gpu_ctx.rbf_sketch_batched([SketchJob(n, n, d, l, ptr(X), d, ptr(X), d, None, None, ptr(Om), n, ptr(Y[k]), n, 0.5 / d,
+                                          *plan) for k in range(copies)])
+    one = torch.empty(l, n, device="cuda")
+    gpu_ctx.rbf_sketch(n, n, d, l, ptr(X), d, ptr(X), d, 0, None, None, ptr(Om), n, ptr(one), n, 0.5 / d)
+    gpu_ctx.sync()
+    assert all(torch.equal(one, y) for y in Y)
