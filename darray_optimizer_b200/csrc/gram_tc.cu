@@ -15,7 +15,7 @@
 //     are kept (the rest lie below the truncation); all products of one group g = s + t share a scale, so each
 //     group is a single s32 accumulator in TMEM fed by tcgen05.mma kind::i8 (exact integer sums:
 //     KS * 16384 * 127^2 < 2^31).  A CTA's k range lies inside one chunk.
-//  4. The epilogue folds the groups in FP64 (Horner in 2^-7), scales by 2^(e_cp + e_cq) and adds the 128 x 64 tile
+//  4. The epilogue folds the groups in FP64 (Horner in 2^-BITS), scales by 2^(e_cp + e_cq) and adds the 128 x 64 tile
 //     into M with FP64 atomics (the n dimension is split across CTAs).
 //
 // The result differs from the exact Z~^T Z~ by the dropped groups and the truncation only, about 2e-8, 3e-10,
@@ -27,12 +27,12 @@
 // groups can add up to is less: 6 x 128^2 x 2^-70 a row against 7 x 127^2 x 2^-70.  Mean error against 64-bit sums, in
 // ||Z~_p|| ||Z~_q||, this form and 8 base-128 digits (4096 rows, restated on the CPU): Gaussian columns 6e-18 and 1.4e-17,
 // the diagonal 3e-18 and 4e-16, entries over six decades 5e-17 and 8e-17, over eighteen 4e-17 and 8e-17, a spike on a
-// column of 1e-6 of it 1.3e-15 and 2.1e-15 (with 54 bits 2e-16, 2e-16 and 5e-15 in these three).  The digits of an integer v are the bytes of
-// v + 128 (256^7 - 1) / 255, each less 128: one addition instead of eight shifts and masks.  The s32 sums stay exact:
-// 7 * 16384 * 128^2 < 2^31.  The
-// kernels are instantiated for each KS; the barrier solver
-// still refines each Newton step against the exact FP64 operator and falls back to the FP64 Gram if refinement
-// stalls.
+// column of 1e-6 of it 1.3e-15 and 2.1e-15 (with 54 bits 2e-16, 2e-16 and 5e-15 in these three).  The digits of an
+// integer v are the bytes of v + 128 (256^7 - 1) / 255, each less 128: one addition instead of eight shifts and masks.
+// The s32 sums stay exact: 7 * 16384 * 128^2 < 2^31.
+//
+// The kernels are instantiated for each KS; the barrier solver still refines each Newton step against the exact FP64
+// operator and falls back to the FP64 Gram if refinement stalls.
 #include <cuda.h>
 #include <cooperative_groups.h>
 #include <cudaTypedefs.h>
@@ -501,7 +501,8 @@ int gram_tc_run(db200_context* ctx, int n, int r, const double* Z, long long ldz
 }  // namespace
 
 // M (upper triangle, FP64, r x r) += Z~^T Z~ with Z~ = diag(sqrt(w)) Z from `slices` int8 digits per value (5..8 base-128
-// ones: error about 2e-8, 3e-10, 3e-12, 3e-14 of ||Z~_p|| ||Z~_q||; kGramBase256: seven base-256 ones, about 1e-15).  `scratch` holds gram_tc_scratch_bytes.
+// ones: error about 2e-8, 3e-10, 3e-12, 3e-14 of ||Z~_p|| ||Z~_q||; kGramBase256: seven base-256 ones, about 1e-15).
+// `scratch` holds gram_tc_scratch_bytes.
 int gram_tc_weighted(db200_context* ctx, int n, int r, const double* Z, long long ldz, const double* w, double* M,
                      int ldm, void* scratch, int slices) {
   switch (slices) {

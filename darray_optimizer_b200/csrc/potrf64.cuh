@@ -4,16 +4,17 @@
 // Every warp holds 16 columns x 64 rows as mma.sync.m16n8k8.f64 accumulators of the transposed tile (column g of the
 // group, rows 8 b + 2 t and + 1 in d0, d1; column g + 8 in d2, d3), which are at once the A fragments of a product
 // over those rows (the pairing k = 2t, 2t + 1 inside the instruction is free).  Warps 0..3 hold the block's own column
-// groups, the others column groups of the block row.  In four steps p of 16 rows:
+// groups, the others column groups of the block row.  In up to four steps p of 16 rows:
 //   warp p factors its 16 x 16 diagonal block (factor16, whose elimination keeps the factor's backward error at a few u):
 //     one warp, lane = column, with the 16 columns of the identity in the other half-warp, so it also leaves W = R_pp^-T;
 //   every later group solves its rows p, X = W B, then X += W (B - R_pp^T X): the correction makes the solve as
 //     backward stable as substitution, whose 16 dependent steps it replaces by three 16 x 16 products;
 //   every later group subtracts R_pr^T X_p from its rows r > p.
 // What bounds it is the chain of 64 pivots, taken two at a time (a shuffle, a reciprocal, the reduced row through shared
-// memory and some products per pair): 23.6 k cycles for a full block with 64 columns of its block row, of which the four 16 x 16 factors take 16 k.  One
-// 64-column step of the blocked factor takes 21.5 us; with a barrier, a division and a strip update per pivot, and the
-// block row solved by 64 dependent shuffle steps, it took 38.8 us.
+// memory and some products per pair): 23.6 k cycles for a full block with 64 columns of its block row, of which the four
+// 16 x 16 factors take 16 k.  One 64-column step of the blocked factor takes 21.5 us; with a barrier, a division and a
+// strip update per pivot, and the block row solved by 64 dependent shuffle steps, it took 38.8 us.  A block of fewer
+// columns stops at its last 16.
 #pragma once
 #include <cstdint>
 

@@ -9,7 +9,8 @@
 //   2. cluster barrier (the block row is complete, the diagonal block has been read); one CTA writes R11;
 //   3. the trailing matrix is updated in 16 x 16 tiles, one warp each, fragments read straight from the block row
 //      (k contiguous, so a fragment is a 16-byte load); cluster barrier.
-// The matrix stays in L2 (2.2 MB at l = 528), which all CTAs reach at full rate: 52 us at l = 138, 219 us at l = 528.
+// The matrix stays in L2 (2.2 MB at l = 528), which all CTAs reach at full rate: 52 us at l = 138, 219 us at l = 528 (and
+// 3 and 10 us less since a short last block stops at its last 16 columns).
 // The form that kept the triangle in the CTAs' shared memory (67 and 372 us) spent a quarter of its time on the
 // all-to-all copy of the block row through distributed shared memory (~170 bytes per cycle for 13 CTAs), and the rest
 // about equally on its one-warp 32-pivot chains, its substitution and its update over column-cyclic slots.

@@ -415,7 +415,7 @@ int svm_barrier_impl(db200_context* ctx, int n, int r, const double* Z, int ldz,
       if (dmax / dmin > 1e18) break;  // tests/testsvm.cpp:258-263 (the factorisation above goes unused)
       const double lastg = 0.5 * ww - suma - sumlog / t;
       // Newton direction s = -(Z Z^T + D)^-1 g by Woodbury.  Mixed: capacity matrix M = I + Z^T D^-1 Z on the
-      // int8 tensor cores (Ozaki slices, ~1e-12 of the column norms) factored in FP64, then iterative refinement
+      // int8 tensor cores (Ozaki slices, ~1e-15 of the column norms) factored in FP64, then iterative refinement
       // against the exact FP64 operator
       // until the relative residual is <= 1e-10; a step that does not get there is recomputed with the FP64
       // capacity matrix.  FP64: the capacity matrix on the FP64 pipes, no refinement.
@@ -483,7 +483,7 @@ int svm_barrier_impl(db200_context* ctx, int n, int r, const double* Z, int ldz,
       // out = -H~^-1 rhs: one Woodbury application of the factored capacity matrix, no refinement.
       auto apply = [&](const double* rhs, double* out, double* rd) -> int { return woodbury(rhs, out, rd); };
       // Newton direction s = -(Z Z^T + D)^-1 g.  Mixed: capacity matrix on the int8 tensor cores (Ozaki slices,
-      // ~1e-12 of the column norms) factored in FP64, then refinement; a step whose refinement misses 1e-10 is
+      // ~1e-15 of the column norms) factored in FP64, then refinement; a step whose refinement misses 1e-10 is
       // recomputed with the FP64 capacity matrix.  FP64: the capacity matrix on the FP64 pipes, no refinement.
       //
       // With the bias, the bordered system [H y; y^T 0][s; nu] = [-g; 0].  With s~_y = -H~^-1 y (one more
@@ -551,7 +551,7 @@ int svm_barrier_impl(db200_context* ctx, int n, int r, const double* Z, int ldz,
       if ((st = newton_dir(mixed && tc_ok, &conv))) return st;
       if (mixed && tc_ok && !conv && tc_level == 0) {
         // the barrier's D only grows more ill-conditioned with t: once the 6-digit capacity matrix no longer
-        // preconditions well enough, this and the remaining Newton steps take the 8-digit one
+        // preconditions well enough, this and the remaining Newton steps take the base-256 one
         tc_level = 1;
         v_current = false;
         if ((st = newton_dir(true, &conv))) return st;
